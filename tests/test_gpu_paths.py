@@ -36,3 +36,23 @@ def test_tree_reports_each_pair_once_whatever_the_sizes(gpu, n, sizes):
         w.step(1e-4)
         got[algo] = w.pairs()
     assert_bit_equal(got[gpu.TREE], got[gpu.SAP], f"{n} {sizes}")
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 515])
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_batch_poses_reach_any_array(gpu, n, offset):
+    """Poses of a tile's edge sizes into pinned arrays on and off 16 bytes and
+    into pageable ones, with nothing written around them."""
+    import torch
+
+    sc = scenes.generate(scenes.MIXED_VOLUME, n, 7)
+    b = gpu.GpuBatch([sc], iterations=2)
+    b.step(1 / 60, 2)
+    pos, rot, _, _ = b.bodies()
+    for make in (lambda k: torch.full((k,), 7.0).pin_memory().numpy(), lambda k: np.full(k, 7.0, np.float32)):
+        p, q = make(3 * n + 8), make(4 * n + 8)
+        b.read_poses(p[offset:offset + 3 * n], q[offset:offset + 4 * n])
+        assert_bit_equal(p[offset:offset + 3 * n].reshape(n, 3), pos, "positions")
+        assert_bit_equal(q[offset:offset + 4 * n].reshape(n, 4), rot, "rotations")
+        for a, k in ((p, 3), (q, 4)):
+            assert np.all(a[:offset] == 7.0) and np.all(a[offset + k * n:] == 7.0)
