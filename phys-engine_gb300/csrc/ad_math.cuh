@@ -1,10 +1,9 @@
 // Scalar-generic math for the differentiable rollout.  The same formulas as the
 // engine's float math (pe_math.cuh), written over a scalar type S so that one
-// source serves float (GPU), double (the FP64 CPU adjoint) and forward-mode
-// dual numbers (Jacobians of contact geometry and contact preparation).  With
-// S = float the operations, their order and their constants are the engine's,
-// so values are bit-identical; a dual number's value part is computed by the
-// same operations as the plain scalar.  Compiles as CUDA and as plain C++.
+// source serves float (GPU) and double (the FP64 CPU adjoint), and the reverse
+// of the pieces that the adjoint runs through.  With S = float the operations
+// of the forward functions, their order and their constants are the engine's,
+// so values are bit-identical.  Compiles as CUDA and as plain C++.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -27,120 +26,13 @@ AD_HD double ssqrt(double v) { return sqrt(v); }
 AD_HD float sabs(float v) { return fabsf(v); }
 AD_HD double sabs(double v) { return fabs(v); }
 
-// ------------------------------------------------------------ dual numbers ---
-// Value plus K tangent components.  Comparisons use the value only, so a dual
-// evaluation takes exactly the branches of the plain evaluation.
-template <class T, int K> struct Dual {
-    T v;
-    T d[K];
-};
-template <class T, int K> AD_HD Dual<T, K> dconst(T v) {
-    Dual<T, K> r;
-    r.v = v;
-    for (int k = 0; k < K; ++k) r.d[k] = T(0);
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator+(const Dual<T, K> &a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a.v + b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] + b.d[k];
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator-(const Dual<T, K> &a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a.v - b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] - b.d[k];
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator-(const Dual<T, K> &a) {
-    Dual<T, K> r;
-    r.v = -a.v;
-    for (int k = 0; k < K; ++k) r.d[k] = -a.d[k];
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator*(const Dual<T, K> &a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a.v * b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator/(const Dual<T, K> &a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a.v / b.v;
-    const T inv = T(1) / b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * inv;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator+(const Dual<T, K> &a, T b) {
-    Dual<T, K> r = a;
-    r.v = a.v + b;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator+(T a, const Dual<T, K> &b) {
-    Dual<T, K> r = b;
-    r.v = a + b.v;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator-(const Dual<T, K> &a, T b) {
-    Dual<T, K> r = a;
-    r.v = a.v - b;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator-(T a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a - b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = -b.d[k];
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator*(const Dual<T, K> &a, T b) {
-    Dual<T, K> r;
-    r.v = a.v * b;
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator*(T a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a * b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = a * b.d[k];
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator/(const Dual<T, K> &a, T b) {
-    Dual<T, K> r;
-    r.v = a.v / b;
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] / b;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> operator/(T a, const Dual<T, K> &b) {
-    Dual<T, K> r;
-    r.v = a / b.v;
-    const T inv = T(1) / b.v;
-    for (int k = 0; k < K; ++k) r.d[k] = -r.v * b.d[k] * inv;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> &operator+=(Dual<T, K> &a, const Dual<T, K> &b) {
-    a = a + b;
-    return a;
-}
-template <class T, int K> AD_HD Dual<T, K> ssqrt(const Dual<T, K> &a) {
-    Dual<T, K> r;
-    r.v = ssqrt(a.v);
-    const T g = r.v > T(0) ? T(0.5) / r.v : T(0);
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * g;
-    return r;
-}
-template <class T, int K> AD_HD Dual<T, K> sabs(const Dual<T, K> &a) { return a.v < T(0) ? -a : a; }
-
 AD_HD float val(float v) { return v; }
 AD_HD double val(double v) { return v; }
-template <class T, int K> AD_HD T val(const Dual<T, K> &a) { return a.v; }
 
 // Scalar S built from a constant of its value type (float constants first
 // rounded to float, as the reference writes them).
 template <class S> struct Lit {
     template <class C> AD_HD static S make(C c) { return S(c); }
-};
-template <class T, int K> struct Lit<Dual<T, K>> {
-    template <class C> AD_HD static Dual<T, K> make(C c) { return dconst<T, K>(T(c)); }
 };
 #define ADL(S, c) ::pe::ad::Lit<S>::make(c)
 
@@ -258,6 +150,72 @@ template <class S> AD_HD void qmulAdj(const Q<S> &a, const Q<S> &o, const Q<S> &
     ob.y = ob.y + (-r.x * a.z + r.y * a.w + r.z * a.x - r.w * a.y);
     ob.z = ob.z + (r.x * a.y - r.y * a.x + r.z * a.w - r.w * a.z);
     ob.w = ob.w + (r.x * a.x + r.y * a.y + r.z * a.z + r.w * a.w);
+}
+
+// r = rotate(q, v): for any q the product q v q* is
+// (w^2 - u.u) v + 2 (u.v) u + 2 w (u x v), so with the adjoint g of r
+template <class S> AD_HD void rotateAdj(const Q<S> &q, const V3<S> &v, const V3<S> &g, Q<S> &qb, V3<S> &vb) {
+    const V3<S> u{q.x, q.y, q.z};
+    const S two = S(2), ug = dot(u, g), uv = dot(u, v), vg = dot(v, g), ww = q.w * q.w - dot(u, u);
+    const V3<S> vxg = cross(v, g), gxu = cross(g, u);
+    vb += g * ww + u * (two * ug) + gxu * (two * q.w);
+    qb.x = qb.x + two * (ug * v.x + uv * g.x - vg * u.x + q.w * vxg.x);
+    qb.y = qb.y + two * (ug * v.y + uv * g.y - vg * u.y + q.w * vxg.y);
+    qb.z = qb.z + two * (ug * v.z + uv * g.z - vg * u.z + q.w * vxg.z);
+    qb.w = qb.w + two * (q.w * vg + dot(u, vxg));
+}
+// r = rotate(conj(q), v).
+template <class S> AD_HD void rotateConjAdj(const Q<S> &q, const V3<S> &v, const V3<S> &g, Q<S> &qb, V3<S> &vb) {
+    Q<S> cb{S(0), S(0), S(0), S(0)};
+    rotateAdj(conj(q), v, g, cb, vb);
+    qb.x = qb.x - cb.x;
+    qb.y = qb.y - cb.y;
+    qb.z = qb.z - cb.z;
+    qb.w = qb.w + cb.w;
+}
+// l = toLocal(w, t), w = toWorld(l, t).
+template <class S> AD_HD void toLocalAdj(const V3<S> &w, const Tf<S> &t, const V3<S> &g, Tf<S> &tb, V3<S> &wb) {
+    V3<S> d{S(0), S(0), S(0)};
+    rotateConjAdj(t.q, w - t.p, g, tb.q, d);
+    wb += d;
+    tb.p += -d;
+}
+template <class S> AD_HD void toWorldAdj(const V3<S> &l, const Tf<S> &t, const V3<S> &g, Tf<S> &tb) {
+    V3<S> lb{S(0), S(0), S(0)};
+    rotateAdj(t.q, l, g, tb.q, lb);
+    tb.p += g;
+}
+// m = toMat3(q).
+template <class S> AD_HD void toMat3Adj(const Q<S> &q, const M3<S> &b, Q<S> &qb) {
+    const S two = S(2), four = S(4);
+    const S p01 = b.m01 + b.m10, p02 = b.m02 + b.m20, p12 = b.m12 + b.m21;
+    const S d01 = b.m10 - b.m01, d02 = b.m02 - b.m20, d12 = b.m21 - b.m12;
+    qb.x = qb.x + two * (q.y * p01 + q.z * p02 + q.w * d12) - four * q.x * (b.m11 + b.m22);
+    qb.y = qb.y + two * (q.x * p01 + q.z * p12 + q.w * d02) - four * q.y * (b.m00 + b.m22);
+    qb.z = qb.z + two * (q.x * p02 + q.y * p12 + q.w * d01) - four * q.z * (b.m00 + b.m11);
+    qb.w = qb.w + two * (q.z * d01 + q.y * d02 + q.x * d12);
+}
+// r = mul(m, v): adjoint of m (outer product) and of v.
+template <class S> AD_HD void mulAdj(const M3<S> &m, const V3<S> &v, const V3<S> &g, M3<S> &mb, V3<S> &vb) {
+    mb.m00 = mb.m00 + g.x * v.x;
+    mb.m01 = mb.m01 + g.x * v.y;
+    mb.m02 = mb.m02 + g.x * v.z;
+    mb.m10 = mb.m10 + g.y * v.x;
+    mb.m11 = mb.m11 + g.y * v.y;
+    mb.m12 = mb.m12 + g.y * v.z;
+    mb.m20 = mb.m20 + g.z * v.x;
+    mb.m21 = mb.m21 + g.z * v.y;
+    mb.m22 = mb.m22 + g.z * v.z;
+    vb += mul(transpose(m), g);
+}
+// I = inverseInertiaWorld(q, d) = R diag(d) R^T: the adjoint of R's column k is
+// d_k (Ib + Ib^T) R_k.
+template <class S> AD_HD void inverseInertiaAdj(const Q<S> &q, const V3<S> &d, const M3<S> &b, Q<S> &qb) {
+    const M3<S> R = toMat3(q);
+    const M3<S> s{b.m00 + b.m00, b.m01 + b.m10, b.m02 + b.m20, b.m10 + b.m01, b.m11 + b.m11,
+                  b.m12 + b.m21, b.m20 + b.m02, b.m21 + b.m12, b.m22 + b.m22};
+    const S z = S(0);
+    toMat3Adj(q, mul(mul(s, R), M3<S>{d.x, z, z, z, d.y, z, z, z, d.z}), qb);
 }
 
 } // namespace ad

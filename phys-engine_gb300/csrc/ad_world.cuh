@@ -1,113 +1,45 @@
 // Differentiable world step: PhysicsWorld::step (src/world/physics_world.cpp:
-// 518-782) for a small world of sphere/box bodies, written for a team of
-// threads (one CUDA thread block, or one host thread) over a scalar type S,
-// plus its hand-written reverse (adjoint) with the contact set of the forward
-// pass frozen: the pairs, the separating axes / kept vertices, the colour
-// order, the warm-start matches and every clamp branch are the ones the
-// forward evaluation took; everything continuous is differentiated, including
-// the contact points, normals and depths as functions of the poses.
+// 518-782) for a small world of sphere/box bodies over a scalar type S, plus
+// its hand-written reverse (adjoint) with the contact set of the forward pass
+// frozen: the pairs, the separating axes / kept vertices, the colour order, the
+// warm-start matches and every clamp branch are the ones the forward evaluation
+// took; everything continuous is differentiated, including the contact points,
+// normals and depths as functions of the poses.
 //
 // Forward (mirrors the engine stage by stage): velocity integration, AABBs,
-// all-pairs AABB test in lexicographic order (= the SAP pair set and order),
-// narrowphase in pair order, greedy colouring by manifold priority (= the
-// engine's colouring), solve order (colour, index), prepare + warm-start
-// matching, warm start, velocity iterations, cache rebuild, pose integration.
+// sweep along x with the pairs in lexicographic order, narrowphase in pair
+// order, greedy colouring by manifold priority (= the engine's colouring),
+// solve order (colour, index), prepare + warm-start matching, warm start,
+// velocity iterations, cache rebuild, pose integration.
 //
 // Reverse, per step, given the adjoints of the step's outputs (poses,
 // velocities, and the final impulses that the next step's warm start read):
 //   pose integration -> velocity iterations (colours in reverse, points in
 //   reverse, from a tape of the pre-update velocities and impulses) -> warm
 //   start -> warm-start matching (to the previous step's impulses) -> contact
-//   geometry + preparation (forward-mode dual numbers, four directions at a
-//   time) -> materials (friction = sqrt(fa fb), restitution = max) -> velocity
-//   integration.
+//   preparation -> contact geometry -> materials (friction = sqrt(fa fb),
+//   restitution = max) -> velocity integration.
+//
+// This file holds the pieces of the step and its evaluation by one host thread
+// (double precision); ad_block.cuh runs the same pieces on a thread block.
 #pragma once
 #include "ad_geom.cuh"
 
 #if !defined(__CUDACC__)
 #include <algorithm>
 #include <cstring>
+#include <vector>
 #endif
 
 namespace pe {
 namespace ad {
 
 constexpr uint32_t kAdMaxColors = 128;  // colours per window of the per-body colour masks
-constexpr int kDualChunk = 4;
-constexpr int kDualInputs = 29;  // xA 3, qA 4, xB 3, qB 4, v1A 3, w1A 3, v1B 3, w1B 3, mA, mB, restitution
+constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 constexpr int kTapeScalars = 24; // vA, wA, vB, wB, then 4 x (n, t1, t2)
 constexpr int kPmScalars = 20;   // IA (9), IB (9), imA, imB
 
-enum : uint32_t { kAdErrPairs = 1, kAdErrManifolds = 2, kAdErrColors = 4, kAdErrCache = 8, kAdErrReplay = 16 };
-
-// ------------------------------------------------------------------ teams ---
-#if !defined(__CUDACC__)
-struct HostTeam {
-    static uint32_t tid() { return 0; }
-    static uint32_t size() { return 1; }
-    static void sync() {}
-    template <class S> static void add(S *p, S v) { *p += v; }
-    static void orErr(uint32_t *p, uint32_t v) { *p |= v; }
-    static uint32_t scan(uint32_t v, uint32_t &total) {
-        total = v;
-        return 0;
-    }
-    static void sortU64(unsigned long long *k, uint32_t n) { std::sort(k, k + n); }
-};
-#else
-struct BlockTeam {
-    static __device__ __forceinline__ uint32_t tid() { return threadIdx.x; }
-    static __device__ __forceinline__ uint32_t size() { return blockDim.x; }
-    static __device__ __forceinline__ void sync() { __syncthreads(); }
-    template <class S> static __device__ __forceinline__ void add(S *p, S v) { atomicAdd(p, v); }
-    static __device__ __forceinline__ void orErr(uint32_t *p, uint32_t v) { atomicOr(p, v); }
-    // Exclusive scan over the block (multiple of 32 threads, <= 1024).
-    static __device__ uint32_t scan(uint32_t v, uint32_t &total) {
-        __shared__ uint32_t s[33];
-        const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        uint32_t incl = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((int)lane >= o) incl += n;
-        }
-        if (lane == 31) s[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t x = lane < nw ? s[lane] : 0u;
-            uint32_t xi = x;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t n = __shfl_up_sync(0xffffffffu, xi, o);
-                if ((int)lane >= o) xi += n;
-            }
-            if (lane < nw) s[lane] = xi - x;
-            if (lane == 31) s[32] = xi;
-        }
-        __syncthreads();
-        const uint32_t r = s[warp] + incl - v;
-        total = s[32];
-        __syncthreads();
-        return r;
-    }
-    // Bitonic sort of n (power of two) keys by the whole block.
-    static __device__ void sortU64(unsigned long long *k, uint32_t n) {
-        for (uint32_t size = 2; size <= n; size <<= 1)
-            for (uint32_t j = size >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-                    const uint32_t ixj = i ^ j;
-                    if (ixj > i) {
-                        const unsigned long long a = k[i], b = k[ixj];
-                        const bool up = (i & size) == 0;
-                        if ((a > b) == up) {
-                            k[i] = b;
-                            k[ixj] = a;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-    }
-};
-#endif
+enum : uint32_t { kAdErrPairs = 1, kAdErrManifolds = 2, kAdErrColors = 4, kAdErrCache = 8 };
 
 AD_HD uint32_t nextPow2u(uint32_t v) {
     uint32_t p = 1;
@@ -154,7 +86,6 @@ template <class S> struct CacheView {
 
 template <class S> struct StepScratch {
     S *aabb;                        // 6 per body
-    uint32_t *pairA, *pairB;        // maxPairs
     uint32_t *mA, *mB, *mCount;     // manifolds in pair order
     uint32_t *mFeature;             // 4 per manifold
     S *mNormal;                     // 3
@@ -162,6 +93,7 @@ template <class S> struct StepScratch {
     S *mAnchorA, *mAnchorB;         // 12 each
     S *mDepth;                      // 4
     uint32_t *color, *order;        // maxManifolds
+    uint32_t *rank;                 // maxManifolds: place of a manifold in the order (thread blocks)
     unsigned long long *sortKeys;   // maxManifolds
     unsigned long long *bodyUsed;   // 2 per body
     uint32_t *colorStart;           // maxManifolds + 1 (colours <= manifolds)
@@ -171,7 +103,7 @@ template <class S> struct StepScratch {
     S *lamInit;                     // 3 per (k, p)
     int32_t *match;                 // per (k, p): matched cache entry or -1
     S *tape;                        // iterations * maxManifolds * kTapeScalars
-    uint32_t *cacheSrc;             // per cache-out entry: k * 4 + p
+    uint32_t *cacheSlot;            // per (k, p): its entry of the output cache, or kNoSlot
     uint32_t *counts;               // [0] pairs, [1] manifolds, [2] colours, [3] error bits
     // broadphase scratch (not recorded: it may be shared by the steps of a segment)
     unsigned long long *bpEntries;  // nextPow2(n): (min.x key << 32) | body
@@ -190,10 +122,14 @@ template <class S> struct AdjointView {
     S *ax, *aq, *av, *aw;        // per body (3, 4, 3, 3)
     S *alam;                     // 3 per (k, p)
     S *app;                      // kPreparedScalars per (k, p)
+    S *acache;                   // 3 per entry of the step's input cache
+    // one host thread
     S *apm;                      // kPmScalars per k
     S *an;                       // 3 per k
-    S *amuM, *arestM;            // per k
-    S *acache;                   // 3 per entry of the step's input cache
+    S *amuM;                     // per k
+    // thread blocks
+    S *aext;                     // kAdjointExtra per (k, p)
+    S *dv, *dw;                  // 3 per body: additions to av, aw
     S *amass, *amu, *arest;      // per body, accumulated over steps
 };
 
@@ -224,7 +160,7 @@ template <class S> struct PointIn {
     S ln, l1, l2;
 };
 template <class S>
-AD_HDN void pointForward(const V3<S> &n, const S &friction, const S *c, const S &imA, const S &imB, bool sA, bool sB,
+AD_HD void pointForward(const V3<S> &n, const S &friction, const S *c, const S &imA, const S &imB, bool sA, bool sB,
                         PointIn<S> &st) {
     const S iem = c[kPIem];
     if (val(iem) <= 0.0f) return;
@@ -274,212 +210,354 @@ AD_HDN void pointForward(const V3<S> &n, const S &friction, const S *c, const S 
     }
 }
 
-// Reverse of pointForward.  `in` holds the point's inputs; `a` holds the
-// adjoints of its outputs on entry and of its inputs on exit.  Adjoints of the
-// prepared constants go to ac[], of the normal to an, of the friction to amu,
-// of the inverse masses to aimA / aimB.
+// Reverse of pointForward, in three parts so that a thread block can run the
+// first and the last for all points of a manifold at once and only the second
+// point after point.
+//
+// Part 1: the forward intermediates at the point's inputs.
+template <class S> struct PointMid {
+    V3<S> rel;
+    S num, raw, ln, applied, mu0, limit, tv1, tv2, a1, a2, u1, u2, kq;
+    bool live, fric, scaled;
+};
 template <class S>
-AD_HDN void pointReverse(const V3<S> &n, const S &friction, const S *c, const S &imA, const S &imB, bool sA, bool sB,
-                        const PointIn<S> &in, PointIn<S> &a, S *ac, V3<S> &an, S &amu, S &aimA, S &aimB) {
-    const S iem = c[kPIem];
-    if (val(iem) <= 0.0f) return;
-    const S z = S(0);
+AD_HD PointMid<S> pointMid(const V3<S> &n, const S &friction, const S *c, const PointIn<S> &in) {
+    PointMid<S> m;
+    const S z = S(0), iem = c[kPIem];
+    m.live = !(iem <= 0.0f);
+    m.fric = false;
+    m.scaled = false;
+    if (!m.live) return m;
     const V3<S> offA = pv(c, kPOffA), offB = pv(c, kPOffB), t1 = pv(c, kPT1), t2 = pv(c, kPT2);
-    // recompute the forward intermediates
     const V3<S> vAp = in.vA + cross(in.wA, offA), vBp = in.vB + cross(in.wB, offB);
-    const V3<S> rel = vBp - vAp;
-    const S vn = dot(rel, n);
-    const S num = vn + c[kPRv] - c[kPBias];
-    const S delta = -num / iem;
+    m.rel = vBp - vAp;
+    const S vn = dot(m.rel, n);
+    m.num = vn + c[kPRv] - c[kPBias];
+    const S delta = -m.num / iem;
     const S prev = in.ln;
-    const S raw = prev + delta;
-    const S ln = smax(raw, z);
-    const S applied = ln - prev;
-    const V3<S> impulse = n * applied;
+    m.raw = prev + delta;
+    m.ln = smax(m.raw, z);
+    m.applied = m.ln - prev;
+    m.fric = !(c[kPItm00] <= z || c[kPItm11] <= z);
+    if (m.fric) {
+        m.mu0 = smax(friction, z);
+        m.limit = m.mu0 * m.ln;
+        m.tv1 = dot(m.rel, t1) + c[kPNtr1] * m.applied;
+        m.tv2 = dot(m.rel, t2) + c[kPNtr2] * m.applied;
+        const S d1 = -(c[kPItm00] * m.tv1 + c[kPItm01] * m.tv2);
+        const S d2 = -(c[kPItm01] * m.tv1 + c[kPItm11] * m.tv2);
+        const S r1 = in.l1 + d1, r2 = in.l2 + d2;
+        const S lsq = r1 * r1 + r2 * r2;
+        m.scaled = lsq > m.limit * m.limit;
+        S f1 = r1, f2 = r2;
+        if (m.scaled) {
+            const S L = ssqrt(lsq);
+            m.kq = m.limit / L;
+            f1 = r1 * m.kq;
+            f2 = r2 * m.kq;
+            m.u1 = r1 / L;
+            m.u2 = r2 / L;
+        }
+        m.a1 = f1 - in.l1;
+        m.a2 = f2 - in.l2;
+    }
+    return m;
+}
+
+// Part 2: `a` holds the adjoints of the point's outputs on entry and of its
+// inputs on exit; what part 3 needs is kept in the return value.
+template <class S> struct PointAdj {
+    V3<S> vA, wA, vB, wB;  // adjoints of the point's output velocities
+    V3<S> ati, arel;
+    S aa1, aa2, ar1, ar2, alimit, atv1, atv2, adelta, anum;
+};
+template <class S>
+AD_HD PointAdj<S> pointChain(const V3<S> &n, const S *c, const S &imA, const S &imB, bool sA, bool sB,
+                             const PointMid<S> &m, PointIn<S> &a) {
+    PointAdj<S> r{};
+    if (!m.live) return r;
+    const S z = S(0), iem = c[kPIem];
+    r.vA = a.vA;
+    r.wA = a.wA;
+    r.vB = a.vB;
+    r.wB = a.wB;
+    V3<S> ati{z, z, z};
+    if (!sB) ati += a.vB * imB;
+    if (!sA) ati += -(a.vA * imA);
+    r.ati = ati;
+    r.aa1 = r.aa2 = r.ar1 = r.ar2 = r.alimit = r.atv1 = r.atv2 = z;
     S aln = a.ln, aapplied = z, aprev = z;
     V3<S> arel{z, z, z};
-    const bool fric = !(c[kPItm00] <= z || c[kPItm11] <= z);
-    if (fric) {
-        const S mu0 = smax(friction, z);
-        const S limit = mu0 * ln;
-        const S tv1 = dot(rel, t1) + c[kPNtr1] * applied;
-        const S tv2 = dot(rel, t2) + c[kPNtr2] * applied;
-        const S d1 = -(c[kPItm00] * tv1 + c[kPItm01] * tv2);
-        const S d2 = -(c[kPItm01] * tv1 + c[kPItm11] * tv2);
-        const S p1 = in.l1, p2 = in.l2;
-        const S r1 = p1 + d1, r2 = p2 + d2;
-        const S lsq = r1 * r1 + r2 * r2;
-        const bool scaled = lsq > limit * limit;
-        S f1 = r1, f2 = r2, L = z;
-        if (scaled) {
-            L = ssqrt(lsq);
-            const S s = limit / L;
-            f1 = r1 * s;
-            f2 = r2 * s;
-        }
-        const S a1 = f1 - p1, a2 = f2 - p2;
-        const V3<S> ti = t1 * a1 + t2 * a2;
-        // velocities after the friction update
-        V3<S> ati{z, z, z}, arA{z, z, z}, arB{z, z, z};
-        if (!sB) {
-            ati += a.vB * imB;
-            aimB = aimB + dot(a.vB, ti);
-            arB = a.wB;
-        }
-        if (!sA) {
-            ati += -(a.vA * imA);
-            aimA = aimA - dot(a.vA, ti);
-            arA = -a.wA;
-        }
-        S aa1 = dot(ati, t1) + dot(arA, pv(c, kPTrA1)) + dot(arB, pv(c, kPTrB1));
-        S aa2 = dot(ati, t2) + dot(arA, pv(c, kPTrA2)) + dot(arB, pv(c, kPTrB2));
-        auto acc3 = [&](int f, const V3<S> &v) {
-            ac[3 * f] = ac[3 * f] + v.x;
-            ac[3 * f + 1] = ac[3 * f + 1] + v.y;
-            ac[3 * f + 2] = ac[3 * f + 2] + v.z;
-        };
-        acc3(kPT1, ati * a1);
-        acc3(kPT2, ati * a2);
-        acc3(kPTrA1, arA * a1);
-        acc3(kPTrA2, arA * a2);
-        acc3(kPTrB1, arB * a1);
-        acc3(kPTrB2, arB * a2);
+    if (m.fric) {
+        V3<S> arA{z, z, z}, arB{z, z, z};
+        if (!sB) arB = a.wB;
+        if (!sA) arA = -a.wA;
+        r.aa1 = dot(ati, pv(c, kPT1)) + dot(arA, pv(c, kPTrA1)) + dot(arB, pv(c, kPTrB1));
+        r.aa2 = dot(ati, pv(c, kPT2)) + dot(arA, pv(c, kPTrA2)) + dot(arB, pv(c, kPTrB2));
         // a = f - p; the outputs l1, l2 are f
-        S af1 = a.l1 + aa1, af2 = a.l2 + aa2;
-        S ap1 = -aa1, ap2 = -aa2;
-        S ar1 = af1, ar2 = af2, alimit = z;
-        if (scaled) {
-            const S u1 = r1 / L, u2 = r2 / L;
-            const S ua = u1 * af1 + u2 * af2;
-            const S k = limit / L;
-            ar1 = k * (af1 - u1 * ua);
-            ar2 = k * (af2 - u2 * ua);
-            alimit = ua;
+        const S af1 = a.l1 + r.aa1, af2 = a.l2 + r.aa2;
+        r.ar1 = af1;
+        r.ar2 = af2;
+        if (m.scaled) {
+            const S ua = m.u1 * af1 + m.u2 * af2;
+            r.ar1 = m.kq * (af1 - m.u1 * ua);
+            r.ar2 = m.kq * (af2 - m.u2 * ua);
+            r.alimit = ua;
         }
-        ap1 = ap1 + ar1;
-        ap2 = ap2 + ar2;
-        const S ad1 = ar1, ad2 = ar2;
-        const S atv1 = -(ad1 * c[kPItm00] + ad2 * c[kPItm01]);
-        const S atv2 = -(ad1 * c[kPItm01] + ad2 * c[kPItm11]);
-        ac[kPItm00] = ac[kPItm00] - ad1 * tv1;
-        ac[kPItm01] = ac[kPItm01] - (ad1 * tv2 + ad2 * tv1);
-        ac[kPItm11] = ac[kPItm11] - ad2 * tv2;
-        arel += t1 * atv1 + t2 * atv2;
-        acc3(kPT1, rel * atv1);
-        acc3(kPT2, rel * atv2);
-        ac[kPNtr1] = ac[kPNtr1] + atv1 * applied;
-        ac[kPNtr2] = ac[kPNtr2] + atv2 * applied;
-        aapplied = aapplied + atv1 * c[kPNtr1] + atv2 * c[kPNtr2];
-        if (!(friction < z)) amu = amu + alimit * ln;
-        aln = aln + alimit * mu0;
-        a.l1 = ap1;
-        a.l2 = ap2;
+        a.l1 = -r.aa1 + r.ar1;
+        a.l2 = -r.aa2 + r.ar2;
+        r.atv1 = -(r.ar1 * c[kPItm00] + r.ar2 * c[kPItm01]);
+        r.atv2 = -(r.ar1 * c[kPItm01] + r.ar2 * c[kPItm11]);
+        arel += pv(c, kPT1) * r.atv1 + pv(c, kPT2) * r.atv2;
+        aapplied = aapplied + r.atv1 * c[kPNtr1] + r.atv2 * c[kPNtr2];
+        aln = aln + r.alimit * m.mu0;
     }
     // normal update
-    V3<S> aimp{z, z, z};
-    if (!sB) {
-        aimp += a.vB * imB;
-        aimB = aimB + dot(a.vB, impulse);
-        const V3<S> nrB = pv(c, kPNrB);
-        ac[3 * kPNrB] = ac[3 * kPNrB] + a.wB.x * applied;
-        ac[3 * kPNrB + 1] = ac[3 * kPNrB + 1] + a.wB.y * applied;
-        ac[3 * kPNrB + 2] = ac[3 * kPNrB + 2] + a.wB.z * applied;
-        aapplied = aapplied + dot(a.wB, nrB);
-    }
-    if (!sA) {
-        aimp += -(a.vA * imA);
-        aimA = aimA - dot(a.vA, impulse);
-        const V3<S> nrA = pv(c, kPNrA);
-        ac[3 * kPNrA] = ac[3 * kPNrA] - a.wA.x * applied;
-        ac[3 * kPNrA + 1] = ac[3 * kPNrA + 1] - a.wA.y * applied;
-        ac[3 * kPNrA + 2] = ac[3 * kPNrA + 2] - a.wA.z * applied;
-        aapplied = aapplied - dot(a.wA, nrA);
-    }
-    an += aimp * applied;
-    aapplied = aapplied + dot(aimp, n);
+    if (!sB) aapplied = aapplied + dot(a.wB, pv(c, kPNrB));
+    if (!sA) aapplied = aapplied - dot(a.wA, pv(c, kPNrA));
+    aapplied = aapplied + dot(ati, n);
     aln = aln + aapplied;
     aprev = aprev - aapplied;
-    const S araw = (raw < z) ? z : aln;
+    const S araw = (m.raw < z) ? z : aln;
     aprev = aprev + araw;
-    const S adelta = araw;
-    const S anum = -adelta / iem;
-    ac[kPIem] = ac[kPIem] + adelta * num / (iem * iem);
-    ac[kPRv] = ac[kPRv] + anum;
-    ac[kPBias] = ac[kPBias] - anum;
-    arel += n * anum;
-    an += rel * anum;
+    r.adelta = araw;
+    r.anum = -araw / iem;
+    arel += n * r.anum;
+    r.arel = arel;
     // rel = (vB + wB x offB) - (vA + wA x offA)
     a.vB += arel;
     a.vA += -arel;
-    V3<S> aoffB{z, z, z}, aoffA{z, z, z}, awB = a.wB, awA = a.wA;
-    crossAdj(in.wB, offB, arel, awB, aoffB);
-    crossAdj(in.wA, offA, -arel, awA, aoffA);
-    a.wB = awB;
-    a.wA = awA;
-    ac[3 * kPOffB] = ac[3 * kPOffB] + aoffB.x;
-    ac[3 * kPOffB + 1] = ac[3 * kPOffB + 1] + aoffB.y;
-    ac[3 * kPOffB + 2] = ac[3 * kPOffB + 2] + aoffB.z;
-    ac[3 * kPOffA] = ac[3 * kPOffA] + aoffA.x;
-    ac[3 * kPOffA + 1] = ac[3 * kPOffA + 1] + aoffA.y;
-    ac[3 * kPOffA + 2] = ac[3 * kPOffA + 2] + aoffA.z;
+    a.wB += cross(pv(c, kPOffB), arel);
+    a.wA += cross(pv(c, kPOffA), -arel);
     a.ln = aprev;
+    return r;
 }
 
-// ------------------------------------------------------------------ forward --
-template <class S, class T>
-AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const CacheView<S> &cin, StateView<S> out,
-                       CacheView<S> cout, StepScratch<S> sc, bool record) {
-    const uint32_t tid = T::tid(), nt = T::size(), n = W.n;
+// Part 3: adjoints of the prepared constants to ac[], of the normal to an, of
+// the friction to amu, of the inverse masses to aimA / aimB.
+template <class S>
+AD_HD void pointAccumulate(const V3<S> &n, const S &friction, const S *c, const PointIn<S> &in, bool sA, bool sB,
+                           const PointMid<S> &m, const PointAdj<S> &r, S *ac, V3<S> &an, S &amu, S &aimA, S &aimB) {
+    if (!m.live) return;
+    const S z = S(0), iem = c[kPIem];
+    auto acc3 = [&](int f, const V3<S> &v) {
+        ac[3 * f] = ac[3 * f] + v.x;
+        ac[3 * f + 1] = ac[3 * f + 1] + v.y;
+        ac[3 * f + 2] = ac[3 * f + 2] + v.z;
+    };
+    if (m.fric) {
+        const V3<S> ti = pv(c, kPT1) * m.a1 + pv(c, kPT2) * m.a2;
+        V3<S> arA{z, z, z}, arB{z, z, z};
+        if (!sB) {
+            aimB = aimB + dot(r.vB, ti);
+            arB = r.wB;
+        }
+        if (!sA) {
+            aimA = aimA - dot(r.vA, ti);
+            arA = -r.wA;
+        }
+        acc3(kPT1, r.ati * m.a1);
+        acc3(kPT2, r.ati * m.a2);
+        acc3(kPTrA1, arA * m.a1);
+        acc3(kPTrA2, arA * m.a2);
+        acc3(kPTrB1, arB * m.a1);
+        acc3(kPTrB2, arB * m.a2);
+        ac[kPItm00] = ac[kPItm00] - r.ar1 * m.tv1;
+        ac[kPItm01] = ac[kPItm01] - (r.ar1 * m.tv2 + r.ar2 * m.tv1);
+        ac[kPItm11] = ac[kPItm11] - r.ar2 * m.tv2;
+        acc3(kPT1, m.rel * r.atv1);
+        acc3(kPT2, m.rel * r.atv2);
+        ac[kPNtr1] = ac[kPNtr1] + r.atv1 * m.applied;
+        ac[kPNtr2] = ac[kPNtr2] + r.atv2 * m.applied;
+        if (!(friction < z)) amu = amu + r.alimit * m.ln;
+    }
+    const V3<S> impulse = n * m.applied;
+    if (!sB) {
+        aimB = aimB + dot(r.vB, impulse);
+        acc3(kPNrB, r.wB * m.applied);
+    }
+    if (!sA) {
+        aimA = aimA - dot(r.vA, impulse);
+        acc3(kPNrA, r.wA * (-m.applied));
+    }
+    an += r.ati * m.applied;
+    ac[kPIem] = ac[kPIem] + r.adelta * m.num / (iem * iem);
+    ac[kPRv] = ac[kPRv] + r.anum;
+    ac[kPBias] = ac[kPBias] - r.anum;
+    an += m.rel * r.anum;
+    acc3(kPOffB, cross(r.arel, in.wB));
+    acc3(kPOffA, cross(-r.arel, in.wA));
+}
+
+// Velocities after the forward pass's integration (integrateVelocity without an
+// applied force).
+template <class S> AD_HD V3<S> integratedVelocity(const WorldParams<S> &W, uint32_t i, V3<S> v) {
+    if (!W.isStatic[i]) {
+        const S z = ADL(S, 0.0f);
+        const V3<S> g{W.gx, W.gy, W.gz}, f{z, z, z};
+        const V3<S> acc = g + f * inverseMass(false, W.mass[i]);
+        v += acc * W.dt;
+    }
+    return v;
+}
+
+template <class S> AD_HD void bodyAabb(const WorldParams<S> &W, uint32_t i, const V3<S> &p, const Q<S> &q, V3<S> &mn,
+                                       V3<S> &mx) {
+    if (W.shape[i] == 0) {
+        const S r = W.dims[3 * i];
+        const V3<S> rr{r, r, r};
+        mn = p - rr;
+        mx = p + rr;
+    } else {
+        const M3<S> m = toMat3(q);
+        const S hx = W.dims[3 * i], hy = W.dims[3 * i + 1], hz = W.dims[3 * i + 2];
+        const V3<S> e{sabs(m.m00) * hx + sabs(m.m01) * hy + sabs(m.m02) * hz,
+                      sabs(m.m10) * hx + sabs(m.m11) * hy + sabs(m.m12) * hz,
+                      sabs(m.m20) * hx + sabs(m.m21) * hy + sabs(m.m22) * hz};
+        mn = p - e;
+        mx = p + e;
+    }
+}
+
+// Pose integration (rigid_body.cpp:103-125) of one body and its reverse.
+template <class S> AD_HD void poseForward(const S &dt, const V3<S> &lin, const V3<S> &ang, V3<S> &pos, Q<S> &rot) {
+    pos += lin * dt;
+    const Q<S> spin{ang.x, ang.y, ang.z, ADL(S, 0.0f)};
+    const Q<S> d = qmul(spin, rot);
+    const S h = ADL(S, 0.5f) * dt;
+    rot.x = rot.x + h * d.x;
+    rot.y = rot.y + h * d.y;
+    rot.z = rot.z + h * d.z;
+    rot.w = rot.w + h * d.w;
+    rot = qnormalized(rot);
+}
+// rot, ang: the inputs; aq: adjoint of the new rotation in, of the old one out;
+// av, aw: adjoints of the velocities, added to.
+template <class S>
+AD_HD void poseReverse(const S &dt, const Q<S> &rot, const V3<S> &ang, const V3<S> &ax, Q<S> &aq, V3<S> &av, V3<S> &aw) {
+    const S z = S(0);
+    av += ax * dt;
+    const Q<S> spin{ang.x, ang.y, ang.z, z};
+    const Q<S> d = qmul(spin, rot);
+    const S h = S(0.5f) * dt;
+    const Q<S> u{rot.x + h * d.x, rot.y + h * d.y, rot.z + h * d.z, rot.w + h * d.w};
+    const S len = ssqrt(u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w);
+    Q<S> au{z, z, z, z};
+    if (len != z) {
+        const Q<S> q1{u.x / len, u.y / len, u.z / len, u.w / len};
+        const S qa = q1.x * aq.x + q1.y * aq.y + q1.z * aq.z + q1.w * aq.w;
+        au = Q<S>{(aq.x - q1.x * qa) / len, (aq.y - q1.y * qa) / len, (aq.z - q1.z * qa) / len,
+                  (aq.w - q1.w * qa) / len};
+    }
+    Q<S> arot = au, aspin{z, z, z, z};
+    const Q<S> ad{h * au.x, h * au.y, h * au.z, h * au.w};
+    qmulAdj(spin, rot, ad, aspin, arot);
+    aw += V3<S>{aspin.x, aspin.y, aspin.z};
+    aq = arot;
+}
+
+// Impulses of a matched cache entry (normal, tangents) clamped to the friction
+// cone (sequential_impulse_solver.cpp:448-490), and the reverse: adjoints of
+// the clamped impulses in, of the entry's out; the friction's is added to.
+template <class S> AD_HD void warmClamp(const S &friction, const S &cn, const S &c1, const S &c2, S &l0, S &l1, S &l2) {
     const S z = ADL(S, 0.0f);
-    const V3<S> g{W.gx, W.gy, W.gz};
+    const S ni = smax(cn, z);
+    const S limit = smax(friction, z) * ni;
+    const S tlsq = c1 * c1 + c2 * c2;
+    const S scale = val(tlsq) > val(limit * limit) ? limit / ssqrt(tlsq) : ADL(S, 1.0f);
+    l0 = ni;
+    l1 = c1 * scale;
+    l2 = c2 * scale;
+}
+template <class S>
+AD_HD V3<S> warmClampReverse(const S &mu, const S &cn, const S &c1, const S &c2, const V3<S> &alam, S &amu) {
+    const S z = S(0);
+    const S ni = smax(cn, z);
+    const S mu0 = smax(mu, z);
+    const S limit = mu0 * ni;
+    const S tlsq = c1 * c1 + c2 * c2;
+    S ani = alam.x;
+    const S af1 = alam.y, af2 = alam.z;
+    S ac1 = af1, ac2 = af2;
+    if (tlsq > limit * limit) {
+        const S L = ssqrt(tlsq);
+        const S u1 = c1 / L, u2 = c2 / L;
+        const S ua = u1 * af1 + u2 * af2;
+        ac1 = (limit / L) * (af1 - u1 * ua);
+        ac2 = (limit / L) * (af2 - u2 * ua);
+        ani = ani + ua * mu0;
+        if (!(mu < z)) amu = amu + ua * ni;
+    }
+    return {(cn < z) ? z : ani, ac1, ac2};
+}
+
+// The warm start's application of one matched point in reverse (the body
+// adjoints pass through): adjoints of the initial impulses, of the prepared
+// constants, of the normal and of the inverse masses and inertias are added to.
+template <class S>
+AD_HD void warmReverse(const V3<S> &n, const S *pp, const V3<S> &lam, const M3<S> &IA, const M3<S> &IB, const S &imA,
+                       const S &imB, bool sA, bool sB, const V3<S> &avA, const V3<S> &awA, const V3<S> &avB,
+                       const V3<S> &awB, V3<S> &alam, S *ac, V3<S> &an, M3<S> &aIA, M3<S> &aIB, S &aimA, S &aimB) {
+    const S z = S(0);
+    const V3<S> t1 = pv(pp, kPT1), t2 = pv(pp, kPT2), offA = pv(pp, kPOffA), offB = pv(pp, kPOffB);
+    const V3<S> wi = n * lam.x + t1 * lam.y + t2 * lam.z;
+    const V3<S> nw = -wi;
+    V3<S> awi{z, z, z};
+    auto acc3 = [&](int f, const V3<S> &v) {
+        ac[3 * f] = ac[3 * f] + v.x;
+        ac[3 * f + 1] = ac[3 * f + 1] + v.y;
+        ac[3 * f + 2] = ac[3 * f + 2] + v.z;
+    };
+    if (!sB) {
+        awi += avB * imB;
+        aimB = aimB + dot(avB, wi);
+        V3<S> ay{z, z, z}, aoff{z, z, z};
+        mulAdj(IB, cross(offB, wi), awB, aIB, ay);
+        crossAdj(offB, wi, ay, aoff, awi);
+        acc3(kPOffB, aoff);
+    }
+    if (!sA) {
+        V3<S> anw = avA * imA;
+        aimA = aimA + dot(avA, nw);
+        V3<S> ay{z, z, z}, aoff{z, z, z};
+        mulAdj(IA, cross(offA, nw), awA, aIA, ay);
+        crossAdj(offA, nw, ay, aoff, anw);
+        acc3(kPOffA, aoff);
+        awi += -anw;
+    }
+    alam.x = alam.x + dot(awi, n);
+    alam.y = alam.y + dot(awi, t1);
+    alam.z = alam.z + dot(awi, t2);
+    an += awi * lam.x;
+    acc3(kPT1, awi * lam.y);
+    acc3(kPT2, awi * lam.z);
+}
+
+// --------------------------------------- one host thread: forward, reverse --
+#if !defined(__CUDACC__)
+template <class S>
+inline void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const CacheView<S> &cin, StateView<S> out,
+                       CacheView<S> cout, StepScratch<S> sc, bool record) {
+    const uint32_t n = W.n;
+    const S z = ADL(S, 0.0f);
     // 1. velocity integration (RigidBody::integrateVelocity, no applied force) and AABBs
-    for (uint32_t i = tid; i < n; i += nt) {
-        V3<S> v = ld3(in.v, i);
-        const bool st = W.isStatic[i] != 0;
-        if (!st) {
-            const V3<S> f{z, z, z};
-            const V3<S> acc = g + f * inverseMass(false, W.mass[i]);
-            v += acc * W.dt;
-        }
-        st3(out.v, i, v);
+    for (uint32_t i = 0; i < n; ++i) {
+        st3(out.v, i, integratedVelocity(W, i, ld3(in.v, i)));
         st3(out.w, i, ld3(in.w, i));
-        const V3<S> p = ld3(in.x, i);
-        const Q<S> q = ld4q(in.q, i);
         V3<S> mn, mx;
-        if (W.shape[i] == 0) {
-            const S r = W.dims[3 * i];
-            const V3<S> rr{r, r, r};
-            mn = p - rr;
-            mx = p + rr;
-        } else {
-            const M3<S> m = toMat3(q);
-            const S hx = W.dims[3 * i], hy = W.dims[3 * i + 1], hz = W.dims[3 * i + 2];
-            const V3<S> e{sabs(m.m00) * hx + sabs(m.m01) * hy + sabs(m.m02) * hz,
-                          sabs(m.m10) * hx + sabs(m.m11) * hy + sabs(m.m12) * hz,
-                          sabs(m.m20) * hx + sabs(m.m21) * hy + sabs(m.m22) * hz};
-            mn = p - e;
-            mx = p + e;
-        }
+        bodyAabb(W, i, ld3(in.x, i), ld4q(in.q, i), mn, mx);
         st3(sc.aabb, 2 * i, mn);
         st3(sc.aabb, 2 * i + 1, mx);
     }
-    if (tid == 0) {
-        sc.counts[0] = 0;
-        sc.counts[1] = 0;
-        sc.counts[3] = 0;
-    }
-    T::sync();
+    sc.counts[0] = sc.counts[1] = sc.counts[3] = 0;
     // 2. every pair (i < j) with overlapping AABBs (touching counts), in
     // lexicographic order: sort and sweep along x (broadphase.cpp:195-291) —
     // bodies sorted by min.x, each tested against the later ones whose min.x
     // does not exceed its max.x (the one of an overlapping pair sorted first
     // always meets the other) — then the pairs sorted by (first, second).
-    const uint32_t n2 = nextPow2u(n > 0 ? n : 1);
-    for (uint32_t i = tid; i < n2; i += nt)
-        sc.bpEntries[i] = i < n ? ((unsigned long long)adOrderedKey(val(sc.aabb[6 * i])) << 32) | i : ~0ull;
-    T::sync();
-    T::sortU64(sc.bpEntries, n2);
-    T::sync();
+    for (uint32_t i = 0; i < n; ++i)
+        sc.bpEntries[i] = ((unsigned long long)adOrderedKey(val(sc.aabb[6 * i])) << 32) | i;
+    std::sort(sc.bpEntries, sc.bpEntries + n);
     auto overlapsYZ = [&](uint32_t a, uint32_t b) {
         const V3<S> amn = ld3(sc.aabb, 2 * a), amx = ld3(sc.aabb, 2 * a + 1);
         const V3<S> bmn = ld3(sc.aabb, 2 * b), bmx = ld3(sc.aabb, 2 * b + 1);
@@ -487,97 +565,57 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
                val(amx.z) >= val(bmn.z);
     };
     uint32_t P = 0;
-    for (uint32_t k0 = 0; k0 < n; k0 += nt) {
-        const uint32_t k = k0 + tid;
-        uint32_t hits = 0;
-        uint32_t i = 0;
-        if (k < n) {
-            i = (uint32_t)sc.bpEntries[k];
-            const auto maxX = val(sc.aabb[6 * i + 3]);
-            for (uint32_t kk = k + 1; kk < n; ++kk) {
-                const uint32_t j = (uint32_t)sc.bpEntries[kk];
-                if (val(sc.aabb[6 * j]) > maxX) break;
-                if (overlapsYZ(i, j)) ++hits;
-            }
+    for (uint32_t k = 0; k < n; ++k) {
+        const uint32_t i = (uint32_t)sc.bpEntries[k];
+        const auto maxX = val(sc.aabb[6 * i + 3]);
+        for (uint32_t kk = k + 1; kk < n; ++kk) {
+            const uint32_t j = (uint32_t)sc.bpEntries[kk];
+            if (val(sc.aabb[6 * j]) > maxX) break;
+            if (!overlapsYZ(i, j)) continue;
+            if (P < W.maxPairs) sc.bpPairs[P] = ((unsigned long long)(i < j ? i : j) << 32) | (i < j ? j : i);
+            ++P;
         }
-        uint32_t cnt;
-        uint32_t slot = P + T::scan(hits, cnt);
-        if (k < n && hits) {
-            const auto maxX = val(sc.aabb[6 * i + 3]);
-            for (uint32_t kk = k + 1; kk < n; ++kk) {
-                const uint32_t j = (uint32_t)sc.bpEntries[kk];
-                if (val(sc.aabb[6 * j]) > maxX) break;
-                if (!overlapsYZ(i, j)) continue;
-                if (slot < W.maxPairs)
-                    sc.bpPairs[slot] = ((unsigned long long)(i < j ? i : j) << 32) | (i < j ? j : i);
-                ++slot;
-            }
-        }
-        P += cnt;
     }
     if (P > W.maxPairs) {
-        if (tid == 0) T::orErr(&sc.counts[3], kAdErrPairs);
+        sc.counts[3] |= kAdErrPairs;
         P = W.maxPairs;
     }
-    const uint32_t P2 = nextPow2u(P > 0 ? P : 1);
-    for (uint32_t p = P + tid; p < P2; p += nt) sc.bpPairs[p] = ~0ull;
-    T::sync();
-    T::sortU64(sc.bpPairs, P2);
-    T::sync();
-    for (uint32_t p = tid; p < P; p += nt) {
-        sc.pairA[p] = (uint32_t)(sc.bpPairs[p] >> 32);
-        sc.pairB[p] = (uint32_t)sc.bpPairs[p];
-    }
-    if (tid == 0) sc.counts[0] = P;
-    T::sync();
+    std::sort(sc.bpPairs, sc.bpPairs + P);
+    sc.counts[0] = P;
     // 3. narrowphase in pair order, manifolds compacted in that order
     uint32_t M = 0;
-    for (uint32_t t0 = 0; t0 < P; t0 += nt) {
-        const uint32_t p = t0 + tid;
-        Contact<S> c;
-        c.count = 0;
-        bool hit = false;
-        uint32_t a = 0, b = 0;
-        if (p < P) {
-            a = sc.pairA[p];
-            b = sc.pairB[p];
-            const Tf<S> tA{ld3(in.x, a), ld4q(in.q, a)}, tB{ld3(in.x, b), ld4q(in.q, b)};
-            hit = contactPair<S>(W.shape[a], ld3(W.dims, a), tA, W.shape[b], ld3(W.dims, b), tB, c);
+    for (uint32_t p = 0; p < P; ++p) {
+        const uint32_t a = (uint32_t)(sc.bpPairs[p] >> 32), b = (uint32_t)sc.bpPairs[p];
+        Contact<S> c{};
+        const Tf<S> tA{ld3(in.x, a), ld4q(in.q, a)}, tB{ld3(in.x, b), ld4q(in.q, b)};
+        if (!contactPair<S>(W.shape[a], ld3(W.dims, a), tA, W.shape[b], ld3(W.dims, b), tB, c)) continue;
+        const uint32_t m = M++;
+        if (m >= W.maxManifolds) continue;
+        sc.mA[m] = a;
+        sc.mB[m] = b;
+        sc.mCount[m] = c.count;
+        st3(sc.mNormal, m, c.normal);
+        sc.mRest[m] = smax(W.rest[a], W.rest[b]);
+        sc.mMu[m] = ssqrt(smax(W.mu[a], z) * smax(W.mu[b], z));
+        for (uint32_t k = 0; k < 4; ++k) {
+            const bool live = k < c.count;
+            st3(sc.mAnchorA, 4 * m + k, live ? c.anchorA[k] : V3<S>{z, z, z});
+            st3(sc.mAnchorB, 4 * m + k, live ? c.anchorB[k] : V3<S>{z, z, z});
+            sc.mDepth[4 * m + k] = live ? c.depth[k] : z;
+            sc.mFeature[4 * m + k] = live ? c.feature[k] | (c.axis << kAdAxisShift) : 0u;
         }
-        uint32_t cnt;
-        const uint32_t m = M + T::scan(hit ? 1u : 0u, cnt);
-        if (hit && m < W.maxManifolds) {
-            sc.mA[m] = a;
-            sc.mB[m] = b;
-            sc.mCount[m] = c.count;
-            st3(sc.mNormal, m, c.normal);
-            sc.mRest[m] = smax(W.rest[a], W.rest[b]);
-            sc.mMu[m] = ssqrt(smax(W.mu[a], z) * smax(W.mu[b], z));
-            for (uint32_t k = 0; k < 4; ++k) {
-                const bool live = k < c.count;
-                st3(sc.mAnchorA, 4 * m + k, live ? c.anchorA[k] : V3<S>{z, z, z});
-                st3(sc.mAnchorB, 4 * m + k, live ? c.anchorB[k] : V3<S>{z, z, z});
-                sc.mDepth[4 * m + k] = live ? c.depth[k] : z;
-                sc.mFeature[4 * m + k] = live ? c.feature[k] : 0u;
-            }
-        }
-        M += cnt;
     }
     if (M > W.maxManifolds) {
-        if (tid == 0) T::orErr(&sc.counts[3], kAdErrManifolds);
+        sc.counts[3] |= kAdErrManifolds;
         M = W.maxManifolds;
     }
-    if (tid == 0) sc.counts[1] = M;
+    sc.counts[1] = M;
     // 4. colouring: greedy in decreasing priority over manifolds that share a
     // dynamic body (the engine's colouring), then order = (colour, index)
-    const uint32_t M2 = nextPow2u(M > 0 ? M : 1);
-    for (uint32_t i = tid; i < M2; i += nt)
-        sc.sortKeys[i] = i < M ? ((unsigned long long)(~adColorPriority(i)) << 32) | i : ~0ull;
-    for (uint32_t i = tid; i < 2 * n; i += nt) sc.bodyUsed[i] = 0ull;
-    T::sync();
-    T::sortU64(sc.sortKeys, M2);
-    T::sync();
-    if (tid == 0) {
+    for (uint32_t i = 0; i < M; ++i) sc.sortKeys[i] = ((unsigned long long)(~adColorPriority(i)) << 32) | i;
+    for (uint32_t i = 0; i < 2 * n; ++i) sc.bodyUsed[i] = 0ull;
+    std::sort(sc.sortKeys, sc.sortKeys + M);
+    {
         // Colour windows of kAdMaxColors: a manifold whose higher-priority
         // neighbours use the whole window waits for the next window, in which
         // only the waiting manifolds take colours (the engine's rule, so the
@@ -625,25 +663,20 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
         }
         sc.counts[2] = colors;
     }
-    T::sync();
-    for (uint32_t i = tid; i < M2; i += nt)
-        sc.sortKeys[i] = i < M ? ((unsigned long long)sc.color[i] << 32) | i : ~0ull;
-    T::sync();
-    T::sortU64(sc.sortKeys, M2);
-    T::sync();
+    for (uint32_t i = 0; i < M; ++i) sc.sortKeys[i] = ((unsigned long long)sc.color[i] << 32) | i;
+    std::sort(sc.sortKeys, sc.sortKeys + M);
     const uint32_t C = sc.counts[2];
-    for (uint32_t k = tid; k < M; k += nt) {
+    for (uint32_t k = 0; k < M; ++k) {
         sc.order[k] = (uint32_t)sc.sortKeys[k];
         const uint32_t ck = (uint32_t)(sc.sortKeys[k] >> 32);
         const uint32_t cp = k == 0 ? 0xFFFFFFFFu : (uint32_t)(sc.sortKeys[k - 1] >> 32);
         for (uint32_t c = (k == 0 ? 0 : cp + 1); c <= ck; ++c) sc.colorStart[c] = k;
     }
-    if (tid == 0) sc.colorStart[C] = M;
-    T::sync();
+    sc.colorStart[C] = M;
     // 5. prepare + warm-start matching (sequential_impulse_solver.cpp:101-214, :448-490)
     const S inverseDt = ADL(S, 1.0f) / smax(W.dt, ADL(S, 1e-6f));
     const uint32_t cacheN = *cin.count;
-    for (uint32_t k = tid; k < M; k += nt) {
+    for (uint32_t k = 0; k < M; ++k) {
         const uint32_t m = sc.order[k];
         const uint32_t a = sc.mA[m], b = sc.mB[m];
         const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
@@ -690,13 +723,7 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
                         const V3<S> da = ld3(cin.anchorA, e) - anA, db = ld3(cin.anchorB, e) - anB;
                         if (val(dot(da, da)) > matchSq || val(dot(db, db)) > matchSq) continue;
                         const S cn = cin.lam[3 * e], c1 = cin.lam[3 * e + 1], c2 = cin.lam[3 * e + 2];
-                        const S ni = smax(cn, z);
-                        const S limit = smax(friction, z) * ni;
-                        const S tlsq = c1 * c1 + c2 * c2;
-                        const S scale = val(tlsq) > val(limit * limit) ? limit / ssqrt(tlsq) : ADL(S, 1.0f);
-                        l0 = ni;
-                        l1 = c1 * scale;
-                        l2 = c2 * scale;
+                        warmClamp(friction, cn, c1, c2, l0, l1, l2);
                         match = (int32_t)e;
                         break;
                     }
@@ -708,10 +735,9 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
             sc.lamInit[3 * kp + 2] = sc.lam[3 * kp + 2] = l2;
         }
     }
-    T::sync();
     // 6. warm start, colour by colour (warmStartPrepared :453-490)
     for (uint32_t c = 0; c < C; ++c) {
-        for (uint32_t k = sc.colorStart[c] + tid; k < sc.colorStart[c + 1]; k += nt) {
+        for (uint32_t k = sc.colorStart[c]; k < sc.colorStart[c + 1]; ++k) {
             const uint32_t m = sc.order[k];
             const uint32_t a = sc.mA[m], b = sc.mB[m];
             const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
@@ -747,12 +773,11 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
                 st3(out.w, b, angB);
             }
         }
-        T::sync();
     }
     // 7. velocity iterations in colour order, with the tape of each manifold update
     for (int it = 0; it < W.iterations; ++it)
         for (uint32_t c = 0; c < C; ++c) {
-            for (uint32_t k = sc.colorStart[c] + tid; k < sc.colorStart[c + 1]; k += nt) {
+            for (uint32_t k = sc.colorStart[c]; k < sc.colorStart[c + 1]; ++k) {
                 const uint32_t m = sc.order[k];
                 const uint32_t a = sc.mA[m], b = sc.mB[m];
                 const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
@@ -786,22 +811,16 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
                     st3(out.w, b, s.wB);
                 }
             }
-            T::sync();
         }
     // 8. cache rebuild: entries sorted by (body A, body B), stable in solve order (:623-681)
-    for (uint32_t i = tid; i < M2; i += nt) {
-        unsigned long long key = ~0ull;
-        if (i < M) {
-            const uint32_t m = sc.order[i];
-            key = ((unsigned long long)sc.mA[m] << 44) | ((unsigned long long)sc.mB[m] << 24) | i;
-        }
-        sc.sortKeys[i] = key;
+    for (uint32_t i = 0; i < M; ++i) {
+        const uint32_t m = sc.order[i];
+        sc.sortKeys[i] = ((unsigned long long)sc.mA[m] << 44) | ((unsigned long long)sc.mB[m] << 24) | i;
     }
-    T::sync();
-    T::sortU64(sc.sortKeys, M2);
-    T::sync();
-    if (tid == 0) {
+    std::sort(sc.sortKeys, sc.sortKeys + M);
+    {
         uint32_t e = 0;
+        for (uint32_t kp = 0; kp < 4 * M; ++kp) sc.cacheSlot[kp] = kNoSlot;
         for (uint32_t r = 0; r < M; ++r) {
             const uint32_t k = (uint32_t)(sc.sortKeys[r] & 0xFFFFFFu);
             const uint32_t m = sc.order[k];
@@ -817,164 +836,49 @@ AD_HD void forwardStep(const WorldParams<S> &W, const StateView<S> &in, const Ca
                 cout.lam[3 * e] = sc.lam[3 * kp];
                 cout.lam[3 * e + 1] = sc.lam[3 * kp + 1];
                 cout.lam[3 * e + 2] = sc.lam[3 * kp + 2];
-                sc.cacheSrc[e] = (uint32_t)kp;
+                sc.cacheSlot[kp] = e;
             }
         }
         *cout.count = e < cout.cap ? e : cout.cap;
     }
     // 9. pose integration (rigid_body.cpp:103-125)
-    for (uint32_t i = tid; i < n; i += nt) {
+    for (uint32_t i = 0; i < n; ++i) {
         V3<S> pos = ld3(in.x, i);
         Q<S> rot = ld4q(in.q, i);
-        if (!W.isStatic[i]) {
-            const V3<S> lin = ld3(out.v, i), ang = ld3(out.w, i);
-            pos += lin * W.dt;
-            const Q<S> spin{ang.x, ang.y, ang.z, z};
-            const Q<S> d = qmul(spin, rot);
-            const S h = ADL(S, 0.5f) * W.dt;
-            rot.x = rot.x + h * d.x;
-            rot.y = rot.y + h * d.y;
-            rot.z = rot.z + h * d.z;
-            rot.w = rot.w + h * d.w;
-            rot = qnormalized(rot);
-        }
+        if (!W.isStatic[i]) poseForward(W.dt, ld3(out.v, i), ld3(out.w, i), pos, rot);
         st3(out.x, i, pos);
         st4q(out.q, i, rot);
     }
-    T::sync();
 }
 
 // ------------------------------------------------------------------ reverse --
-// Contact geometry + preparation of manifold k as a function of the 29 inputs,
-// evaluated in dual numbers for directions [base, base + kDualChunk); returns
-// the directional derivatives of sum(adjoint * output) in g[].
 template <class S>
-AD_HDN bool manifoldDualChunk(const WorldParams<S> &W, const StateView<S> &in, const StateView<S> &v1,
-                             const StepScratch<S> &sc, const AdjointView<S> &adj, uint32_t k, int base, S *g) {
-    using D = Dual<S, kDualChunk>;
-    const uint32_t m = sc.order[k];
-    const uint32_t a = sc.mA[m], b = sc.mB[m];
-    const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
-    auto seed = [&](S value, int dir) {
-        D r = dconst<S, kDualChunk>(value);
-        const int j = dir - base;
-        if (j >= 0 && j < kDualChunk) r.d[j] = S(1);
-        return r;
-    };
-    auto seed3 = [&](const S *p, uint32_t i, int dir) {
-        return V3<D>{seed(p[3 * i], dir), seed(p[3 * i + 1], dir + 1), seed(p[3 * i + 2], dir + 2)};
-    };
-    auto c3 = [&](const S *p, uint32_t i) {
-        return V3<D>{dconst<S, kDualChunk>(p[3 * i]), dconst<S, kDualChunk>(p[3 * i + 1]),
-                     dconst<S, kDualChunk>(p[3 * i + 2])};
-    };
-    const V3<D> xA = seed3(in.x, a, 0), xB = seed3(in.x, b, 7);
-    const Q<D> qA{seed(in.q[4 * a], 3), seed(in.q[4 * a + 1], 4), seed(in.q[4 * a + 2], 5), seed(in.q[4 * a + 3], 6)};
-    const Q<D> qB{seed(in.q[4 * b], 10), seed(in.q[4 * b + 1], 11), seed(in.q[4 * b + 2], 12),
-                  seed(in.q[4 * b + 3], 13)};
-    const V3<D> linA = seed3(v1.v, a, 14), angA = seed3(v1.w, a, 17), linB = seed3(v1.v, b, 20),
-                angB = seed3(v1.w, b, 23);
-    const D mA = seed(W.mass[a], 26), mB = seed(W.mass[b], 27), rest = seed(sc.mRest[m], 28);
-    Contact<D> c;
-    const bool hit = contactPair<D>(W.shape[a], c3(W.dims, a), Tf<D>{xA, qA}, W.shape[b], c3(W.dims, b),
-                                    Tf<D>{xB, qB}, c);
-    bool ok = hit && c.count == sc.mCount[m];
-    for (uint32_t p = 0; ok && p < c.count; ++p) ok = c.feature[p] == sc.mFeature[4 * m + p];
-    if (!ok) return false;
-    const M3<D> IA = inverseInertiaWorld(qA, dconst<S, kDualChunk>(W.iinv[3 * a]),
-                                         dconst<S, kDualChunk>(W.iinv[3 * a + 1]),
-                                         dconst<S, kDualChunk>(W.iinv[3 * a + 2]));
-    const M3<D> IB = inverseInertiaWorld(qB, dconst<S, kDualChunk>(W.iinv[3 * b]),
-                                         dconst<S, kDualChunk>(W.iinv[3 * b + 1]),
-                                         dconst<S, kDualChunk>(W.iinv[3 * b + 2]));
-    const D imA = inverseMass(sA, mA), imB = inverseMass(sB, mB);
-    const D inverseDt = ADL(D, 1.0f) / smax(dconst<S, kDualChunk>(W.dt), ADL(D, 1e-6f));
-    for (int j = 0; j < kDualChunk; ++j) g[j] = S(0);
-    auto acc = [&](const D &o, S adjv) {
-        for (int j = 0; j < kDualChunk; ++j) g[j] = g[j] + adjv * o.d[j];
-    };
-    const S *apm = adj.apm + (size_t)k * kPmScalars;
-    const D *ia = &IA.m00, *ib = &IB.m00;
-    for (int e = 0; e < 9; ++e) {
-        acc(ia[e], apm[e]);
-        acc(ib[e], apm[9 + e]);
-    }
-    acc(imA, apm[18]);
-    acc(imB, apm[19]);
-    acc(c.normal.x, adj.an[3 * k]);
-    acc(c.normal.y, adj.an[3 * k + 1]);
-    acc(c.normal.z, adj.an[3 * k + 2]);
-    for (uint32_t p = 0; p < c.count; ++p) {
-        Prepared<D> pr;
-        preparePoint(c.normal, c.anchorA[p], c.anchorB[p], c.depth[p], qA, qB, IA, IB, imA, imB, linA, angA, linB,
-                     angB, rest, inverseDt, pr);
-        D flat[kPreparedScalars];
-        preparedPack(pr, flat);
-        const S *ac = adj.app + ((size_t)k * 4 + p) * kPreparedScalars;
-        for (int e = 0; e < kPreparedScalars; ++e) acc(flat[e], ac[e]);
-    }
-    return true;
-}
-
-template <class S, class T>
-AD_HD void backwardStep(const WorldParams<S> &W, const StateView<S> &in, const CacheView<S> &cin,
-                        const StateView<S> &out, StateView<S> v1, const StepScratch<S> &sc, AdjointView<S> adj) {
-    const uint32_t tid = T::tid(), nt = T::size(), n = W.n;
+inline void backwardStep(const WorldParams<S> &W, const StateView<S> &in, const CacheView<S> &cin,
+                         const StateView<S> &out, const StepScratch<S> &sc, AdjointView<S> adj) {
+    const uint32_t n = W.n;
     const S z = S(0);
     const uint32_t M = sc.counts[1], C = sc.counts[2];
     // clear the per-step adjoints of constants
-    for (uint32_t i = tid; i < M * 4 * kPreparedScalars; i += nt) adj.app[i] = z;
-    for (uint32_t i = tid; i < M * kPmScalars; i += nt) adj.apm[i] = z;
-    for (uint32_t i = tid; i < 3 * M; i += nt) adj.an[i] = z;
-    for (uint32_t i = tid; i < M; i += nt) adj.amuM[i] = adj.arestM[i] = z;
-    for (uint32_t i = tid; i < 3 * (*cin.count); i += nt) adj.acache[i] = z;
-    // velocities after gravity (the prepare step's input), for the dual pass
-    const V3<S> g{W.gx, W.gy, W.gz};
-    for (uint32_t i = tid; i < n; i += nt) {
-        V3<S> v = ld3(in.v, i);
-        if (!W.isStatic[i]) {
-            const V3<S> f{z, z, z};
-            const V3<S> acc = g + f * inverseMass(false, W.mass[i]);
-            v += acc * W.dt;
-        }
-        st3(v1.v, i, v);
-        st3(v1.w, i, ld3(in.w, i));
-    }
+    for (uint32_t i = 0; i < M * 4 * kPreparedScalars; ++i) adj.app[i] = z;
+    for (uint32_t i = 0; i < M * kPmScalars; ++i) adj.apm[i] = z;
+    for (uint32_t i = 0; i < 3 * M; ++i) adj.an[i] = z;
+    for (uint32_t i = 0; i < M; ++i) adj.amuM[i] = z;
+    for (uint32_t i = 0; i < 3 * (*cin.count); ++i) adj.acache[i] = z;
     // 1. pose integration
-    for (uint32_t i = tid; i < n; i += nt) {
+    for (uint32_t i = 0; i < n; ++i) {
         if (W.isStatic[i]) continue;
-        const V3<S> ax1 = ld3(adj.ax, i);
-        const Q<S> aq1 = ld4q(adj.aq, i);
+        Q<S> aq = ld4q(adj.aq, i);
         V3<S> av = ld3(adj.av, i), aw = ld3(adj.aw, i);
-        av += ax1 * W.dt;
-        const Q<S> rot = ld4q(in.q, i);
-        const V3<S> ang = ld3(out.w, i);
-        const Q<S> spin{ang.x, ang.y, ang.z, z};
-        const Q<S> d = qmul(spin, rot);
-        const S h = S(0.5f) * W.dt;
-        const Q<S> u{rot.x + h * d.x, rot.y + h * d.y, rot.z + h * d.z, rot.w + h * d.w};
-        const S len = ssqrt(u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w);
-        Q<S> au{z, z, z, z};
-        if (len != z) {
-            const Q<S> q1{u.x / len, u.y / len, u.z / len, u.w / len};
-            const S qa = q1.x * aq1.x + q1.y * aq1.y + q1.z * aq1.z + q1.w * aq1.w;
-            au = Q<S>{(aq1.x - q1.x * qa) / len, (aq1.y - q1.y * qa) / len, (aq1.z - q1.z * qa) / len,
-                      (aq1.w - q1.w * qa) / len};
-        }
-        Q<S> arot = au, aspin{z, z, z, z};
-        const Q<S> ad{h * au.x, h * au.y, h * au.z, h * au.w};
-        qmulAdj(spin, rot, ad, aspin, arot);
-        aw += V3<S>{aspin.x, aspin.y, aspin.z};
+        poseReverse(W.dt, ld4q(in.q, i), ld3(out.w, i), ld3(adj.ax, i), aq, av, aw);
         st3(adj.av, i, av);
         st3(adj.aw, i, aw);
-        st4q(adj.aq, i, arot);
+        st4q(adj.aq, i, aq);
     }
-    T::sync();
     // 2. velocity iterations in reverse
     for (int it = W.iterations - 1; it >= 0; --it)
         for (int ci = (int)C - 1; ci >= 0; --ci) {
             const uint32_t c = (uint32_t)ci;
-            for (uint32_t k = sc.colorStart[c] + tid; k < sc.colorStart[c + 1]; k += nt) {
+            for (uint32_t k = sc.colorStart[c]; k < sc.colorStart[c + 1]; ++k) {
                 const uint32_t m = sc.order[k];
                 const uint32_t a = sc.mA[m], b = sc.mB[m];
                 const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
@@ -1000,11 +904,14 @@ AD_HD void backwardStep(const WorldParams<S> &W, const StateView<S> &in, const C
                 S aimA = apm[18], aimB = apm[19];
                 for (int p = (int)npts - 1; p >= 0; --p) {
                     const size_t kp = (size_t)k * 4 + p;
+                    const S *c = sc.pp + kp * kPreparedScalars;
                     ab.ln = adj.alam[3 * kp];
                     ab.l1 = adj.alam[3 * kp + 1];
                     ab.l2 = adj.alam[3 * kp + 2];
-                    pointReverse(n3, mu, sc.pp + kp * kPreparedScalars, pm[18], pm[19], sA, sB, ins[p], ab,
-                                 adj.app + kp * kPreparedScalars, an, amu, aimA, aimB);
+                    const PointMid<S> mid = pointMid(n3, mu, c, ins[p]);
+                    const PointAdj<S> r = pointChain(n3, c, pm[18], pm[19], sA, sB, mid, ab);
+                    pointAccumulate(n3, mu, c, ins[p], sA, sB, mid, r, adj.app + kp * kPreparedScalars, an, amu, aimA,
+                                    aimB);
                     adj.alam[3 * kp] = ab.ln;
                     adj.alam[3 * kp + 1] = ab.l1;
                     adj.alam[3 * kp + 2] = ab.l2;
@@ -1022,165 +929,89 @@ AD_HD void backwardStep(const WorldParams<S> &W, const StateView<S> &in, const C
                     st3(adj.aw, b, ab.wB);
                 }
             }
-            T::sync();
         }
-    // 3. warm start in reverse (additive: body adjoints pass through)
-    for (uint32_t k = tid; k < M; k += nt) {
+    // 3. warm start and its matching, 4. preparation, 5. contact geometry, 6. materials.
+    // The preparation's velocity adjoints wait until every warm start has read
+    // the body adjoints.
+    std::vector<V3<S>> dv(n, V3<S>{z, z, z}), dw(n, V3<S>{z, z, z});
+    const S inverseDt = S(1) / smax(W.dt, ADL(S, 1e-6f));
+    for (uint32_t k = 0; k < M; ++k) {
         const uint32_t m = sc.order[k];
         const uint32_t a = sc.mA[m], b = sc.mB[m];
         const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
         const S *pm = sc.pm + (size_t)k * kPmScalars;
-        S *apm = adj.apm + (size_t)k * kPmScalars;
+        const S *apm = adj.apm + (size_t)k * kPmScalars;
         const M3<S> IA = ldm(pm), IB = ldm(pm + 9);
         const V3<S> n3 = ld3(sc.mNormal, m);
         const V3<S> avA = ld3(adj.av, a), awA = ld3(adj.aw, a), avB = ld3(adj.av, b), awB = ld3(adj.aw, b);
-        V3<S> an = ld3(adj.an, k);
+        const S mu = sc.mMu[m], rest = sc.mRest[m];
+        const Tf<S> tA{ld3(in.x, a), ld4q(in.q, a)}, tB{ld3(in.x, b), ld4q(in.q, b)};
+        const V3<S> linA = integratedVelocity(W, a, ld3(in.v, a)), angA = ld3(in.w, a);
+        const V3<S> linB = integratedVelocity(W, b, ld3(in.v, b)), angB = ld3(in.w, b);
+        S amu = adj.amuM[k];
+        PrepareGrad<S> g{};
+        g.n = ld3(adj.an, k);
+        g.imA = apm[18];
+        g.imB = apm[19];
+        Tf<S> gA{{z, z, z}, {z, z, z, z}}, gB = gA;
+        V3<S> gn{z, z, z};
         for (uint32_t p = 0; p < sc.mCount[m]; ++p) {
             const size_t kp = (size_t)k * 4 + p;
-            if (sc.match[kp] < 0) continue;
             const S *pp = sc.pp + kp * kPreparedScalars;
             S *ac = adj.app + kp * kPreparedScalars;
-            const S ln = sc.lamInit[3 * kp], l1 = sc.lamInit[3 * kp + 1], l2 = sc.lamInit[3 * kp + 2];
-            const V3<S> t1 = pv(pp, kPT1), t2 = pv(pp, kPT2), offA = pv(pp, kPOffA), offB = pv(pp, kPOffB);
-            const V3<S> wi = n3 * ln + t1 * l1 + t2 * l2;
-            const V3<S> nw = -wi;
-            V3<S> awi{z, z, z};
-            if (!sB) {
-                awi += avB * pm[19];
-                apm[19] = apm[19] + dot(avB, wi);
-                const V3<S> y = cross(offB, wi);
-                const V3<S> ay = mul(transpose(IB), awB);
-                const S *yy = &y.x;
-                const S *aww = &awB.x;
-                for (int r = 0; r < 3; ++r)
-                    for (int cc = 0; cc < 3; ++cc) apm[9 + 3 * r + cc] = apm[9 + 3 * r + cc] + aww[r] * yy[cc];
-                V3<S> aoff{z, z, z};
-                crossAdj(offB, wi, ay, aoff, awi);
-                ac[3 * kPOffB] = ac[3 * kPOffB] + aoff.x;
-                ac[3 * kPOffB + 1] = ac[3 * kPOffB + 1] + aoff.y;
-                ac[3 * kPOffB + 2] = ac[3 * kPOffB + 2] + aoff.z;
-            }
-            if (!sA) {
-                V3<S> anw = avA * pm[18];
-                apm[18] = apm[18] + dot(avA, nw);
-                const V3<S> y = cross(offA, nw);
-                const V3<S> ay = mul(transpose(IA), awA);
-                const S *yy = &y.x;
-                const S *aww = &awA.x;
-                for (int r = 0; r < 3; ++r)
-                    for (int cc = 0; cc < 3; ++cc) apm[3 * r + cc] = apm[3 * r + cc] + aww[r] * yy[cc];
-                V3<S> aoff{z, z, z};
-                crossAdj(offA, nw, ay, aoff, anw);
-                ac[3 * kPOffA] = ac[3 * kPOffA] + aoff.x;
-                ac[3 * kPOffA + 1] = ac[3 * kPOffA + 1] + aoff.y;
-                ac[3 * kPOffA + 2] = ac[3 * kPOffA + 2] + aoff.z;
-                awi += -anw;
-            }
-            adj.alam[3 * kp] = adj.alam[3 * kp] + dot(awi, n3);
-            adj.alam[3 * kp + 1] = adj.alam[3 * kp + 1] + dot(awi, t1);
-            adj.alam[3 * kp + 2] = adj.alam[3 * kp + 2] + dot(awi, t2);
-            an += awi * ln;
-            ac[3 * kPT1] = ac[3 * kPT1] + awi.x * l1;
-            ac[3 * kPT1 + 1] = ac[3 * kPT1 + 1] + awi.y * l1;
-            ac[3 * kPT1 + 2] = ac[3 * kPT1 + 2] + awi.z * l1;
-            ac[3 * kPT2] = ac[3 * kPT2] + awi.x * l2;
-            ac[3 * kPT2 + 1] = ac[3 * kPT2 + 1] + awi.y * l2;
-            ac[3 * kPT2 + 2] = ac[3 * kPT2 + 2] + awi.z * l2;
-        }
-        st3(adj.an, k, an);
-        // 4. warm-start matching: lambda_init from the previous step's impulses
-        const S mu = sc.mMu[m];
-        S amu = adj.amuM[k];
-        for (uint32_t p = 0; p < sc.mCount[m]; ++p) {
-            const size_t kp = (size_t)k * 4 + p;
             const int32_t e = sc.match[kp];
-            if (e < 0) continue;
-            const S cn = cin.lam[3 * e], c1 = cin.lam[3 * e + 1], c2 = cin.lam[3 * e + 2];
-            const S ni = smax(cn, z);
-            const S mu0 = smax(mu, z);
-            const S limit = mu0 * ni;
-            const S tlsq = c1 * c1 + c2 * c2;
-            S ani = adj.alam[3 * kp];
-            const S af1 = adj.alam[3 * kp + 1], af2 = adj.alam[3 * kp + 2];
-            S ac1 = af1, ac2 = af2;
-            if (tlsq > limit * limit) {
-                const S L = ssqrt(tlsq);
-                const S u1 = c1 / L, u2 = c2 / L;
-                const S ua = u1 * af1 + u2 * af2;
-                ac1 = (limit / L) * (af1 - u1 * ua);
-                ac2 = (limit / L) * (af2 - u2 * ua);
-                ani = ani + ua * mu0;
-                if (!(mu < z)) amu = amu + ua * ni;
+            if (e >= 0) {
+                V3<S> alam = ld3(adj.alam, (uint32_t)kp);
+                warmReverse(n3, pp, ld3(sc.lamInit, (uint32_t)kp), IA, IB, pm[18], pm[19], sA, sB, avA, awA, avB, awB,
+                            alam, ac, g.n, g.IA, g.IB, g.imA, g.imB);
+                const V3<S> o = warmClampReverse(mu, cin.lam[3 * e], cin.lam[3 * e + 1], cin.lam[3 * e + 2], alam, amu);
+                st3(adj.acache, (uint32_t)e, ld3(adj.acache, (uint32_t)e) + o);
             }
-            const S acn = (cn < z) ? z : ani;
-            T::add(&adj.acache[3 * e], acn);
-            T::add(&adj.acache[3 * e + 1], ac1);
-            T::add(&adj.acache[3 * e + 2], ac2);
+            g.anchorA = g.anchorB = V3<S>{z, z, z};
+            g.depth = z;
+            const V3<S> anchorA = ld3(sc.mAnchorA, 4 * m + p), anchorB = ld3(sc.mAnchorB, 4 * m + p);
+            preparePointReverse(n3, anchorA, anchorB, sc.mDepth[4 * m + p], tA.q, tB.q, IA, IB, pm[18] + pm[19], linA,
+                                angA, linB, angB, rest, inverseDt, pp, ac, g);
+            // a one-point manifold's normal goes with its point; the points of
+            // two boxes only add to it
+            const bool last = p + 1 == sc.mCount[m];
+            if (last) gn += g.n;
+            contactPointReverse(W.shape[a], ld3(W.dims, a), tA, W.shape[b], ld3(W.dims, b), tB, n3,
+                                sc.mFeature[4 * m + p], PointGrad<S>{g.anchorA, g.anchorB, g.depth}, gn, gA, gB);
         }
-        adj.amuM[k] = amu;
-    }
-    T::sync();
-    // 5. contact geometry + preparation (dual numbers): one (manifold, chunk of
-    // four directions) per thread; 6. materials with the last chunk
-    constexpr int kChunks = (kDualInputs + kDualChunk - 1) / kDualChunk;
-    for (uint32_t item = tid; item < M * kChunks; item += nt) {
-        const uint32_t k = item / kChunks;
-        const int chunk = (int)(item % kChunks), base = chunk * kDualChunk;
-        const uint32_t m = sc.order[k];
-        const uint32_t a = sc.mA[m], b = sc.mB[m];
-        const bool sA = W.isStatic[a] != 0, sB = W.isStatic[b] != 0;
-        S gr[kDualChunk];
-        if (!manifoldDualChunk(W, in, v1, sc, adj, k, base, gr)) {
-            T::orErr(&sc.counts[3], kAdErrReplay);
-            continue;
+        if (W.shape[a] == 1 && W.shape[b] == 1)
+            boxNormalReverse(tA, tB, (sc.mFeature[4 * m] & kAdAxisMask) >> kAdAxisShift, n3, gn, gA, gB);
+        inverseInertiaAdj(tA.q, ld3(W.iinv, a), g.IA, g.qA);
+        inverseInertiaAdj(tB.q, ld3(W.iinv, b), g.IB, g.qB);
+        auto body = [&](uint32_t i, const Tf<S> &t, const Q<S> &gq, const V3<S> &lin, const V3<S> &ang, const S &im,
+                        const S &aim) {
+            st3(adj.ax, i, ld3(adj.ax, i) + t.p);
+            const Q<S> q = ld4q(adj.aq, i);
+            st4q(adj.aq, i, Q<S>{q.x + (t.q.x + gq.x), q.y + (t.q.y + gq.y), q.z + (t.q.z + gq.z), q.w + (t.q.w + gq.w)});
+            dv[i] += lin;
+            dw[i] += ang;
+            adj.amass[i] = adj.amass[i] - aim * im * im;  // im = 1 / mass
+        };
+        if (!sA) body(a, gA, g.qA, g.linA, g.angA, pm[18], g.imA);
+        if (!sB) body(b, gB, g.qB, g.linB, g.angB, pm[19], g.imB);
+        if (W.rest[a] < W.rest[b]) {
+            if (!sB) adj.arest[b] = adj.arest[b] + g.rest;
+        } else if (!sA) {
+            adj.arest[a] = adj.arest[a] + g.rest;
         }
-        for (int j = 0; j < kDualChunk; ++j) {
-            const int d = base + j;
-            if (d >= kDualInputs) break;
-            const S gv = gr[j];
-            if (d < 3) {
-                if (!sA) T::add(&adj.ax[3 * a + d], gv);
-            } else if (d < 7) {
-                if (!sA) T::add(&adj.aq[4 * a + (d - 3)], gv);
-            } else if (d < 10) {
-                if (!sB) T::add(&adj.ax[3 * b + (d - 7)], gv);
-            } else if (d < 14) {
-                if (!sB) T::add(&adj.aq[4 * b + (d - 10)], gv);
-            } else if (d < 17) {
-                if (!sA) T::add(&adj.av[3 * a + (d - 14)], gv);
-            } else if (d < 20) {
-                if (!sA) T::add(&adj.aw[3 * a + (d - 17)], gv);
-            } else if (d < 23) {
-                if (!sB) T::add(&adj.av[3 * b + (d - 20)], gv);
-            } else if (d < 26) {
-                if (!sB) T::add(&adj.aw[3 * b + (d - 23)], gv);
-            } else if (d == 26) {
-                if (!sA) T::add(&adj.amass[a], gv);
-            } else if (d == 27) {
-                if (!sB) T::add(&adj.amass[b], gv);
-            } else {
-                // restitution = max(ra, rb)
-                const S arest = adj.arestM[k] + gv;
-                if (W.rest[a] < W.rest[b]) {
-                    if (!sB) T::add(&adj.arest[b], arest);
-                } else if (!sA) {
-                    T::add(&adj.arest[a], arest);
-                }
-            }
-        }
-        if (chunk == 0) {
-            // friction = sqrt(max(fa, 0) * max(fb, 0))
-            const S fm = sc.mMu[m];
-            if (fm > z) {
-                const S fa = smax(W.mu[a], z), fb = smax(W.mu[b], z);
-                const S amu = adj.amuM[k] * (S(0.5f) / fm);
-                if (!sA && !(W.mu[a] < z)) T::add(&adj.amu[a], amu * fb);
-                if (!sB && !(W.mu[b] < z)) T::add(&adj.amu[b], amu * fa);
-            }
+        if (mu > z) {
+            const S fa = smax(W.mu[a], z), fb = smax(W.mu[b], z);
+            const S h = amu * (S(0.5f) / mu);
+            if (!sA && !(W.mu[a] < z)) adj.amu[a] = adj.amu[a] + h * fb;
+            if (!sB && !(W.mu[b] < z)) adj.amu[b] = adj.amu[b] + h * fa;
         }
     }
-    T::sync();
+    for (uint32_t i = 0; i < n; ++i) {
+        st3(adj.av, i, ld3(adj.av, i) + dv[i]);
+        st3(adj.aw, i, ld3(adj.aw, i) + dw[i]);
+    }
 }
+#endif // host
 
 } // namespace ad
 } // namespace pe

@@ -5,15 +5,13 @@
 #include <stdexcept>
 #include <string>
 
-#include "ad_world.cuh"
+#include "ad_block.cuh"
 #include "rollout.h"
 
 namespace pe {
 namespace {
 
 using namespace ad;
-using F = float;
-
 __host__ __device__ constexpr size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
 // Byte offsets inside one world's slot of the arena.
@@ -23,10 +21,10 @@ struct Layout {
     size_t sState, sCount, sKey, sA, sB, sLam;  // within a snapshot
     // step scratch (one per step of a segment)
     size_t scr0, scrStride;
-    size_t aabb, pairA, pairB, mA, mB, mCount, mFeature, mNormal, mMu, mRest, mAnchorA, mAnchorB, mDepth, color,
-        order, sortKeys, bodyUsed, colorStart, pp, pm, lam, lamInit, match, tape, cacheSrc, counts;
+    size_t aabb, mA, mB, mCount, mFeature, mNormal, mMu, mRest, mAnchorA, mAnchorB, mDepth, color, order, rank,
+        sortKeys, bodyUsed, colorStart, pp, pm, lam, lamInit, match, tape, cacheSlot, counts;
     // adjoints
-    size_t ax, aq, av, aw, alam, app, apm, an, amuM, arestM, acache, amass, amu, arest, v1v, v1w;
+    size_t ax, aq, av, aw, alam, app, aext, acache, amass, amu, arest, dv, dw;
     // broadphase sort buffers, shared by the steps (not part of any record)
     size_t bpEntries, bpPairs;
     size_t stride;
@@ -51,8 +49,6 @@ __host__ __device__ Layout makeLayout(uint32_t nMax, uint32_t maxPairs, uint32_t
     L.snapStride = o;
     o = 0;
     L.aabb = take(sizeof(F) * 6 * nMax);
-    L.pairA = take(4ull * maxPairs);
-    L.pairB = take(4ull * maxPairs);
     L.mA = take(4ull * maxM);
     L.mB = take(4ull * maxM);
     L.mCount = take(4ull * maxM);
@@ -65,6 +61,7 @@ __host__ __device__ Layout makeLayout(uint32_t nMax, uint32_t maxPairs, uint32_t
     L.mDepth = take(sizeof(F) * 4 * maxM);
     L.color = take(4ull * maxM);
     L.order = take(4ull * maxM);
+    L.rank = take(4ull * maxM);
     L.sortKeys = take(8ull * maxM);
     L.bodyUsed = take(16ull * nMax);
     L.colorStart = take(4ull * (maxM + 1));
@@ -74,7 +71,7 @@ __host__ __device__ Layout makeLayout(uint32_t nMax, uint32_t maxPairs, uint32_t
     L.lamInit = take(sizeof(F) * 12 * maxM);
     L.match = take(16ull * maxM);
     L.tape = take(sizeof(F) * (size_t)(iterations > 0 ? iterations : 1) * maxM * kTapeScalars);
-    L.cacheSrc = take(4ull * cap);
+    L.cacheSlot = take(4ull * cap);
     L.counts = take(16);
     L.scrStride = o;
     o = 0;
@@ -86,16 +83,13 @@ __host__ __device__ Layout makeLayout(uint32_t nMax, uint32_t maxPairs, uint32_t
     L.aw = take(sizeof(F) * 3 * nMax);
     L.alam = take(sizeof(F) * 12 * maxM);
     L.app = take(sizeof(F) * 4 * maxM * kPreparedScalars);
-    L.apm = take(sizeof(F) * maxM * kPmScalars);
-    L.an = take(sizeof(F) * 3 * maxM);
-    L.amuM = take(sizeof(F) * maxM);
-    L.arestM = take(sizeof(F) * maxM);
+    L.aext = take(sizeof(F) * 4 * maxM * kAdjointExtra);
     L.acache = take(sizeof(F) * 3 * cap);
     L.amass = take(sizeof(F) * nMax);
     L.amu = take(sizeof(F) * nMax);
     L.arest = take(sizeof(F) * nMax);
-    L.v1v = take(sizeof(F) * 3 * nMax);
-    L.v1w = take(sizeof(F) * 3 * nMax);
+    L.dv = take(sizeof(F) * 3 * nMax);
+    L.dw = take(sizeof(F) * 3 * nMax);
     L.bpEntries = take(8ull * ad::nextPow2u(nMax > 0 ? nMax : 1));
     L.bpPairs = take(8ull * ad::nextPow2u(maxPairs > 0 ? maxPairs : 1));
     L.stride = o;
@@ -166,8 +160,6 @@ __device__ __forceinline__ StepScratch<F> scratch(const Slot &ws, uint32_t j) {
     const Layout &L = ws.L;
     StepScratch<F> s;
     s.aabb = at<F>(p, L.aabb);
-    s.pairA = at<uint32_t>(p, L.pairA);
-    s.pairB = at<uint32_t>(p, L.pairB);
     s.mA = at<uint32_t>(p, L.mA);
     s.mB = at<uint32_t>(p, L.mB);
     s.mCount = at<uint32_t>(p, L.mCount);
@@ -180,6 +172,7 @@ __device__ __forceinline__ StepScratch<F> scratch(const Slot &ws, uint32_t j) {
     s.mDepth = at<F>(p, L.mDepth);
     s.color = at<uint32_t>(p, L.color);
     s.order = at<uint32_t>(p, L.order);
+    s.rank = at<uint32_t>(p, L.rank);
     s.sortKeys = at<unsigned long long>(p, L.sortKeys);
     s.bodyUsed = at<unsigned long long>(p, L.bodyUsed);
     s.colorStart = at<uint32_t>(p, L.colorStart);
@@ -189,7 +182,7 @@ __device__ __forceinline__ StepScratch<F> scratch(const Slot &ws, uint32_t j) {
     s.lamInit = at<F>(p, L.lamInit);
     s.match = at<int32_t>(p, L.match);
     s.tape = at<F>(p, L.tape);
-    s.cacheSrc = at<uint32_t>(p, L.cacheSrc);
+    s.cacheSlot = at<uint32_t>(p, L.cacheSlot);
     s.counts = at<uint32_t>(p, L.counts);
     s.bpEntries = at<unsigned long long>(ws.base, L.bpEntries);
     s.bpPairs = at<unsigned long long>(ws.base, L.bpPairs);
@@ -217,21 +210,6 @@ __device__ __forceinline__ WorldParams<F> params(const Args &a, uint32_t w, cons
     return W;
 }
 
-__device__ void copySnap(const Snap &from, const Snap &to, uint32_t n) {
-    for (uint32_t i = threadIdx.x; i < 13 * n; i += blockDim.x) to.s.x[i] = from.s.x[i];
-    const uint32_t c = *from.c.count;
-    for (uint32_t e = threadIdx.x; e < c; e += blockDim.x) {
-        to.c.key[e] = from.c.key[e];
-        for (int j = 0; j < 3; ++j) {
-            to.c.anchorA[3 * e + j] = from.c.anchorA[3 * e + j];
-            to.c.anchorB[3 * e + j] = from.c.anchorB[3 * e + j];
-            to.c.lam[3 * e + j] = from.c.lam[3 * e + j];
-        }
-    }
-    if (threadIdx.x == 0) *to.c.count = c;
-    __syncthreads();
-}
-
 __device__ __forceinline__ uint32_t nextWorld(const Args &a) {
     __shared__ uint32_t s_w;
     __syncthreads();
@@ -245,78 +223,58 @@ __device__ __forceinline__ uint32_t nextWorld(const Args &a) {
 
 // Forward: steps every world, keeps a checkpoint every ckEvery steps (and the
 // final state), writes the final state.
-// Four blocks per SM (at most 128 registers a thread): the forward pass is
-// latency-bound, and the fourth resident world measured 102 -> 83 ms on
-// 1,024 worlds of 64 boxes (the adjoint keeps its registers: capping it
-// spilled and doubled its time).
-__global__ void __launch_bounds__(128, 4) k_rollout_forward(Args a, const F *x0, const F *q0, const F *v0, const F *w0,
-                                                       F *xT, F *qT, F *vT, F *wT) {
+template <int T, int B>
+__global__ void __launch_bounds__(T, B) k_rollout_forward(Args a, const F *x0, const F *q0, const F *v0, const F *w0,
+                                                          F *xT, F *qT, F *vT, F *wT) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ BlockScratch sh;
     for (;;) {
         const uint32_t w = nextWorld(a);
         if (w >= a.worlds) return;
         const Slot ws = slotOf(a, w);
         const WorldParams<F> W = params(a, w, ws);
         const uint32_t n = W.n, b = a.bodyStart[w];
-        Snap ck0 = snapshot(ws, 0, n);
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            for (int j = 0; j < 3; ++j) {
-                ck0.s.x[3 * i + j] = x0[3 * (b + i) + j];
-                ck0.s.v[3 * i + j] = v0[3 * (b + i) + j];
-                ck0.s.w[3 * i + j] = w0[3 * (b + i) + j];
-            }
-            for (int j = 0; j < 4; ++j) ck0.s.q[4 * i + j] = q0[4 * (b + i) + j];
+        Snap cur = snapshot(ws, 0, n);
+        for (uint32_t i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+            cur.s.x[i] = x0[3 * (size_t)b + i];
+            cur.s.v[i] = v0[3 * (size_t)b + i];
+            cur.s.w[i] = w0[3 * (size_t)b + i];
         }
-        if (threadIdx.x == 0) *ck0.c.count = 0;
+        for (uint32_t i = threadIdx.x; i < 4 * n; i += blockDim.x) cur.s.q[i] = q0[4 * (size_t)b + i];
+        if (threadIdx.x == 0) *cur.c.count = 0;
         __syncthreads();
-        Snap cur = ck0;
         bool failed = false;
         const StepScratch<F> sc = scratch(ws, 0);
         for (uint32_t t = 0; t < a.steps && !failed; ++t) {
-            Snap out = snapshot(ws, a.nCk + (t & 1), n);
-            forwardStep<F, BlockTeam>(W, cur.s, cur.c, out.s, out.c, sc, false);
+            // a checkpoint's step writes the checkpoint itself
+            const uint32_t s = t + 1;
+            const bool keep = s % a.ckEvery == 0 || s == a.steps;
+            const Snap out = snapshot(ws, keep ? (s + a.ckEvery - 1) / a.ckEvery : a.nCk + (t & 1), n);
+            forwardStepBlock(W, cur.s, cur.c, out.s, out.c, sc, false, s_dyn, sh);
             if (sc.counts[3]) {
                 if (threadIdx.x == 0) atomicOr(&a.err[w], sc.counts[3]);
                 failed = true;
-                break;
             }
-            const uint32_t s = t + 1;
-            if (s % a.ckEvery == 0 || s == a.steps) {
-                const Snap ck = snapshot(ws, (s + a.ckEvery - 1) / a.ckEvery, n);
-                copySnap(out, ck, n);
-                cur = ck;
-            } else {
-                cur = out;
-            }
+            cur = out;
         }
         if (failed) continue;
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            for (int j = 0; j < 3; ++j) {
-                xT[3 * (b + i) + j] = cur.s.x[3 * i + j];
-                vT[3 * (b + i) + j] = cur.s.v[3 * i + j];
-                wT[3 * (b + i) + j] = cur.s.w[3 * i + j];
-            }
-            for (int j = 0; j < 4; ++j) qT[4 * (b + i) + j] = cur.s.q[4 * i + j];
+        for (uint32_t i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+            xT[3 * (size_t)b + i] = cur.s.x[i];
+            vT[3 * (size_t)b + i] = cur.s.v[i];
+            wT[3 * (size_t)b + i] = cur.s.w[i];
         }
+        for (uint32_t i = threadIdx.x; i < 4 * n; i += blockDim.x) qT[4 * (size_t)b + i] = cur.s.q[i];
     }
-}
-
-__device__ void mapCacheAdjoint(const Slot &ws, const StepScratch<F> &prev, uint32_t count) {
-    F *alam = at<F>(ws.base, ws.L.alam);
-    const F *acache = at<F>(ws.base, ws.L.acache);
-    for (uint32_t i = threadIdx.x; i < 12 * ws.maxM; i += blockDim.x) alam[i] = 0.0f;
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < count; e += blockDim.x) {
-        const uint32_t kp = prev.cacheSrc[e];
-        for (int j = 0; j < 3; ++j) alam[3 * kp + j] += acache[3 * e + j];
-    }
-    __syncthreads();
 }
 
 // Adjoint: per segment (last first) recompute from the checkpoint with the
 // tape, then reverse step by step.
-__global__ void __launch_bounds__(128) k_rollout_backward(Args a, const F *gx, const F *gq, const F *gv,
-                                                        const F *gw, F *gx0, F *gq0, F *gv0, F *gw0, F *gmass,
-                                                        F *gmu, F *grest) {
+template <int T, int B>
+__global__ void __launch_bounds__(T, B) k_rollout_backward(Args a, const F *gx, const F *gq, const F *gv, const F *gw,
+                                                           F *gx0, F *gq0, F *gv0, F *gw0, F *gmass, F *gmu,
+                                                           F *grest) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ BlockScratch sh;
     for (;;) {
         const uint32_t w = nextWorld(a);
         if (w >= a.worlds) return;
@@ -325,74 +283,78 @@ __global__ void __launch_bounds__(128) k_rollout_backward(Args a, const F *gx, c
         const Layout &L0 = ws.L;
         const WorldParams<F> W = params(a, w, ws);
         const uint32_t n = W.n, b = a.bodyStart[w];
-        AdjointView<F> adj{at<F>(base, L0.ax),     at<F>(base, L0.aq),     at<F>(base, L0.av),
-                           at<F>(base, L0.aw),     at<F>(base, L0.alam),   at<F>(base, L0.app),
-                           at<F>(base, L0.apm),    at<F>(base, L0.an),     at<F>(base, L0.amuM),
-                           at<F>(base, L0.arestM), at<F>(base, L0.acache), at<F>(base, L0.amass),
-                           at<F>(base, L0.amu),    at<F>(base, L0.arest)};
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            for (int j = 0; j < 3; ++j) {
-                adj.ax[3 * i + j] = gx ? gx[3 * (b + i) + j] : 0.0f;
-                adj.av[3 * i + j] = gv ? gv[3 * (b + i) + j] : 0.0f;
-                adj.aw[3 * i + j] = gw ? gw[3 * (b + i) + j] : 0.0f;
-            }
-            for (int j = 0; j < 4; ++j) adj.aq[4 * i + j] = gq ? gq[4 * (b + i) + j] : 0.0f;
-            adj.amass[i] = adj.amu[i] = adj.arest[i] = 0.0f;
+        AdjointView<F> adj{};
+        adj.ax = at<F>(base, L0.ax);
+        adj.aq = at<F>(base, L0.aq);
+        adj.av = at<F>(base, L0.av);
+        adj.aw = at<F>(base, L0.aw);
+        adj.alam = at<F>(base, L0.alam);
+        adj.app = at<F>(base, L0.app);
+        adj.aext = at<F>(base, L0.aext);
+        adj.acache = at<F>(base, L0.acache);
+        adj.amass = at<F>(base, L0.amass);
+        adj.amu = at<F>(base, L0.amu);
+        adj.arest = at<F>(base, L0.arest);
+        adj.dv = at<F>(base, L0.dv);
+        adj.dw = at<F>(base, L0.dw);
+        for (uint32_t i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+            adj.ax[i] = gx ? gx[3 * (size_t)b + i] : 0.0f;
+            adj.av[i] = gv ? gv[3 * (size_t)b + i] : 0.0f;
+            adj.aw[i] = gw ? gw[3 * (size_t)b + i] : 0.0f;
         }
-        for (uint32_t i = threadIdx.x; i < 12 * ws.maxM; i += blockDim.x) adj.alam[i] = 0.0f;
+        for (uint32_t i = threadIdx.x; i < 4 * n; i += blockDim.x) adj.aq[i] = gq ? gq[4 * (size_t)b + i] : 0.0f;
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) adj.amass[i] = adj.amu[i] = adj.arest[i] = 0.0f;
         __syncthreads();
-        ad::StateView<F> v1{nullptr, nullptr, at<F>(base, L0.v1v), at<F>(base, L0.v1w)};
         const uint32_t nSeg = (a.steps + a.ckEvery - 1) / a.ckEvery;
-        bool pending = false, failed = false;
-        uint32_t pendingCount = 0;
+        bool failed = false;
         for (int s = (int)nSeg - 1; s >= 0 && !failed; --s) {
             const uint32_t t0 = (uint32_t)s * a.ckEvery;
             const uint32_t L = min(a.steps, t0 + a.ckEvery) - t0;
-            copySnap(snapshot(ws, (uint32_t)s, n), snapshot(ws, a.nCk, n), n);
-            for (uint32_t i = 0; i < L; ++i) {
-                const Snap in = snapshot(ws, a.nCk + i, n), out = snapshot(ws, a.nCk + i + 1, n);
+            // state i of the segment: its checkpoint, then the recomputed steps
+            auto state = [&](uint32_t i) { return snapshot(ws, i == 0 ? (uint32_t)s : a.nCk + i, n); };
+            for (uint32_t i = 0; i < L && !failed; ++i) {
+                const Snap in = state(i), out = state(i + 1);
                 const StepScratch<F> sc = scratch(ws, i);
-                forwardStep<F, BlockTeam>(W, in.s, in.c, out.s, out.c, sc, true);
+                forwardStepBlock(W, in.s, in.c, out.s, out.c, sc, true, s_dyn, sh);
                 if (sc.counts[3]) {
                     if (threadIdx.x == 0) atomicOr(&a.err[w], sc.counts[3]);
                     failed = true;
-                    break;
                 }
             }
-            if (failed) break;
-            if (pending) mapCacheAdjoint(ws, scratch(ws, L - 1), pendingCount);
-            for (int i = (int)L - 1; i >= 0; --i) {
-                const Snap in = snapshot(ws, a.nCk + i, n), out = snapshot(ws, a.nCk + i + 1, n);
-                const StepScratch<F> sc = scratch(ws, (uint32_t)i);
-                backwardStep<F, BlockTeam>(W, in.s, in.c, out.s, v1, sc, adj);
-                if (sc.counts[3]) {
-                    if (threadIdx.x == 0) atomicOr(&a.err[w], sc.counts[3]);
-                    failed = true;
-                    break;
-                }
-                const uint32_t cnt = *in.c.count;
-                if (i > 0) {
-                    mapCacheAdjoint(ws, scratch(ws, (uint32_t)i - 1), cnt);
-                } else {
-                    pending = t0 > 0;
-                    pendingCount = cnt;
-                }
+            for (int i = (int)L - 1; i >= 0 && !failed; --i) {
+                const Snap in = state((uint32_t)i), out = state((uint32_t)i + 1);
+                backwardStepBlock(W, in.s, in.c, out.s, scratch(ws, (uint32_t)i), adj, t0 + (uint32_t)i + 1 == a.steps,
+                                  s_dyn);
             }
         }
         if (failed) continue;
+        for (uint32_t i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+            if (gx0) gx0[3 * (size_t)b + i] = adj.ax[i];
+            if (gv0) gv0[3 * (size_t)b + i] = adj.av[i];
+            if (gw0) gw0[3 * (size_t)b + i] = adj.aw[i];
+        }
+        if (gq0)
+            for (uint32_t i = threadIdx.x; i < 4 * n; i += blockDim.x) gq0[4 * (size_t)b + i] = adj.aq[i];
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            for (int j = 0; j < 3; ++j) {
-                if (gx0) gx0[3 * (b + i) + j] = adj.ax[3 * i + j];
-                if (gv0) gv0[3 * (b + i) + j] = adj.av[3 * i + j];
-                if (gw0) gw0[3 * (b + i) + j] = adj.aw[3 * i + j];
-            }
-            for (int j = 0; j < 4; ++j)
-                if (gq0) gq0[4 * (b + i) + j] = adj.aq[4 * i + j];
             if (gmass) gmass[b + i] = adj.amass[i];
             if (gmu) gmu[b + i] = adj.amu[i];
             if (grest) grest[b + i] = adj.arest[i];
         }
     }
+}
+
+// Block size and register budget: small worlds take 128 threads (32 manifolds
+// at once), others 256 (64 manifolds).
+constexpr uint32_t kSmallWorld = 36;
+using ForwardKernel = void (*)(Args, const F *, const F *, const F *, const F *, F *, F *, F *, F *);
+using BackwardKernel = void (*)(Args, const F *, const F *, const F *, const F *, F *, F *, F *, F *, F *, F *, F *);
+
+// Blocks that the device holds at once, at most one a world.
+template <class Kernel> uint32_t residentBlocks(Kernel k, int threads, size_t smem, uint32_t worlds, int device) {
+    int sms = 0, per = 0;
+    PE_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, smem));
+    return std::min<uint32_t>(worlds, (uint32_t)(std::max(1, per) * sms));
 }
 
 template <class T> void uploadVec(DeviceArray<T> &d, const std::vector<T> &h) {
@@ -507,8 +469,7 @@ void Rollout::checkErrors(cudaStream_t s, const char *what) {
             const char *m = (b & kAdErrPairs)       ? "candidate pairs exceed the world's capacity"
                             : (b & kAdErrManifolds) ? "contact manifolds exceed the world's capacity"
                             : (b & kAdErrColors)    ? "solver colouring failed"
-                            : (b & kAdErrCache)     ? "warm-start cache overflow"
-                                                    : "the adjoint's replay of a contact differed from the forward";
+                                                    : "warm-start cache overflow";
             throw std::runtime_error(std::string(what) + ": world " + std::to_string(w) + ": " + m);
         }
 }
@@ -549,13 +510,13 @@ void Rollout::forward(const float *x0, const float *q0, const float *v0, const f
     a.dt = dt_;
     a.queueHead = queue_.ptr;
     a.err = err_.ptr;
-    int sms = 0;
-    PE_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    int per = 0;
-    PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rollout_forward, 128, 0));
-    const uint32_t blocks = std::min<uint32_t>(a.worlds, (uint32_t)std::max(1, per) * sms);
+    const bool small = nMax_ <= kSmallWorld;
+    const ForwardKernel kernel = small ? k_rollout_forward<128, 4> : k_rollout_forward<256, 2>;
+    const int threads = small ? 128 : 256;
+    const size_t smem = sharedBytes(nMax_);
+    const uint32_t blocks = residentBlocks(kernel, threads, smem, a.worlds, device_);
     PE_CHECK(cudaEventRecord(e0_, s));
-    k_rollout_forward<<<blocks, 128, 0, s>>>(a, x0, q0, v0, w0, xT, qT, vT, wT);
+    kernel<<<blocks, threads, smem, s>>>(a, x0, q0, v0, w0, xT, qT, vT, wT);
     PE_LAUNCHED();
     PE_CHECK(cudaEventRecord(e1_, s));
     checkErrors(s, "rollout forward");
@@ -595,14 +556,13 @@ void Rollout::backward(const float *gx, const float *gq, const float *gv, const 
     a.dt = dt_;
     a.queueHead = queue_.ptr;
     a.err = err_.ptr;
-    int sms = 0;
-    PE_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    int per = 0;
-    PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rollout_backward, 128, 0));
-    const uint32_t blocks = std::min<uint32_t>(a.worlds, (uint32_t)std::max(1, per) * sms);
+    const bool small = nMax_ <= kSmallWorld;
+    const BackwardKernel kernel = small ? k_rollout_backward<128, 2> : k_rollout_backward<256, 1>;
+    const int threads = small ? 128 : 256;
+    const size_t smem = sharedBytes(nMax_);
+    const uint32_t blocks = residentBlocks(kernel, threads, smem, a.worlds, device_);
     PE_CHECK(cudaEventRecord(e0_, s));
-    k_rollout_backward<<<blocks, 128, 0, s>>>(a, gx, gq, gv, gw, gx0, gq0, gv0, gw0, gmass, gfriction,
-                                              grestitution);
+    kernel<<<blocks, threads, smem, s>>>(a, gx, gq, gv, gw, gx0, gq0, gv0, gw0, gmass, gfriction, grestitution);
     PE_LAUNCHED();
     PE_CHECK(cudaEventRecord(e1_, s));
     checkErrors(s, "rollout backward");

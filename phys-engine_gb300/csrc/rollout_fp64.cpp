@@ -39,21 +39,19 @@ struct CacheMem {
 
 struct ScratchMem {
     std::vector<S> aabb, mNormal, mMu, mRest, mAnchorA, mAnchorB, mDepth, pp, pm, lam, lamInit, tape;
-    std::vector<uint32_t> pairA, pairB, mA, mB, mCount, mFeature, color, order, colorStart, cacheSrc, counts;
+    std::vector<uint32_t> mA, mB, mCount, mFeature, color, order, colorStart, cacheSlot, counts;
     std::vector<unsigned long long> sortKeys, bodyUsed, bpEntries, bpPairs;
     std::vector<int32_t> match;
     ScratchMem(uint32_t n, uint32_t maxPairs, uint32_t maxM, int iterations)
         : aabb(6 * n), mNormal(3 * maxM), mMu(maxM), mRest(maxM), mAnchorA(12 * maxM), mAnchorB(12 * maxM),
           mDepth(4 * maxM), pp((size_t)4 * maxM * kPreparedScalars), pm((size_t)maxM * kPmScalars), lam(12 * maxM),
-          lamInit(12 * maxM), tape((size_t)(iterations > 0 ? iterations : 1) * maxM * kTapeScalars), pairA(maxPairs),
-          pairB(maxPairs), mA(maxM), mB(maxM), mCount(maxM), mFeature(4 * maxM), color(maxM), order(maxM),
-          colorStart(maxM + 1), cacheSrc(4 * maxM), counts(4), sortKeys(maxM), bodyUsed(2 * n),
+          lamInit(12 * maxM), tape((size_t)(iterations > 0 ? iterations : 1) * maxM * kTapeScalars),
+          mA(maxM), mB(maxM), mCount(maxM), mFeature(4 * maxM), color(maxM), order(maxM),
+          colorStart(maxM + 1), cacheSlot(4 * maxM), counts(4), sortKeys(maxM), bodyUsed(2 * n),
           bpEntries(nextPow2u(n > 0 ? n : 1)), bpPairs(nextPow2u(maxPairs > 0 ? maxPairs : 1)), match(4 * maxM) {}
     StepScratch<S> view() {
-        StepScratch<S> s;
+        StepScratch<S> s{};
         s.aabb = aabb.data();
-        s.pairA = pairA.data();
-        s.pairB = pairB.data();
         s.mA = mA.data();
         s.mB = mB.data();
         s.mCount = mCount.data();
@@ -75,7 +73,7 @@ struct ScratchMem {
         s.lamInit = lamInit.data();
         s.match = match.data();
         s.tape = tape.data();
-        s.cacheSrc = cacheSrc.data();
+        s.cacheSlot = cacheSlot.data();
         s.counts = counts.data();
         s.bpEntries = bpEntries.data();
         s.bpPairs = bpPairs.data();
@@ -88,7 +86,6 @@ const char *errorText(uint32_t bits) {
     if (bits & kAdErrManifolds) return "contact manifolds exceed the rollout's manifold capacity";
     if (bits & kAdErrColors) return "more than 128 solver colours";
     if (bits & kAdErrCache) return "warm-start cache overflow";
-    if (bits & kAdErrReplay) return "the adjoint's replay of a contact differed from the forward pass";
     return "rollout failed";
 }
 
@@ -172,7 +169,7 @@ int pe_fp64_rollout(uint32_t n, const uint8_t *shape, const uint8_t *is_static, 
         scratch.emplace_back(n, maxPairs, maxM, iterations);
         StateView<S> in = state[t].view();
         CacheView<S> cin = cache[t].view();
-        forwardStep<S, HostTeam>(W, in, cin, state[t + 1].view(), cache[t + 1].view(), scratch[t].view(), true);
+        forwardStep<S>(W, in, cin, state[t + 1].view(), cache[t + 1].view(), scratch[t].view(), true);
         if (scratch[t].counts[3]) return setErr(err, err_len, errorText(scratch[t].counts[3])), 2;
     }
     const StateMem &fin = state[steps];
@@ -188,24 +185,31 @@ int pe_fp64_rollout(uint32_t n, const uint8_t *shape, const uint8_t *is_static, 
     if (d_final_v) std::memcpy(av.data(), d_final_v, 3 * n * sizeof(S));
     if (d_final_w) std::memcpy(aw.data(), d_final_w, 3 * n * sizeof(S));
     std::vector<S> alam(12 * maxM, 0.0), app((size_t)4 * maxM * kPreparedScalars), apm((size_t)maxM * kPmScalars),
-        an(3 * maxM), amuM(maxM), arestM(maxM), acache(12 * maxM), amass(n, 0.0), amu(n, 0.0), arest(n, 0.0);
-    std::vector<S> v1v(3 * n), v1w(3 * n);
-    AdjointView<S> adj{ax.data(),    aq.data(),    av.data(),   aw.data(),     alam.data(),
-                       app.data(),   apm.data(),   an.data(),   amuM.data(),   arestM.data(),
-                       acache.data(), amass.data(), amu.data(), arest.data()};
+        an(3 * maxM), amuM(maxM), acache(12 * maxM), amass(n, 0.0), amu(n, 0.0), arest(n, 0.0);
+    AdjointView<S> adj{};
+    adj.ax = ax.data();
+    adj.aq = aq.data();
+    adj.av = av.data();
+    adj.aw = aw.data();
+    adj.alam = alam.data();
+    adj.app = app.data();
+    adj.apm = apm.data();
+    adj.an = an.data();
+    adj.amuM = amuM.data();
+    adj.acache = acache.data();
+    adj.amass = amass.data();
+    adj.amu = amu.data();
+    adj.arest = arest.data();
     for (int t = (int)steps - 1; t >= 0; --t) {
-        StateView<S> v1{nullptr, nullptr, v1v.data(), v1w.data()};
-        backwardStep<S, HostTeam>(W, state[t].view(), cache[t].view(), state[t + 1].view(), v1, scratch[t].view(),
-                                  adj);
-        if (scratch[t].counts[3]) return setErr(err, err_len, errorText(scratch[t].counts[3])), 3;
+        backwardStep<S>(W, state[t].view(), cache[t].view(), state[t + 1].view(), scratch[t].view(), adj);
         // adjoint of this step's input cache -> adjoint of the previous step's final impulses
         std::fill(alam.begin(), alam.end(), 0.0);
         if (t > 0) {
-            const uint32_t cnt = cache[t].count;
-            for (uint32_t e = 0; e < cnt; ++e) {
-                const uint32_t kp = scratch[t - 1].cacheSrc[e];
-                for (int j = 0; j < 3; ++j) alam[3 * kp + j] += acache[3 * e + j];
-            }
+            const std::vector<uint32_t> &slot = scratch[t - 1].cacheSlot;
+            const uint32_t points = 4 * scratch[t - 1].counts[1];
+            for (uint32_t kp = 0; kp < points; ++kp)
+                if (slot[kp] != kNoSlot)
+                    for (int j = 0; j < 3; ++j) alam[3 * kp + j] = acache[3 * slot[kp] + j];
         }
     }
     if (d_x0) std::memcpy(d_x0, ax.data(), 3 * n * sizeof(S));

@@ -56,3 +56,101 @@ def test_batch_poses_reach_any_array(gpu, n, offset):
         assert_bit_equal(q[offset:offset + 4 * n].reshape(n, 4), rot, "rotations")
         for a, k in ((p, 3), (q, 4)):
             assert np.all(a[:offset] == 7.0) and np.all(a[offset + k * n:] == 7.0)
+
+
+def boxes_on_floor(n, seed):
+    """n boxes pressed 2 cm into a floor and sliding (no stick-slip switch)."""
+    sc = scenes.generate(scenes.BOXES_ON_PLANE, n, seed)
+    rng = np.random.default_rng(seed)
+    ang = rng.uniform(0, 2 * np.pi, n)
+    sc.linvel[1:] = (2.0 * np.stack([np.cos(ang), np.zeros(n), np.sin(ang)], 1)).astype(np.float32)
+    sc.pos[1:, 1] -= np.float32(0.02)
+    return sc
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 37, 63, 64, 65, 200])
+def test_rollout_block_paths(gpu, n):
+    """One world at the sizes where the block's paths change: a group of lanes
+    for every manifold or several manifolds a group (32 / 64 manifolds), 128 or
+    256 threads (36 bodies).  Forward against the batched engine, bit for bit; gradients against
+    the FP64 adjoint, float rounding (6e-8) grown by the 4 steps' condition: the
+    1e-3 that this adjoint is held to elsewhere."""
+    import torch
+
+    from phys_gb300 import rollout
+
+    sc = boxes_on_floor(n, 3)
+    steps, dt, iters = 4, 1 / 120, 10
+    roll = rollout.GpuRollout([sc], steps, dt, iterations=iters, checkpoint_every=3)
+    start = roll.initial_state()
+    args = [torch.tensor(a, device="cuda:0") for a in (*start, roll.mass, roll.friction, roll.restitution)]
+    outs = roll.forward(*args)
+    batch = gpu.GpuBatch([sc], iterations=iters)
+    batch.step(dt, steps)
+    for k, (o, r) in enumerate(zip(outs, batch.bodies())):
+        assert_bit_equal(o.cpu().numpy(), r, f"state {k}")
+    rng = np.random.default_rng(5)
+    d = [rng.normal(size=tuple(o.shape)).astype(np.float32) for o in outs]
+    grads = roll.backward(*[torch.tensor(a, device="cuda:0") for a in d])
+    _, iinv, he = rollout.body_properties(sc)
+    _, ref = rollout.fp64_rollout(sc.shape, sc.is_static, he, iinv, start, roll.mass, roll.friction, roll.restitution,
+                                  steps, dt, iters, d_final=d)
+    dyn = ~sc.is_static.astype(bool)
+    for name, g, r in zip(("x0", "q0", "v0", "w0", "mass", "friction", "restitution"), grads, ref):
+        g, r = g.cpu().numpy()[dyn], r[dyn]
+        assert np.linalg.norm(g - r) <= 1e-3 * max(np.linalg.norm(r), 1e-6), name
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1055])
+def test_rollout_of_a_large_world_equals_its_parts(gpu, n):
+    """Velocities in shared memory up to 1,024 bodies, in global memory beyond:
+    boxes that touch the floor alone move in one world as they do in worlds of
+    at most 31 boxes, and have the same gradients (one manifold a body: nothing
+    is summed in another order)."""
+    import torch
+
+    from phys_gb300 import rollout
+
+    sc = boxes_on_floor(n, 3)
+    rows = np.arange(1, n + 1)
+    parts = [np.concatenate([[0], rows[i:i + 31]]) for i in range(0, n, 31)]
+    rng = np.random.default_rng(6)
+    d = [rng.normal(size=(n + 1, k)).astype(np.float32) for k in (3, 4, 3, 3)]
+    got = []
+    for worlds in ([np.arange(n + 1)], parts):
+        roll = rollout.GpuRollout([sc.subset(w) for w in worlds], 4, 1 / 120, iterations=10, checkpoint_every=3)
+        args = [torch.tensor(a, device="cuda:0")
+                for a in (*roll.initial_state(), roll.mass, roll.friction, roll.restitution)]
+        outs = roll.forward(*args)
+        pick = np.concatenate(worlds)
+        grads = roll.backward(*[torch.tensor(a[pick], device="cuda:0") for a in d])
+        moving = pick > 0
+        got.append([t.cpu().numpy()[moving] for t in (*outs, *grads)])
+    for k, (a, b) in enumerate(zip(*got)):
+        assert_bit_equal(a, b, f"output {k}")
+
+
+def test_rollout_of_a_pile(gpu):
+    """Several colours and islands: spheres and boxes in two layers on a floor
+    (bodies with many manifolds), more manifolds than the block has groups."""
+    import torch
+
+    from phys_gb300 import rollout
+
+    sc = scenes.mixed_field(90, 4)
+    sc.pos[1:] *= np.float32([0.64, 0.6, 0.64])  # neighbours overlap by a few centimetres
+    steps, dt, iters = 2, 1 / 120, 8
+    roll = rollout.GpuRollout([sc], steps, dt, iterations=iters, checkpoint_every=2, manifolds_per_body=8)
+    start = roll.initial_state()
+    args = [torch.tensor(a, device="cuda:0") for a in (*start, roll.mass, roll.friction, roll.restitution)]
+    outs = roll.forward(*args)
+    batch = gpu.GpuBatch([sc], iterations=iters)
+    batch.step(dt, steps)
+    st = batch.stats(0)
+    assert st["contact_count"] > 64 and st["color_count"] > 3
+    for k, (o, r) in enumerate(zip(outs, batch.bodies())):
+        assert_bit_equal(o.cpu().numpy(), r, f"state {k}")
+    rng = np.random.default_rng(5)
+    d = [torch.tensor(rng.normal(size=tuple(o.shape)).astype(np.float32), device="cuda:0") for o in outs]
+    for g in roll.backward(*d):
+        assert bool(torch.isfinite(g).all())
