@@ -45,7 +45,16 @@ __host__ __device__ inline uint32_t sharedBytes(uint32_t n) {
     return sort > stage ? sort : stage;
 }
 
-struct BlockScratch {
+// What the block steps, in shared memory: some sixty pointers and numbers that
+// every thread would otherwise hold in registers or reload from its stack
+// (by value through the step's calls they cost 1.25x the adjoint's time).
+struct BlockWorld {
+    WorldParams<F> W;
+    StateView<F> in, out;   // the step's start and end
+    CacheView<F> cin, cout;
+    StepScratch<F> sc;
+    AdjointView<F> adj;
+    unsigned char *dyn;     // sharedBytes(n) bytes, aligned to 16
     uint32_t scan[33];
     uint32_t pairs, colored, deferred, colors;
 };
@@ -138,11 +147,14 @@ __device__ __noinline__ void blockSort(Key *k, uint32_t n) {
 }
 
 // ------------------------------------------------------ manifold lane groups --
-// Four lanes of a warp work on one manifold; lane p holds point p.
+// Four lanes of a warp work on one manifold; lane p holds point p.  The whole
+// warp takes part in every exchange (its eight groups run in step, those without
+// a manifold idle): exchanges under one mask a group were issued one group after
+// the other, which made a hand-over of the velocities eight times as long.
+constexpr uint32_t kWarp = 0xffffffffu;
 struct Group {
     uint32_t id, count;  // this group, groups of the block
     uint32_t p, first;   // lane in the group, the group's first lane in the warp
-    uint32_t mask;
 };
 __device__ __forceinline__ Group laneGroup() {
     Group g;
@@ -151,27 +163,29 @@ __device__ __forceinline__ Group laneGroup() {
     g.count = blockDim.x >> 2;
     g.p = lane & 3;
     g.first = lane & ~3u;
-    g.mask = 0xFu << g.first;
     return g;
 }
-__device__ __forceinline__ V3<F> shfl3(uint32_t mask, const V3<F> &v, uint32_t from) {
-    return {__shfl_sync(mask, v.x, from), __shfl_sync(mask, v.y, from), __shfl_sync(mask, v.z, from)};
+__device__ __forceinline__ V3<F> shfl3(const V3<F> &v, uint32_t from) {
+    return {__shfl_sync(kWarp, v.x, from), __shfl_sync(kWarp, v.y, from), __shfl_sync(kWarp, v.z, from)};
 }
-// The velocity part of s from lane `from` of the group.
-__device__ __forceinline__ void shareVelocities(const Group &g, PointIn<F> &s, uint32_t from) {
+// The velocity part of s from lane `from` of each group.  dynA: some group of
+// the warp has a moving body A (a static body's velocities stay as they are).
+__device__ __forceinline__ void shareVelocities(const Group &g, PointIn<F> &s, uint32_t from, bool dynA) {
     const uint32_t l = g.first + from;
-    s.vA = shfl3(g.mask, s.vA, l);
-    s.wA = shfl3(g.mask, s.wA, l);
-    s.vB = shfl3(g.mask, s.vB, l);
-    s.wB = shfl3(g.mask, s.wB, l);
+    if (dynA) {
+        s.vA = shfl3(s.vA, l);
+        s.wA = shfl3(s.wA, l);
+    }
+    s.vB = shfl3(s.vB, l);
+    s.wB = shfl3(s.wB, l);
 }
-__device__ __forceinline__ F groupSum(const Group &g, F v) {
-    v += __shfl_xor_sync(g.mask, v, 1);
-    v += __shfl_xor_sync(g.mask, v, 2);
+__device__ __forceinline__ F groupSum(F v) {
+    v += __shfl_xor_sync(kWarp, v, 1);
+    v += __shfl_xor_sync(kWarp, v, 2);
     return v;
 }
-__device__ __forceinline__ V3<F> groupSum(const Group &g, const V3<F> &v) {
-    return {groupSum(g, v.x), groupSum(g, v.y), groupSum(g, v.z)};
+__device__ __forceinline__ V3<F> groupSum(const V3<F> &v) {
+    return {groupSum(v.x), groupSum(v.y), groupSum(v.z)};
 }
 
 // What a manifold's lanes need of it.
@@ -181,8 +195,8 @@ struct ManifoldLane {
     F mu;
     V3<F> n;
 };
-__device__ __forceinline__ ManifoldLane loadManifold(const WorldParams<F> &W, const StepScratch<F> &sc, const Group &g,
-                                                     uint32_t k) {
+__device__ __forceinline__ ManifoldLane loadManifold(const BlockWorld &bw, const Group &g, uint32_t k) {
+    const StepScratch<F> &sc = bw.sc;
     ManifoldLane l;
     l.k = k;
     l.kp = 4 * k + g.p;
@@ -190,8 +204,8 @@ __device__ __forceinline__ ManifoldLane loadManifold(const WorldParams<F> &W, co
     l.a = sc.mA[l.m];
     l.b = sc.mB[l.m];
     l.npts = sc.mCount[l.m];
-    l.sA = W.isStatic[l.a] != 0;
-    l.sB = W.isStatic[l.b] != 0;
+    l.sA = bw.W.isStatic[l.a] != 0;
+    l.sB = bw.W.isStatic[l.b] != 0;
     l.mu = sc.mMu[l.m];
     l.n = ld3(sc.mNormal, l.m);
     return l;
@@ -216,9 +230,12 @@ struct PreparedLane {
     M3<F> IA, IB;
     F imA, imB;
 };
-__device__ __forceinline__ void prepareLane(const WorldParams<F> &W, const StateView<F> &in, const CacheView<F> &cin,
-                                            const StateView<F> &out, const StepScratch<F> &sc, const ManifoldLane &l,
-                                            const Group &g, PreparedLane &o) {
+__device__ __forceinline__ void prepareLane(const BlockWorld &bw, const ManifoldLane &l, const Group &g,
+                                            PreparedLane &o) {
+    const WorldParams<F> &W = bw.W;
+    const StateView<F> &in = bw.in, &out = bw.out;
+    const CacheView<F> &cin = bw.cin;
+    const StepScratch<F> &sc = bw.sc;
     const Q<F> qA = ld4q(in.q, l.a), qB = ld4q(in.q, l.b);
     o.IA = inverseInertiaWorld(qA, W.iinv[3 * l.a], W.iinv[3 * l.a + 1], W.iinv[3 * l.a + 2]);
     o.IB = inverseInertiaWorld(qB, W.iinv[3 * l.b], W.iinv[3 * l.b + 1], W.iinv[3 * l.b + 2]);
@@ -272,15 +289,24 @@ __device__ __forceinline__ void storePair(const ManifoldLane &l, F *v, F *w, con
     }
 }
 
-// Warm start of one manifold (warmStartPrepared :453-490): point after point.
-__device__ __forceinline__ void warmGroup(const Group &g, const ManifoldLane &l, const F *c, const F *lam, int32_t match,
-                                          const M3<F> &IA, const M3<F> &IB, F imA, F imB, F *v, F *w) {
-    PointIn<F> s;
-    loadPair(l, v, w, s);
-    const uint32_t any = __ballot_sync(g.mask, g.p < l.npts && match >= 0) & g.mask;
-    if (!any) return;
-    for (uint32_t q = 0; q < l.npts; ++q) {
-        if (g.p == q && match >= 0) {
+// The number of turns that the warp's points need, over its groups that act.
+__device__ __forceinline__ uint32_t warpTurns(bool act, uint32_t npts) {
+    return __reduce_max_sync(kWarp, act ? npts : 0u);
+}
+
+// Warm start of one manifold a group (warmStartPrepared :453-490): point after
+// point.  act: the group has a manifold in this turn (whole warps call).
+__device__ __forceinline__ void warmGroup(const Group &g, bool act, const ManifoldLane &l, const F *c, const F *lam,
+                                          int32_t match, const M3<F> &IA, const M3<F> &IB, F imA, F imB, F *v, F *w) {
+    const uint32_t matched = __ballot_sync(kWarp, act && g.p < l.npts && match >= 0);
+    const bool any = ((matched >> g.first) & 0xFu) != 0;  // else the bodies are not written
+    const uint32_t turns = warpTurns(any, l.npts);
+    if (!turns) return;
+    const bool dynA = __any_sync(kWarp, any && !l.sA);
+    PointIn<F> s{};
+    if (any) loadPair(l, v, w, s);
+    for (uint32_t q = 0; q < turns; ++q) {
+        if (g.p == q && ((matched >> (g.first + q)) & 1u)) {
             const V3<F> wi = l.n * lam[0] + pv(c, kPT1) * lam[1] + pv(c, kPT2) * lam[2];
             const V3<F> nw = -wi;
             if (!l.sA) {
@@ -292,45 +318,59 @@ __device__ __forceinline__ void warmGroup(const Group &g, const ManifoldLane &l,
                 s.wB += mul(IB, cross(pv(c, kPOffB), wi));
             }
         }
-        if (q + 1 < l.npts) shareVelocities(g, s, q);
+        if (q + 1 < turns) shareVelocities(g, s, q, dynA);
     }
-    if (g.p + 1 == l.npts) storePair(l, v, w, s);
+    if (any && g.p + 1 == turns) storePair(l, v, w, s);
 }
 
-// One velocity update of one manifold; tape (nullable): fields `stride` apart
-// that take the manifold's velocities and impulses from before it.
-__device__ __forceinline__ void solveGroup(const Group &g, const ManifoldLane &l, const F *c, F *lam, F imA, F imB,
-                                           F *v, F *w, F *tape, size_t stride) {
-    PointIn<F> s;
-    loadPair(l, v, w, s);
-    if (tape) {
-        const V3<F> t = g.p == 0 ? s.vA : g.p == 1 ? s.wA : g.p == 2 ? s.vB : s.wB;
-        F *o = tape + l.k;
-        o[(3 * g.p) * stride] = t.x;
-        o[(3 * g.p + 1) * stride] = t.y;
-        o[(3 * g.p + 2) * stride] = t.z;
+// One velocity update of one manifold a group; tape (nullable): fields `stride`
+// apart that take the manifold's velocities and impulses from before it.
+__device__ __forceinline__ void solveGroup(const Group &g, bool act, const ManifoldLane &l, const F *c, F *lam, F imA,
+                                           F imB, F *v, F *w, F *tape, size_t stride) {
+    const uint32_t turns = warpTurns(act, l.npts);
+    if (!turns) return;
+    const bool dynA = __any_sync(kWarp, act && !l.sA);
+    PointIn<F> s{};
+    if (act) {
+        loadPair(l, v, w, s);
+        if (tape) {
+            const V3<F> t = g.p == 0 ? s.vA : g.p == 1 ? s.wA : g.p == 2 ? s.vB : s.wB;
+            F *o = tape + l.k;
+            o[(3 * g.p) * stride] = t.x;
+            o[(3 * g.p + 1) * stride] = t.y;
+            o[(3 * g.p + 2) * stride] = t.z;
 #pragma unroll
-        for (uint32_t e = 0; e < 3; ++e) o[(12 + 3 * g.p + e) * stride] = lam[e];
+            for (uint32_t e = 0; e < 3; ++e) o[(12 + 3 * g.p + e) * stride] = lam[e];
+        }
     }
     s.ln = lam[0];
     s.l1 = lam[1];
     s.l2 = lam[2];
-    for (uint32_t q = 0; q < l.npts; ++q) {
-        if (g.p == q) pointForward(l.n, l.mu, c, imA, imB, l.sA, l.sB, s);
-        if (q + 1 < l.npts) shareVelocities(g, s, q);
+    for (uint32_t q = 0; q < turns; ++q) {
+        if (act && g.p == q && q < l.npts) pointForward(l.n, l.mu, c, imA, imB, l.sA, l.sB, s);
+        if (q + 1 < turns) shareVelocities(g, s, q, dynA);
     }
-    lam[0] = s.ln;
-    lam[1] = s.l1;
-    lam[2] = s.l2;
-    if (g.p + 1 == l.npts) storePair(l, v, w, s);
+    if (act) {
+        lam[0] = s.ln;
+        lam[1] = s.l1;
+        lam[2] = s.l2;
+        if (g.p + 1 == turns) storePair(l, v, w, s);
+    }
 }
 
 // ------------------------------------------------------------------ forward --
-// dyn: sharedBytes(n) bytes, aligned to 16.
-__device__ __forceinline__ void forwardStepBlock(const WorldParams<F> &W, const StateView<F> &in,
-                                                 const CacheView<F> &cin, const StateView<F> &out,
-                                                 const CacheView<F> &cout, const StepScratch<F> &sc, bool record,
-                                                 unsigned char *dyn, BlockScratch &sh) {
+// The step is two calls, so that the iterations' registers are not shared with
+// the narrowphase's.
+//
+// Bodies to ordered manifolds, cache slots and (in v, w) velocities in front of
+// the solve.
+__device__ __noinline__ void contactsBlock(BlockWorld &bw) {
+    const WorldParams<F> &W = bw.W;
+    const StateView<F> &in = bw.in, &out = bw.out;
+    const CacheView<F> &cout = bw.cout;
+    const StepScratch<F> &sc = bw.sc;
+    unsigned char *const dyn = bw.dyn;
+    BlockWorld &sh = bw;
     const uint32_t tid = threadIdx.x, nt = blockDim.x, n = W.n;
     const uint32_t lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const uint32_t sortKeys = sharedSortKeys(n);
@@ -556,18 +596,22 @@ __device__ __forceinline__ void forwardStepBlock(const WorldParams<F> &W, const 
         *cout.count = entryTotal < cout.cap ? entryTotal : cout.cap;
     }
     // velocities into shared memory
-    F *v = out.v, *w = out.w;
     if (staged) {
-        v = reinterpret_cast<F *>(dyn);
-        w = v + 3 * n;
+        F *v = reinterpret_cast<F *>(dyn), *w = v + 3 * n;
         for (uint32_t i = tid; i < 3 * n; i += nt) {
             v[i] = out.v[i];
             w[i] = out.w[i];
         }
     }
     __syncthreads();
+}
 
-    // 5.-7. prepare, warm start, velocity iterations
+// Prepare, warm start, velocity iterations, warm-start cache.
+__device__ __noinline__ void solveStepBlock(const BlockWorld &bw, bool record, F *v, F *w) {
+    const WorldParams<F> &W = bw.W;
+    const CacheView<F> &cout = bw.cout;
+    const StepScratch<F> &sc = bw.sc;
+    const uint32_t M = sc.counts[1], C = sc.counts[2];
     const Group g = laneGroup();
     const size_t K = W.maxManifolds, KP = 4 * K;
     const uint32_t rounds = (uint32_t)W.iterations;
@@ -596,24 +640,23 @@ __device__ __forceinline__ void forwardStepBlock(const WorldParams<F> &W, const 
         // a group for every manifold: its data stay in registers
         const bool live = g.id < M;
         ManifoldLane l{};
-        PreparedLane o;
+        PreparedLane o{};
         uint32_t color = 0;
         if (live) {
-            l = loadManifold(W, sc, g, g.id);
+            l = loadManifold(bw, g, g.id);
             color = sc.color[l.m];
-            prepareLane(W, in, cin, out, sc, l, g, o);
+            prepareLane(bw, l, g, o);
             if (record) keep(l, o);
         }
         __syncthreads();  // every manifold has read the velocities
         for (uint32_t c = 0; c < C; ++c) {
-            if (live && color == c) warmGroup(g, l, o.c, o.lam, o.match, o.IA, o.IB, o.imA, o.imB, v, w);
+            warmGroup(g, live && color == c, l, o.c, o.lam, o.match, o.IA, o.IB, o.imA, o.imB, v, w);
             __syncthreads();
         }
         for (uint32_t it = 0; it < rounds; ++it)
             for (uint32_t c = 0; c < C; ++c) {
-                if (live && color == c)
-                    solveGroup(g, l, o.c, o.lam, o.imA, o.imB, v, w,
-                               record ? sc.tape + it * (kTapeScalars * K) : nullptr, K);
+                solveGroup(g, live && color == c, l, o.c, o.lam, o.imA, o.imB, v, w,
+                           record ? sc.tape + it * (kTapeScalars * K) : nullptr, K);
                 __syncthreads();
             }
         if (live) {
@@ -622,9 +665,9 @@ __device__ __forceinline__ void forwardStepBlock(const WorldParams<F> &W, const 
         }
     } else {
         for (uint32_t k = g.id; k < M; k += g.count) {
-            const ManifoldLane l = loadManifold(W, sc, g, k);
+            const ManifoldLane l = loadManifold(bw, g, k);
             PreparedLane o;
-            prepareLane(W, in, cin, out, sc, l, g, o);
+            prepareLane(bw, l, g, o);
             keep(l, o);
             storeFields(o.lam, sc.lam, KP, l.kp);
         }
@@ -632,8 +675,10 @@ __device__ __forceinline__ void forwardStepBlock(const WorldParams<F> &W, const 
         for (uint32_t pass = 0; pass < rounds + 1; ++pass)
             for (uint32_t c = 0; c < C; ++c) {
                 const uint32_t end = sc.colorStart[c + 1];
-                for (uint32_t k = sc.colorStart[c] + g.id; k < end; k += g.count) {
-                    const ManifoldLane l = loadManifold(W, sc, g, k);
+                for (uint32_t k0 = sc.colorStart[c]; k0 < end; k0 += g.count) {
+                    const bool act = k0 + g.id < end;  // a group past the end idles on the last manifold
+                    const uint32_t k = act ? k0 + g.id : end - 1;
+                    const ManifoldLane l = loadManifold(bw, g, k);
                     F cc[kPreparedScalars], lam[3];
                     loadFields(cc, sc.pp, KP, l.kp);
                     loadFields(lam, sc.lam, KP, l.kp);
@@ -642,24 +687,33 @@ __device__ __forceinline__ void forwardStepBlock(const WorldParams<F> &W, const 
                         F ia[9], ib[9];
                         loadFields(ia, sc.pm, K, k);
                         loadFields(ib, sc.pm + 9 * K, K, k);
-                        warmGroup(g, l, cc, lam, sc.match[l.kp], ldm(ia), ldm(ib), imA, imB, v, w);
+                        warmGroup(g, act, l, cc, lam, sc.match[l.kp], ldm(ia), ldm(ib), imA, imB, v, w);
                     } else {
-                        solveGroup(g, l, cc, lam, imA, imB, v, w,
+                        solveGroup(g, act, l, cc, lam, imA, imB, v, w,
                                    record ? sc.tape + (pass - 1) * (kTapeScalars * K) : nullptr, K);
-                        storeFields(lam, sc.lam, KP, l.kp);
+                        if (act) storeFields(lam, sc.lam, KP, l.kp);
                     }
                 }
                 __syncthreads();
             }
         for (uint32_t k = g.id; k < M; k += g.count) {
-            const ManifoldLane l = loadManifold(W, sc, g, k);
+            const ManifoldLane l = loadManifold(bw, g, k);
             F lam[3];
             loadFields(lam, sc.lam, KP, l.kp);
             writeCache(l, lam);
         }
     }
     __syncthreads();
+}
 
+__device__ __forceinline__ void forwardStepBlock(BlockWorld &bw, bool record) {
+    const WorldParams<F> &W = bw.W;
+    const StateView<F> &in = bw.in, &out = bw.out;
+    const uint32_t tid = threadIdx.x, nt = blockDim.x, n = W.n;
+    contactsBlock(bw);
+    const bool staged = n <= kStageBodies;
+    F *v = staged ? reinterpret_cast<F *>(bw.dyn) : out.v, *w = staged ? v + 3 * n : out.w;
+    solveStepBlock(bw, record, v, w);
     // 8. pose integration
     for (uint32_t i = tid; i < n; i += nt) {
         V3<F> pos = ld3(in.x, i);
@@ -686,11 +740,13 @@ struct AdjointLane {
 };
 constexpr int kAdjointExtra = 6;  // an, amu, aimA, aimB: kept with ac where a group takes several manifolds
 
-// One velocity update of one manifold in reverse.  lam: the impulses before it,
+// One velocity update of one manifold a group in reverse (act as above).  lam: the impulses before it,
 // lamPost: after it; tape: the velocities before it.
-__device__ __forceinline__ void reverseGroup(const Group &g, const ManifoldLane &l, const F *c, const F (&lam)[3],
-                                             const F (&lamPost)[3], F imA, F imB, const F *tape, size_t stride,
-                                             F *av, F *aw, AdjointLane &r) {
+__device__ __forceinline__ void reverseGroup(const Group &g, bool act, const ManifoldLane &l, const F *c,
+                                             const F (&lam)[3], const F (&lamPost)[3], F imA, F imB, const F *tape,
+                                             size_t stride, F *av, F *aw, AdjointLane &r) {
+    const uint32_t turns = warpTurns(act, l.npts);
+    const bool dynA = __any_sync(kWarp, act && !l.sA);
     // velocities in front of every point: the impulses' differences, applied as
     // the forward pass did
     PointIn<F> cur, in;
@@ -700,9 +756,9 @@ __device__ __forceinline__ void reverseGroup(const Group &g, const ManifoldLane 
         cur = PointIn<F>{pv(t, 0), pv(t, 1), pv(t, 2), pv(t, 3), lam[0], lam[1], lam[2]};
     }
     in = cur;
-    const bool live = g.p < l.npts;
-    for (uint32_t q = 0; q + 1 < l.npts; ++q) {
-        if (g.p == q && !(c[kPIem] <= 0.0f)) {
+    const bool live = act && g.p < l.npts;
+    for (uint32_t q = 0; q + 1 < turns; ++q) {
+        if (g.p == q && live && !(c[kPIem] <= 0.0f)) {
             const F applied = lamPost[0] - lam[0];
             const V3<F> impulse = l.n * applied;
             if (!l.sA) {
@@ -726,23 +782,32 @@ __device__ __forceinline__ void reverseGroup(const Group &g, const ManifoldLane 
                 }
             }
         }
-        shareVelocities(g, cur, q);
+        shareVelocities(g, cur, q, dynA);
         if (g.p == q + 1) in = cur;
     }
     // the intermediates of all points at once
     PointMid<F> mid;
-    mid.live = false;
+    mid.live = mid.fric = false;
     if (live) mid = pointMid(l.n, l.mu, c, in);
     // the adjoints, point after point
-    const V3<F> z{0.0f, 0.0f, 0.0f};
-    PointIn<F> a{l.sA ? z : ld3(av, l.a), l.sA ? z : ld3(aw, l.a), l.sB ? z : ld3(av, l.b), l.sB ? z : ld3(aw, l.b),
-                 r.alam[0], r.alam[1], r.alam[2]};
-    PointAdj<F> adj;
-    for (int q = (int)l.npts - 1; q >= 0; --q) {
-        if (g.p == (uint32_t)q) adj = pointChain(l.n, c, imA, imB, l.sA, l.sB, mid, a);
-        if (q > 0) shareVelocities(g, a, (uint32_t)q);
+    PointIn<F> a{};
+    if (act && !l.sA) {
+        a.vA = ld3(av, l.a);
+        a.wA = ld3(aw, l.a);
     }
-    if (g.p == 0) storePair(l, av, aw, a);
+    if (act && !l.sB) {
+        a.vB = ld3(av, l.b);
+        a.wB = ld3(aw, l.b);
+    }
+    a.ln = r.alam[0];
+    a.l1 = r.alam[1];
+    a.l2 = r.alam[2];
+    PointAdj<F> adj{};
+    for (int q = (int)turns - 1; q >= 0; --q) {
+        if (g.p == (uint32_t)q && live) adj = pointChain(l.n, c, imA, imB, l.sA, l.sB, mid, a);
+        if (q > 0) shareVelocities(g, a, (uint32_t)q, dynA);
+    }
+    if (act && g.p == 0) storePair(l, av, aw, a);
     if (live) {
         r.alam[0] = a.ln;
         r.alam[1] = a.l1;
@@ -755,11 +820,17 @@ __device__ __forceinline__ void reverseGroup(const Group &g, const ManifoldLane 
 // reverse; body adjoints are added to with atomics (av, aw: where the
 // velocities' adjoints stand; adj.dv, adj.dw: where new ones go, since other
 // manifolds still read av, aw).
-__device__ __noinline__ void geometryGroup(const WorldParams<F> &W, const StateView<F> &in, const CacheView<F> &cin,
-                                           const StepScratch<F> &sc, const AdjointView<F> &adj, const F *av,
-                                           const F *aw, const Group &g, const ManifoldLane &l, AdjointLane &r) {
+// A call, with its arguments by value: it needs twice the registers of the
+// iterations, and what a call takes by reference leaves the registers.
+__device__ __noinline__ void geometryGroup(const BlockWorld &bw, const F *av, const F *aw, const Group g, bool act,
+                                           const ManifoldLane l, AdjointLane r) {
+    const WorldParams<F> &W = bw.W;
+    const StateView<F> &in = bw.in;
+    const CacheView<F> &cin = bw.cin;
+    const StepScratch<F> &sc = bw.sc;
+    const AdjointView<F> &adj = bw.adj;
     const size_t K = W.maxManifolds, KP = 4 * K;
-    const bool live = g.p < l.npts;
+    const bool live = act && g.p < l.npts;
     F pm[kPmScalars], c[kPreparedScalars];
     loadFields(pm, sc.pm, K, l.k);
     loadFields(c, sc.pp, KP, l.kp);
@@ -797,16 +868,16 @@ __device__ __noinline__ void geometryGroup(const WorldParams<F> &W, const StateV
         inverseInertiaAdj(tA.q, ld3(W.iinv, l.a), gr.IA, gr.qA);
         inverseInertiaAdj(tB.q, ld3(W.iinv, l.b), gr.IB, gr.qB);
     }
-    gn = groupSum(g, gn);
-    if (g.p == 0 && shapeA == 1 && shapeB == 1)
+    gn = groupSum(gn);
+    if (act && g.p == 0 && shapeA == 1 && shapeB == 1)
         boxNormalReverse(tA, tB, (sc.mFeature[4 * l.m] & kAdAxisMask) >> kAdAxisShift, l.n, gn, gA, gB);
     // sums over the points; lane 0 and 1 add body A's, 2 and 3 body B's
-    const F rest = groupSum(g, gr.rest), amu = groupSum(g, live ? r.amu : 0.0f);
+    const F rest = groupSum(gr.rest), amu = groupSum(live ? r.amu : 0.0f);
     auto body = [&](uint32_t i, bool isStatic, bool low, const Tf<F> &t, const Q<F> &gq, const V3<F> &lin,
                     const V3<F> &ang, F aim, F im) {
-        const V3<F> x = groupSum(g, t.p), dv = groupSum(g, lin), dw = groupSum(g, ang);
-        const F qx = groupSum(g, t.q.x + gq.x), qy = groupSum(g, t.q.y + gq.y), qz = groupSum(g, t.q.z + gq.z),
-                qw = groupSum(g, t.q.w + gq.w), m = groupSum(g, aim);
+        const V3<F> x = groupSum(t.p), dv = groupSum(lin), dw = groupSum(ang);
+        const F qx = groupSum(t.q.x + gq.x), qy = groupSum(t.q.y + gq.y), qz = groupSum(t.q.z + gq.z),
+                qw = groupSum(t.q.w + gq.w), m = groupSum(aim);
         if (isStatic) return;
         if (low) {
             atomicAdd(&adj.ax[3 * i], x.x);
@@ -826,9 +897,9 @@ __device__ __noinline__ void geometryGroup(const WorldParams<F> &W, const StateV
             atomicAdd(&adj.amass[i], -(m * im * im));  // im = 1 / mass
         }
     };
-    body(l.a, l.sA || g.p > 1, g.p == 0, gA, gr.qA, gr.linA, gr.angA, gr.imA, imA);
-    body(l.b, l.sB || g.p < 2, g.p == 2, gB, gr.qB, gr.linB, gr.angB, gr.imB, imB);
-    if (g.p == 0) {
+    body(l.a, !act || l.sA || g.p > 1, g.p == 0, gA, gr.qA, gr.linA, gr.angA, gr.imA, imA);
+    body(l.b, !act || l.sB || g.p < 2, g.p == 2, gB, gr.qB, gr.linB, gr.angB, gr.imB, imB);
+    if (act && g.p == 0) {
         // restitution = max(ra, rb), friction = sqrt(max(fa, 0) * max(fb, 0))
         if (W.rest[l.a] < W.rest[l.b]) {
             if (!l.sB) atomicAdd(&adj.arest[l.b], rest);
@@ -847,17 +918,19 @@ __device__ __noinline__ void geometryGroup(const WorldParams<F> &W, const StateV
 // last: the step is the rollout's last (its impulses have no adjoint);
 // otherwise adj.acache holds the adjoint of the step's output cache on entry.
 // It holds that of the input cache on exit.
-__device__ __forceinline__ void backwardStepBlock(const WorldParams<F> &W, const StateView<F> &in,
-                                                  const CacheView<F> &cin, const StateView<F> &out,
-                                                  const StepScratch<F> &sc, const AdjointView<F> &adj, bool last,
-                                                  unsigned char *dyn) {
+__device__ __noinline__ void backwardStepBlock(const BlockWorld &bw, bool last) {
+    const WorldParams<F> &W = bw.W;
+    const StateView<F> &in = bw.in, &out = bw.out;
+    const CacheView<F> &cin = bw.cin;
+    const StepScratch<F> &sc = bw.sc;
+    const AdjointView<F> &adj = bw.adj;
     const uint32_t tid = threadIdx.x, nt = blockDim.x, n = W.n;
     const uint32_t M = sc.counts[1], C = sc.counts[2];
     const size_t K = W.maxManifolds, KP = 4 * K;
     const Group g = laneGroup();
     const bool resident = M <= g.count;  // a group for every manifold
     const bool staged = n <= kStageBodies;
-    F *av = staged ? reinterpret_cast<F *>(dyn) : adj.av, *aw = staged ? av + 3 * n : adj.aw;
+    F *av = staged ? reinterpret_cast<F *>(bw.dyn) : adj.av, *aw = staged ? av + 3 * n : adj.aw;
     // 1. pose integration; adjoints of the velocities into shared memory
     for (uint32_t i = tid; i < n; i += nt) {
         V3<F> v = ld3(adj.av, i), w = ld3(adj.aw, i);
@@ -879,7 +952,7 @@ __device__ __forceinline__ void backwardStepBlock(const WorldParams<F> &W, const
     };
     const uint32_t cacheN = *cin.count;
     ManifoldLane l{};
-    AdjointLane r;
+    AdjointLane r{};
     uint32_t color = 0;
     const bool live = g.id < M;
     auto clear = [&](AdjointLane &x) {
@@ -907,7 +980,7 @@ __device__ __forceinline__ void backwardStepBlock(const WorldParams<F> &W, const
     };
     if (resident) {
         if (live) {
-            l = loadManifold(W, sc, g, g.id);
+            l = loadManifold(bw, g, g.id);
             color = sc.color[l.m];
             clear(r);
             finalImpulses(l.kp, r.alam);
@@ -927,25 +1000,27 @@ __device__ __forceinline__ void backwardStepBlock(const WorldParams<F> &W, const
     for (int it = W.iterations - 1; it >= 0; --it) {
         const F *tape = sc.tape + (size_t)it * (kTapeScalars * K);
         const bool lastIt = it + 1 == W.iterations;
-        auto one = [&](const ManifoldLane &ml, AdjointLane &x) {
+        auto one = [&](bool act, const ManifoldLane &ml, AdjointLane &x) {
             F c[kPreparedScalars], lam[3], lamPost[3];
             loadFields(c, sc.pp, KP, ml.kp);
             loadFields(lam, tape + (12 + 3 * g.p) * K, K, ml.k);
             if (lastIt) loadFields(lamPost, sc.lam, KP, ml.kp);
             else loadFields(lamPost, tape + (kTapeScalars + 12 + 3 * g.p) * K, K, ml.k);
-            reverseGroup(g, ml, c, lam, lamPost, sc.pm[18 * K + ml.k], sc.pm[19 * K + ml.k], tape, K, av, aw, x);
+            reverseGroup(g, act, ml, c, lam, lamPost, sc.pm[18 * K + ml.k], sc.pm[19 * K + ml.k], tape, K, av, aw, x);
         };
         for (int ci = (int)C - 1; ci >= 0; --ci) {
             if (resident) {
-                if (live && color == (uint32_t)ci) one(l, r);
+                const bool act = live && color == (uint32_t)ci;
+                if (__any_sync(kWarp, act)) one(act, l, r);
             } else {
                 const uint32_t end = sc.colorStart[ci + 1];
-                for (uint32_t k = sc.colorStart[ci] + g.id; k < end; k += g.count) {
-                    const ManifoldLane ml = loadManifold(W, sc, g, k);
+                for (uint32_t k0 = sc.colorStart[ci]; k0 < end; k0 += g.count) {
+                    const bool act = k0 + g.id < end;
+                    const ManifoldLane ml = loadManifold(bw, g, act ? k0 + g.id : end - 1);
                     AdjointLane x;
                     loadAdjoint(ml.kp, x);
-                    one(ml, x);
-                    storeAdjoint(ml.kp, x);
+                    one(act, ml, x);
+                    if (act) storeAdjoint(ml.kp, x);
                 }
             }
             __syncthreads();
@@ -953,13 +1028,14 @@ __device__ __forceinline__ void backwardStepBlock(const WorldParams<F> &W, const
     }
     // 3. warm start, matching, preparation, geometry, materials
     if (resident) {
-        if (live) geometryGroup(W, in, cin, sc, adj, av, aw, g, l, r);
+        if (__any_sync(kWarp, live)) geometryGroup(bw, av, aw, g, live, l, r);
     } else {
-        for (uint32_t k = g.id; k < M; k += g.count) {
-            const ManifoldLane ml = loadManifold(W, sc, g, k);
+        for (uint32_t k0 = 0; k0 < M; k0 += g.count) {
+            const bool act = k0 + g.id < M;
+            const ManifoldLane ml = loadManifold(bw, g, act ? k0 + g.id : M - 1);
             AdjointLane x;
             loadAdjoint(ml.kp, x);
-            geometryGroup(W, in, cin, sc, adj, av, aw, g, ml, x);
+            geometryGroup(bw, av, aw, g, act, ml, x);
         }
     }
     __syncthreads();

@@ -569,7 +569,7 @@ template <class S> struct Prepared {
 constexpr int kPreparedScalars = 38;
 
 template <class S>
-AD_HDN void preparePoint(const V3<S> &n, const V3<S> &anchorA, const V3<S> &anchorB, const S &penetration,
+AD_HD void preparePoint(const V3<S> &n, const V3<S> &anchorA, const V3<S> &anchorB, const S &penetration,
                         const Q<S> &qA, const Q<S> &qB, const M3<S> &IA, const M3<S> &IB, const S &imA,
                         const S &imB, const V3<S> &linA, const V3<S> &angA, const V3<S> &linB, const V3<S> &angB,
                         const S &rest, const S &inverseDt, Prepared<S> &o) {
