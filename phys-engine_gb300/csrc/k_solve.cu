@@ -446,10 +446,7 @@ int maxCooperativeBlocks(int smCount) {
     static int perSm = -1;
     if (perSm < 0) {
         configureColor();
-        int a = 0;
-        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_color, kSolveThreads, kColorSmem));
-        const int b = solveIslandsBlocksPerSm();
-        perSm = a < b ? a : b;
+        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color, kSolveThreads, kColorSmem));
         if (perSm < 1) perSm = 1;
     }
     return perSm * smCount;
@@ -515,7 +512,7 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
         k_solve_serial<<<1, 32, 0, s>>>(a);
         PE_LAUNCHED();
     } else {
-        launchSolveIslands(a, coopBlocks, ws, s);
+        launchSolveIslands(a, ws, s);
     }
     k_impulses_out<<<gridFor(mcap), 256, 0, s>>>(a);
     PE_LAUNCHED();

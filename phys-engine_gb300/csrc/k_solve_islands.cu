@@ -22,12 +22,13 @@
 //                 after manifold in that order (a stack of two boxes would
 //                 leave 30 lanes idle); manifolds without a dynamic body
 //                 (nothing to share) are solved alone
-//   k_isl_solve_large : when some island has more than kIslBlockMax
-//                 manifolds (a settled pile), all islands together in
-//                 grid-wide colour sweeps instead: the manifolds bucketed by
-//                 colour, a grid barrier per colour.  Manifolds of one colour
-//                 share no dynamic body, so their order inside a colour does
-//                 not change the result.
+//   k_isl_sweep : when some island has more than kIslBlockMax manifolds (a
+//                 settled pile), all islands together over the whole grid: a
+//                 manifold's update starts as soon as the updates before it at
+//                 its two bodies are done (each body's velocities carry the
+//                 number of updates they have seen), with no barrier between
+//                 colours.  Every body sees its manifolds in (colour, index)
+//                 order, as in colour-by-colour sweeps, so the result is theirs.
 #include <stdexcept>
 
 #include "pe_block.cuh"
@@ -111,7 +112,7 @@ __device__ __forceinline__ uint32_t *islCnt(const SolveArgs &a) { return a.sb.is
 } // namespace
 
 // Per-body counts all zero (they are scanned into list offsets), every dynamic
-// endpoint its own island.
+// endpoint its own island and without colours.
 __global__ void k_isl_init(SolveArgs a) {
     const uint32_t M = min(*a.count, a.mcap);
     uint32_t *par = islPar(a), *cnt = islCnt(a);
@@ -122,8 +123,12 @@ __global__ void k_isl_init(SolveArgs a) {
     for (uint32_t i = t; i < wideC; i += stride) a.sb.colorStart[i] = 0u;
     for (uint32_t m = t; m < M; m += stride) {
         const uint32_t fl = a.sb.dyn[m];
-        if (fl & kFlagDynA) par[a.mv.bodyA[m]] = a.mv.bodyA[m];
-        if (fl & kFlagDynB) par[a.mv.bodyB[m]] = a.mv.bodyB[m];
+        for (int e = 0; e < 2; ++e) {
+            if (!(fl & (e ? kFlagDynB : kFlagDynA))) continue;
+            const uint32_t b = e ? a.mv.bodyB[m] : a.mv.bodyA[m];
+            par[b] = b;
+            a.sb.bodyUsed[2 * b] = a.sb.bodyUsed[2 * b + 1] = 0ull;  // colours of the sweeps, set by k_isl_fill
+        }
     }
 }
 
@@ -174,7 +179,15 @@ __global__ void k_isl_fill(SolveArgs a) {
         if (r == kIslNone) continue;
         a.sb.islList[a.sb.islOff[r] + a.sb.islSlot[m]] = m;
         const uint32_t c = a.sb.color[m];
-        if (cnt[r] >= sweepFrom && c < colorLimit) aggregatedAppendKeyed(colorCounts, c);
+        if (cnt[r] >= sweepFrom && c < colorLimit) {
+            aggregatedAppendKeyed(colorCounts, c);
+            if (!wideC) {
+                const uint32_t fl = a.sb.dyn[m], word = c >> 6;
+                const unsigned long long bit = 1ull << (c & 63);
+                if (fl & kFlagDynA) atomicOr(&a.sb.bodyUsed[2 * a.mv.bodyA[m] + word], bit);
+                if (fl & kFlagDynB) atomicOr(&a.sb.bodyUsed[2 * a.mv.bodyB[m] + word], bit);
+            }
+        }
     }
     // the warp queue: islands of 32 manifolds or more at the front (a warp's
     // lanes all busy; they bound the sweep), those of kIslThread to 31 from
@@ -349,10 +362,6 @@ __global__ void __launch_bounds__(kIslThreads) k_isl_solve(SolveArgs a) {
     }
 }
 
-// Large islands, all together: bucket their manifolds by colour (the
-// bucket lists live in islKeysTmp), then warm start and iterations colour by
-// colour with a grid barrier after each colour.  Every block reads the same
-// counts, so with no large island all return before the first barrier.
 // More than kMaxColors colours: every island in grid-wide sweeps, the
 // per-colour counts in sb.colorStart scanned into starts by block 0, then used
 // as fill cursors (after the fill, colorStart[c] is the end of colour c).
@@ -373,7 +382,7 @@ __device__ void islSolveWide(const SolveArgs &a, uint32_t M, uint32_t C) {
             __syncthreads();
         }
     }
-    if (!gridBarrier(a.sb.bar, &a.st->err)) return;
+    if (!gridBarrier(a.sb.bar + 1, &a.st->err)) return;
     const uint32_t *cnt = islCnt(a);
     uint32_t *list = reinterpret_cast<uint32_t *>(a.sb.islKeysTmp);
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
@@ -383,7 +392,7 @@ __device__ void islSolveWide(const SolveArgs &a, uint32_t M, uint32_t C) {
         if (r == kIslNone || cnt[r] == 0 || c >= C) continue;
         list[aggregatedAppendKeyed(cur, c)] = m;
     }
-    if (!gridBarrier(a.sb.bar, &a.st->err)) return;
+    if (!gridBarrier(a.sb.bar + 1, &a.st->err)) return;
     for (int pass = 0; pass <= a.iterations; ++pass)
         for (uint32_t c = 0; c < C; ++c) {
             const uint32_t lo = c ? __ldcg(&cur[c - 1]) : 0u, hi = __ldcg(&cur[c]);
@@ -391,88 +400,222 @@ __device__ void islSolveWide(const SolveArgs &a, uint32_t M, uint32_t C) {
                 if (pass == 0) warmStartOne(a, k, list[k]);
                 else solveOne(a, k, list[k]);
             }
-            if (!gridBarrier(a.sb.bar, &a.st->err)) return;
+            if (!gridBarrier(a.sb.bar + 1, &a.st->err)) return;
         }
 }
 
-// GlobalVel with the manifold's bodies already loaded.
-struct BodiesGiven {
-    const SolveArgs &a;
-    uint2 b;
-    __device__ __forceinline__ uint2 bodies(uint32_t, uint32_t) const { return b; }
-    __device__ __forceinline__ V3 lin(uint32_t i) const { return f4xyz(ld4(&a.w.nxt.lin[i])); }
-    __device__ __forceinline__ V3 ang(uint32_t i) const { return f4xyz(ld4(&a.w.nxt.ang[i])); }
-    __device__ __forceinline__ void store(uint32_t i, const V3 &l, const V3 &w) const {
-        st4(&a.w.nxt.lin[i], make4(l, 0.0f));
-        st4(&a.w.nxt.ang[i], make4(w, 0.0f));
-    }
-};
-
-// Grid-wide sweeps: each thread keeps one shared-memory slot holding the
-// prepared data of its manifold of the coming colour step (the manifold's
-// normal and masses, then per point the ten prepared vectors and the
-// impulse), laid out field-major across the block's threads.  The copy is
-// issued (cp.async) as soon as the thread has finished its manifold of the
-// current step, so it lands while the grid waits at the colour barrier; after
-// the barrier only the body velocities are loaded from memory.
-constexpr uint32_t kSlotPoint = kPreparedVec4 + 1;                 // prepared vectors + impulse
-constexpr uint32_t kSlotVec4 = 2 + 4 * kSlotPoint;                 // pm, pn, 4 points
-constexpr size_t kLargeSmem = (size_t)kSlotVec4 * kSolveThreads * sizeof(float4);  // 188,416 bytes
-// List entries of the grid-wide sweeps: manifold index | solved points << 29.
+// ----------------------------------------------------------------- sweeps ---
+// A body's velocity vectors carry in .w how many updates the body has seen this
+// solve (0 as the integrate kernel leaves them; the body's last update writes 0
+// again).  The update of pass p at a manifold whose colour has r lower colours
+// among the body's d waits for p d + r and leaves p d + r + 1: data and flag are
+// one 16-byte word, read and written whole, so no fence or barrier goes with it.
+//
+// A warp takes eight manifolds of one colour, four lanes each, one lane a
+// contact point: the point's constants and impulses stay in the lane's registers
+// for the whole solve, the velocities move from lane to lane as the points follow
+// one another, and lane r loads and stores vector r (linear and angular velocity
+// of body A, then of B).  All eight start together once their sixteen bodies are
+// ready; what they wait for has an earlier (pass, colour), so with every warp
+// resident (cooperative launch) and each taking its items in that order some warp
+// can always go on.  With more items than warps a warp reloads the constants.
+//
+// What bounds it is the chain of updates at the busiest bodies: 9 or 21 passes x
+// 8 colours in the piles below, an update about 0.45 us a point and 0.5 us from
+// a store to the load that sees it.  Measured against a grid barrier after each
+// colour (4.0 us a colour step), us a whole step: field of 10,000 bodies (18,000
+// manifolds) 568 -> 428, of 50,000 (84,000, several items a warp) 840 -> 700; 16
+// pyramids with hulls (7,000) 1,056 -> 692, 256 of them (110,000) 1,829 -> 1,373.
+constexpr uint32_t kWarp = 0xffffffffu;
+constexpr uint32_t kItemManifolds = 8;
+// List entries: manifold index | solved points << 29.
 constexpr uint32_t kEntryShift = 29;
 constexpr uint32_t kEntryMask = (1u << kEntryShift) - 1u;
+constexpr uint32_t kNoEntry = 0xFFFFFFFFu;  // (a manifold has at most four points)
 
-__device__ __forceinline__ void cpAsync16(float4 *dst, const float4 *src) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+// 16 bytes read or written in one access at device scope.
+__device__ __forceinline__ float4 loadWord(const float4 *p) {
+    unsigned __int128 v;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
+    return make_float4(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)),
+                       __uint_as_float((uint32_t)(v >> 64)), __uint_as_float((uint32_t)(v >> 96)));
 }
-__device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cpAsyncWaitAll() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// slot: this thread's column (s_slot + threadIdx.x), stride kSolveThreads.
-__device__ __forceinline__ void fetchSlot(const SolveArgs &a, float4 *slot, uint32_t m, uint32_t npts) {
-    const uint32_t mcap = a.mcap;
-    cpAsync16(slot, &a.sb.pm[m]);
-    cpAsync16(slot + kSolveThreads, &a.sb.pn[m]);
-    for (uint32_t p = 0; p < npts; ++p) {
-        float4 *d = slot + (size_t)(2 + p * kSlotPoint) * kSolveThreads;
-#pragma unroll
-        for (uint32_t v = 0; v < (uint32_t)kPreparedVec4; ++v)
-            cpAsync16(d + (size_t)v * kSolveThreads, &a.sb.pp[(size_t)(v * 4 + p) * mcap + m]);
-        cpAsync16(d + (size_t)kPreparedVec4 * kSolveThreads, &a.sb.pimp[(size_t)p * mcap + m]);
-    }
-    cpAsyncCommit();
+__device__ __forceinline__ void storeWord(float4 *p, const V3 &v, uint32_t tag) {
+    const unsigned long long lo = ((unsigned long long)__float_as_uint(v.y) << 32) | __float_as_uint(v.x),
+                             hi = ((unsigned long long)tag << 32) | __float_as_uint(v.z);
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(((unsigned __int128)hi << 64) | lo) : "memory");
 }
 
-// Prepared data of one manifold from this thread's slot; impulses are written
-// back to the solver arrays (the slot is refilled for every colour step).
-struct SlotPrep {
-    const SolveArgs &a;
-    const float4 *slot;
+// One lane's share of a manifold.
+struct SweepLane {
+    float4 o[kPreparedVec4], imp;  // the lane's point
+    V3 n;
+    float friction, imA, imB;
     uint32_t m, npts;
-    __device__ __forceinline__ float4 pm(uint32_t) const { return slot[0]; }
-    __device__ __forceinline__ float4 pn(uint32_t) const { return slot[kSolveThreads]; }
-    __device__ __forceinline__ uint32_t count(uint32_t) const { return npts; }
-    __device__ __forceinline__ float4 inertia(int r, uint32_t) const {
-        return a.sb.pmInertia[(size_t)r * a.mcap + m];
-    }
-    __device__ __forceinline__ float4 pt(int v, uint32_t p, uint32_t) const {
-        return slot[(size_t)(2 + p * kSlotPoint + v) * kSolveThreads];
-    }
-    __device__ __forceinline__ float4 imp(uint32_t p, uint32_t) const {
-        return slot[(size_t)(2 + p * kSlotPoint + kPreparedVec4) * kSolveThreads];
-    }
-    __device__ __forceinline__ void setImp(uint32_t p, uint32_t, const float4 &v) const {
-        a.sb.pimp[(size_t)p * a.mcap + m] = v;
-    }
+    bool act, sA, sB;  // the group has a manifold; its bodies are static
+    // the lane's velocity vector: where it is, whether its updates are counted
+    // (a moving body), whether it is written, lower colours and colours there
+    float4 *addr;
+    bool counted, writes;
+    uint32_t rank, degree;
 };
 
-__global__ void __launch_bounds__(kSolveThreads) k_isl_solve_large(SolveArgs a) {
-    __shared__ uint32_t s_start[kMaxColors + 1];
-    __shared__ uint32_t s_colors[kMaxColors], s_colorN;
-    extern __shared__ float4 s_slot[];
+__device__ __forceinline__ void loadSweepLane(const SolveArgs &a, uint32_t entry, uint32_t p, SweepLane &f) {
+    f.act = entry != kNoEntry;
+    f.m = f.act ? entry & kEntryMask : 0u;
+    f.npts = f.act ? entry >> kEntryShift : 0u;
+    const SolverBuffers &sb = a.sb;
+    const float4 pm = sb.pm[f.m], pn = sb.pn[f.m];
+    const uint2 b = sb.pbody[f.m];
+    const uint32_t fl = sb.dyn[f.m], c = sb.color[f.m];
+    f.n = f4xyz(pn);
+    f.friction = pn.w;
+    f.imA = pm.x;
+    f.imB = pm.z;
+    f.sA = pm.y != 0.0f;
+    f.sB = pm.w != 0.0f;
+    if (p < f.npts) {
+#pragma unroll
+        for (uint32_t v = 0; v < (uint32_t)kPreparedVec4; ++v) f.o[v] = sb.pp[(size_t)(v * 4 + p) * a.mcap + f.m];
+        f.imp = sb.pimp[(size_t)p * a.mcap + f.m];
+    }
+    const uint32_t body = p < 2 ? b.x : b.y;
+    f.addr = (p & 1u ? a.w.nxt.ang : a.w.nxt.lin) + body;
+    f.counted = f.act && (fl & (p < 2 ? kFlagDynA : kFlagDynB)) != 0;
+    f.writes = f.act && !(p < 2 ? f.sA : f.sB);
+    f.rank = f.degree = 0;
+    if (f.counted) {
+        const unsigned long long u0 = __ldcg(&sb.bodyUsed[2 * body]), u1 = __ldcg(&sb.bodyUsed[2 * body + 1]);
+        f.degree = (uint32_t)(__popcll(u0) + __popcll(u1));
+        const unsigned long long below = (1ull << (c & 63)) - 1ull;
+        f.rank = c < 64 ? (uint32_t)__popcll(u0 & below) : (uint32_t)(__popcll(u0) + __popcll(u1 & below));
+    }
+}
+
+__device__ __forceinline__ V3 shfl3(const V3 &v, uint32_t from) {
+    return {__shfl_sync(kWarp, v.x, from), __shfl_sync(kWarp, v.y, from), __shfl_sync(kWarp, v.z, from)};
+}
+
+// The update of pass `pass` (0: the warm start) of the warp's eight manifolds.
+// False when the wait for their bodies ran out.
+__device__ __forceinline__ bool sweepVisit(const SolveArgs &a, SweepLane &f, uint32_t pass, uint32_t passes) {
+    const uint32_t lane = threadIdx.x & 31, p = lane & 3, first = lane & ~3u;
+    const uint32_t want = pass * f.degree + f.rank;
+    float4 own = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    bool ready = !f.act;
+    for (uint32_t spins = 0;;) {
+        if (!ready) {
+            own = loadWord(f.addr);
+            ready = !f.counted || __float_as_uint(own.w) == want;
+        }
+        if (__all_sync(kWarp, ready)) break;
+        if (++spins > spinLimit() || ((spins & 1023u) == 0 && (ldvol(&a.st->err) & kErrTimeout))) {
+            if (lane == 0) atomicOr(&a.st->err, kErrTimeout);
+            return false;
+        }
+    }
+    const V3 v = f4xyz(own);
+    V3 linA = shfl3(v, first), angA = shfl3(v, first + 1), linB = shfl3(v, first + 2), angB = shfl3(v, first + 3);
+    const bool movesA = __any_sync(kWarp, f.act && !f.sA);  // some group's body A (often the floor) moves
+    const uint32_t turns = __reduce_max_sync(kWarp, f.npts);
+    M3 IA, IB;
+    if (pass == 0 && p < f.npts && f.imp.w != 0.0f) {
+        float4 r[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) r[j] = a.sb.pmInertia[(size_t)j * a.mcap + f.m];
+        IA = M3{r[0].x, r[0].y, r[0].z, r[1].x, r[1].y, r[1].z, r[2].x, r[2].y, r[2].z};
+        IB = M3{r[3].x, r[3].y, r[3].z, r[4].x, r[4].y, r[4].z, r[5].x, r[5].y, r[5].z};
+    }
+    for (uint32_t q = 0; q < turns; ++q) {
+        if (p == q && q < f.npts) {
+            const float4(&o)[kPreparedVec4] = f.o;
+            const V3 offA = f4xyz(o[0]), offB = f4xyz(o[1]), t1 = f4xyz(o[2]), t2 = f4xyz(o[3]);
+            if (pass == 0) {
+                // warmStartOne's application
+                if (f.imp.w != 0.0f) {
+                    const V3 wi = f.n * f.imp.x + t1 * f.imp.y + t2 * f.imp.z;
+                    const V3 nw = -wi;
+                    if (!f.sA) {
+                        linA += nw * f.imA;
+                        angA += mul(IA, cross(offA, nw));
+                    }
+                    if (!f.sB) {
+                        linB += wi * f.imB;
+                        angB += mul(IB, cross(offB, wi));
+                    }
+                }
+            } else if (!(o[0].w <= 0.0f)) {
+                // solveOne's update, operation for operation
+                const float iem = o[0].w, bias = o[1].w, rv = o[2].w, itm00 = o[3].w, itm01 = o[4].w, itm11 = o[5].w;
+                const V3 vA = linA + cross(angA, offA);
+                const V3 vB = linB + cross(angB, offB);
+                const V3 rel = vB - vA;
+                const float vn = dot(rel, f.n);
+                const float delta = -(vn + rv - bias) / iem;
+                const float prev = f.imp.x;
+                f.imp.x = smax(prev + delta, 0.0f);
+                const float applied = f.imp.x - prev;
+                const V3 impulse = f.n * applied;
+                if (!f.sA) {
+                    linA += (-impulse) * f.imA;
+                    angA += f4xyz(o[4]) * (-applied);
+                }
+                if (!f.sB) {
+                    linB += impulse * f.imB;
+                    angB += f4xyz(o[5]) * applied;
+                }
+                if (!(itm00 <= 0.0f || itm11 <= 0.0f)) {
+                    const float limit = smax(f.friction, 0.0f) * f.imp.x;
+                    const float tv1 = dot(rel, t1) + o[6].w * applied;
+                    const float tv2 = dot(rel, t2) + o[7].w * applied;
+                    const float d1 = -(itm00 * tv1 + itm01 * tv2);
+                    const float d2 = -(itm01 * tv1 + itm11 * tv2);
+                    const float p1 = f.imp.y, p2 = f.imp.z;
+                    f.imp.y += d1;
+                    f.imp.z += d2;
+                    const float lsq = f.imp.y * f.imp.y + f.imp.z * f.imp.z;
+                    if (lsq > limit * limit) {
+                        const float sc = limit / sqrtf(lsq);
+                        f.imp.y *= sc;
+                        f.imp.z *= sc;
+                    }
+                    const float a1 = f.imp.y - p1, a2 = f.imp.z - p2;
+                    const V3 ti = t1 * a1 + t2 * a2;
+                    const V3 rA = f4xyz(o[6]) * a1 + f4xyz(o[8]) * a2;
+                    const V3 rB = f4xyz(o[7]) * a1 + f4xyz(o[9]) * a2;
+                    if (!f.sA) {
+                        linA += (-ti) * f.imA;
+                        angA += -rA;
+                    }
+                    if (!f.sB) {
+                        linB += ti * f.imB;
+                        angB += rB;
+                    }
+                }
+            }
+        }
+        // on to the next point's lane, and after the last to all four
+        if (movesA) {
+            linA = shfl3(linA, first + q);
+            angA = shfl3(angA, first + q);
+        }
+        linB = shfl3(linB, first + q);
+        angB = shfl3(angB, first + q);
+    }
+    const V3 out = p == 0 ? linA : p == 1 ? angA : p == 2 ? linB : angB;
+    if (f.counted) {
+        const bool end = pass + 1 == passes && f.rank + 1 == f.degree;
+        storeWord(f.addr, out, end ? 0u : want + 1u);
+    } else if (f.writes) {
+        st4(f.addr, make4(out, 0.0f));
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(kSolveThreads, 2) k_isl_sweep(SolveArgs a) {
+    __shared__ uint32_t s_start[kMaxColors + 1];  // first item of each colour
+    const uint32_t M = min(*a.count, a.mcap);
     {
-        const uint32_t M = min(*a.count, a.mcap);
         const uint32_t wideC = islWideColors(a, M);
         if (wideC) {  // every block sees the same colour count
             islSolveWide(a, M, wideC);
@@ -485,13 +628,14 @@ __global__ void __launch_bounds__(kSolveThreads) k_isl_solve_large(SolveArgs a) 
         uint32_t acc = 0;
         for (int c = 0; c < kMaxColors; ++c) {
             s_start[c] = acc;
-            acc += count[c];
+            acc += (count[c] + kItemManifolds - 1) / kItemManifolds;
         }
         s_start[kMaxColors] = acc;
     }
     __syncthreads();
-    if (s_start[kMaxColors] == 0) return;
-    const uint32_t M = min(*a.count, a.mcap);
+    const uint32_t items = s_start[kMaxColors];
+    if (items == 0) return;
+    // the manifolds colour by colour, each colour from a whole item
     const uint32_t *cnt = islCnt(a);
     const uint32_t sweepFrom = islSweepFrom(a, M);
     uint32_t *list = reinterpret_cast<uint32_t *>(a.sb.islKeysTmp);
@@ -500,91 +644,49 @@ __global__ void __launch_bounds__(kSolveThreads) k_isl_solve_large(SolveArgs a) 
         const uint32_t r = a.sb.islRoot[m];
         const uint32_t c = a.sb.color[m];
         if (r == kIslNone || cnt[r] < sweepFrom || c >= (uint32_t)kMaxColors) continue;
-        list[s_start[c] + aggregatedAppendKeyed(fill, c)] = m | min(a.sb.pcount[m], 4u) << kEntryShift;
+        list[kItemManifolds * s_start[c] + aggregatedAppendKeyed(fill, c)] =
+            m | min(a.sb.pcount[m], 4u) << kEntryShift;
     }
-    // the non-empty colours, in order
-    if (threadIdx.x == 0) {
-        uint32_t n = 0;
-        for (int c = 0; c < kMaxColors; ++c)
-            if (s_start[c] != s_start[c + 1]) s_colors[n++] = (uint32_t)c;
-        s_colorN = n;
+    for (uint32_t c = gtid; c < (uint32_t)kMaxColors; c += gstride)
+        for (uint32_t i = kItemManifolds * s_start[c] + count[c]; i < kItemManifolds * s_start[c + 1]; ++i)
+            list[i] = kNoEntry;
+    if (!gridBarrier(a.sb.bar + 1, &a.st->err)) return;
+    const uint32_t lane = threadIdx.x & 31, p = lane & 3, passes = (uint32_t)a.iterations + 1u;
+    // items go round the blocks, so that a colour's are spread over every SM
+    const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
+    auto keepImpulse = [&](const SweepLane &f) {
+        if (p < f.npts) a.sb.pimp[(size_t)p * a.mcap + f.m] = f.imp;
+    };
+    if (items <= warps) {
+        if (warp >= items) return;
+        SweepLane f;
+        loadSweepLane(a, __ldcg(&list[kItemManifolds * warp + (lane >> 2)]), p, f);
+        for (uint32_t pass = 0; pass < passes; ++pass)
+            if (!sweepVisit(a, f, pass, passes)) return;
+        keepImpulse(f);
+        return;
     }
-    if (!gridBarrier(a.sb.bar, &a.st->err)) return;
-    // Colour steps in (pass, colour) order.  A thread's first manifold of a
-    // step is the same in every pass.  Its
-    // list entry is loaded while the step before is solved, its bodies and
-    // (passes after the warm start) its slot right after that step, before
-    // the barrier; further manifolds of the step (more than one per thread)
-    // read the solver arrays.
-    // Solve index j of a colour goes to block j % gridDim.x, thread j /
-    // gridDim.x: a colour's manifolds are spread over every SM of the grid
-    // (a thin colour keeps one warp per block busy, not a few full blocks).
-    const uint32_t nC = s_colorN;
-    const uint32_t nSteps = nC * (uint32_t)(a.iterations + 1);
-    const uint32_t lane = threadIdx.x * gridDim.x + blockIdx.x;
-    float4 *slot = s_slot + threadIdx.x;
-    const GlobalPrep gp{a};
-    auto firstIndex = [&](uint32_t step) { return s_start[s_colors[step % nC]] + lane; };
-    auto stepEnd = [&](uint32_t step) { return s_start[s_colors[step % nC] + 1]; };
-    uint32_t e = 0;
-    uint2 b = make_uint2(0u, 0u);
-    if (firstIndex(0) < stepEnd(0)) {
-        e = __ldcg(&list[firstIndex(0)]);
-        b = __ldcg(&a.sb.pbody[e & kEntryMask]);
-    }
-    for (uint32_t step = 0; step < nSteps; ++step) {
-        const uint32_t pass = step / nC;
-        const uint32_t k0 = firstIndex(step), end = stepEnd(step);
-        const bool next = step + 1 < nSteps && firstIndex(step + 1) < stepEnd(step + 1);
-        const uint32_t eNext = next ? __ldcg(&list[firstIndex(step + 1)]) : 0u;
-        if (k0 < end) {
-            const uint32_t m = e & kEntryMask;
-            const BodiesGiven v{a, b};
-            if (pass == 0) {
-                warmStartOne(gp, k0, m, v);
-            } else {
-                cpAsyncWaitAll();
-                solveOne(SlotPrep{a, slot, m, e >> kEntryShift}, k0, m, v);
-            }
-            for (uint32_t k = k0 + gstride; k < end; k += gstride) {
-                const uint32_t mk = __ldcg(&list[k]) & kEntryMask;
-                const BodiesGiven vk{a, __ldcg(&a.sb.pbody[mk])};
-                if (pass == 0) warmStartOne(gp, k, mk, vk);
-                else solveOneChained(gp, k, mk, vk);
-            }
+    for (uint32_t pass = 0; pass < passes; ++pass)
+        for (uint32_t item = warp; item < items; item += warps) {
+            SweepLane f;
+            loadSweepLane(a, __ldcg(&list[kItemManifolds * item + (lane >> 2)]), p, f);
+            if (!sweepVisit(a, f, pass, passes)) return;
+            keepImpulse(f);
         }
-        if (next) {
-            e = eNext;
-            b = __ldcg(&a.sb.pbody[e & kEntryMask]);
-            if ((step + 1) / nC > 0) fetchSlot(a, slot, e & kEntryMask, e >> kEntryShift);
-        }
-        if (!gridBarrier(a.sb.bar, &a.st->err)) {
-            cpAsyncWaitAll();  // no copy into shared memory outlives the block
-            return;
-        }
-    }
-    cpAsyncWaitAll();
 }
 
-namespace {
-void configureLargeSweeps() {
-    static bool configured = false;
-    if (!configured) {
-        PE_CHECK(cudaFuncSetAttribute(k_isl_solve_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kLargeSmem));
-        configured = true;
+// Blocks of k_isl_sweep that the device holds at once.
+static int sweepBlocks() {
+    static int perSm = -1;
+    if (perSm < 0) {
+        int b = 0;
+        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_isl_sweep, kSolveThreads, 0));
+        perSm = b < 1 ? 1 : b;
     }
-}
-} // namespace
-
-int solveIslandsBlocksPerSm() {
-    configureLargeSweeps();
-    int b = 0;
-    PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_isl_solve_large, kSolveThreads, kLargeSmem));
-    return b;
+    return perSm * smCount();
 }
 
-void launchSolveIslands(const SolveArgs &a, int coopBlocks, Scratch &ws, cudaStream_t s) {
+void launchSolveIslands(const SolveArgs &a, Scratch &ws, cudaStream_t s) {
     const uint32_t mcap = a.mcap;
     k_isl_init<<<islGrid(mcap), kIslThreads, 0, s>>>(a);
     PE_LAUNCHED();
@@ -601,20 +703,18 @@ void launchSolveIslands(const SolveArgs &a, int coopBlocks, Scratch &ws, cudaStr
     PE_LAUNCHED();
     // list entries carry the manifold index in kEntryShift bits
     if (mcap > kEntryMask) throw std::length_error("manifold capacity beyond the grid-wide sweeps' index range");
-    configureLargeSweeps();
     SolveArgs args = a;
     void *params[] = {&args};
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(coopBlocks);
+    cfg.gridDim = dim3(sweepBlocks());
     cfg.blockDim = dim3(kSolveThreads);
-    cfg.dynamicSmemBytes = kLargeSmem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PE_CHECK(cudaLaunchKernelExC(&cfg, (const void *)k_isl_solve_large, params));
+    PE_CHECK(cudaLaunchKernelExC(&cfg, (const void *)k_isl_sweep, params));
     PE_LAUNCHED();
 }
 

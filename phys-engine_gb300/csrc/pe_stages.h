@@ -97,7 +97,7 @@ struct SolverBuffers {
     unsigned long long *cacheKeys, *cacheKeysTmp;
     uint32_t *cacheVals, *cacheValsTmp;
     uint32_t *cacheCounts, *cacheOff;
-    uint32_t *bar;                  // grid barrier [2]
+    uint32_t *bar;                  // grid barriers [2]: colouring, island sweeps (grids of their own)
     uint32_t *counters;             // [4]
     // cluster solver: staging slots by solve index and the body of each slot
     // (colour-phase path); the manifolds of each island, kIslandMax entries
@@ -172,10 +172,10 @@ void launchExpandForces(const float *f3, const uint32_t *bflags, float4 *force, 
 struct SolveArgs;
 // The multi-kernel path's sweeps island by island (after k_color and prepare):
 // a thread, a warp or a block per island by its size; once an island is too
-// large for a block, every island in grid-wide colour sweeps (a cooperative
-// launch of at most coopBlocks blocks).
+// large for a block, every island in sweeps over the whole grid (a cooperative
+// launch).
 constexpr uint32_t kIslCounterWords = 10 + 2 * kMaxColors;
-void launchSolveIslands(const SolveArgs &a, int coopBlocks, Scratch &ws, cudaStream_t s);
+void launchSolveIslands(const SolveArgs &a, Scratch &ws, cudaStream_t s);
 void launchSleepWake(const WorldView &w, const ManifoldView &mv, uint32_t Mhost, uint32_t mcap, uint32_t *flags,
                      float *quiet, uint32_t *err, cudaStream_t s);
 void launchSleepContacts(const WorldView &w, const ManifoldView &mv, DevStats *st, uint32_t mcap, uint32_t *bflags,
@@ -247,8 +247,6 @@ struct ClusterSolveLayout {
 };
 constexpr uint32_t kBlockMaxBodies = 1u << 20;
 int maxCooperativeBlocks(int smCount);
-// Co-resident blocks per SM of the large islands' cooperative sweep kernel.
-int solveIslandsBlocksPerSm();
 void launchGeneratePairs(const float4 *in, float4 *out, uint32_t n, cudaStream_t s);
 
 } // namespace pe
