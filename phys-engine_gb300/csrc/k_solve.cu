@@ -17,6 +17,8 @@
 // with more manifolds sends the step to parallel rounds (Jones-Plassmann): a
 // manifold is coloured once it holds the highest priority among the uncoloured
 // manifolds at both its bodies; the same colouring.
+#include <algorithm>
+
 #include "pe_block.cuh"
 #include "pe_kernels.cuh"
 #include "pe_solve.cuh"
@@ -31,6 +33,14 @@ constexpr uint32_t kColorCached = 6;
 constexpr uint32_t kColorSlots = 2 * kIslandMax;
 constexpr uint32_t kNoNeighbour = 0xFFFFFFFFu;
 constexpr size_t kColorSmem = (size_t)kColorCached * kColorSlots * kSolveThreads * sizeof(uint32_t);  // 196,608 bytes
+
+// A manifold's colour into the masks of its dynamic bodies (colours below 64
+// in the first word).
+__device__ __forceinline__ void addToMasks(const SolveArgs &a, uint32_t m, uint32_t d, uint32_t c) {
+    const unsigned long long bit = 1ull << (c & 63);
+    if (d & 1u) atomicOr(&a.sb.bodyUsed[2 * a.mv.bodyA[m] + (c >> 6)], bit);
+    if (d & 2u) atomicOr(&a.sb.bodyUsed[2 * a.mv.bodyB[m] + (c >> 6)], bit);
+}
 
 __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
     extern __shared__ uint32_t s_hp[];  // [kColorCached][kColorSlots][blockDim.x]
@@ -63,8 +73,10 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
             __stcg(&incCount[bb], 0u);
         }
     }
-    if (blockIdx.x == 0)
+    if (blockIdx.x == 0) {
         for (int c = threadIdx.x; c < kMaxColors; c += blockDim.x) sb.colorCount[c] = 0;
+        for (uint32_t i = threadIdx.x; i < kIslCounterWords; i += blockDim.x) sb.islCounters[i] = 0;
+    }
     if (!gridBarrier(sb.bar, &a.st->err)) return;
     // each dynamic body's manifolds
     for (uint32_t m = gtid; m < M; m += gstride) {
@@ -136,6 +148,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
                     c = kMaxColors - 1;
                 }
                 *(volatile uint32_t *)&sb.color[m] = c;
+                addToMasks(a, m, sb.dyn[m], c);
                 aggregatedAppendKeyed(sb.colorCount, c);
                 aggregatedMax32(&a.st->colors, c + 1);
                 pendingMask &= ~(1u << k);
@@ -189,6 +202,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
                     c = kMaxColors - 1;
                 }
                 *(volatile uint32_t *)&sb.color[m] = c;
+                addToMasks(a, m, sb.dyn[m], c);
                 aggregatedAppendKeyed(sb.colorCount, c);
                 aggregatedMax32(&a.st->colors, c + 1);
             }
@@ -375,6 +389,36 @@ __global__ void k_cache_counts(SolveArgs a) {
         a.sb.cacheCounts[k] = valid ? min(a.mv.pointCount[m], 4u) : 0u;
     }
 }
+// Cache offsets in manifold order (the cache of one manifold per body pair):
+// exclusive scan of the prepared manifolds' points, one pass with look-back.
+__global__ void __launch_bounds__(kScanThreads)
+k_cache_offsets(SolveArgs a, unsigned long long *state, uint32_t *counter, uint32_t *newCount) {
+    __shared__ uint32_t s_tile, s_scan[9], s_prefix, s_abort;
+    const uint32_t M = min(*a.count, a.mcap);
+    const uint32_t ntiles = max((M + kScanThreads - 1) / kScanThreads, 1u);
+    for (;;) {
+        const uint32_t tile = takeTile(counter, &s_tile);
+        if (tile >= ntiles) return;
+        const uint32_t m = tile * kScanThreads + threadIdx.x;
+        const uint32_t v = m < M ? min(a.sb.pcount[m], 4u) : 0u;
+        uint32_t total;
+        const uint32_t excl = blockExclusiveScan(v, total, s_scan);
+        if (threadIdx.x < 32) {
+            bool timedOut;
+            const uint32_t pre = lookbackExclusiveWarp(state, tile, total, &a.st->err, &timedOut);
+            if (threadIdx.x == 0) {
+                s_prefix = pre;
+                s_abort = timedOut ? 1u : 0u;
+            }
+        }
+        __syncthreads();
+        if (s_abort) return;  // a bounded wait ran out: nothing of this tile is written
+        if (m < M) a.sb.cacheOff[m] = s_prefix + excl;
+        if (threadIdx.x == 0 && tile + 1 == ntiles) *newCount = s_prefix + total;
+        __syncthreads();
+    }
+}
+
 // Writes the cache entries of manifold m (npts points) starting at entry base.
 __global__ void k_cache_write(SolveArgs a, CacheView nc, uint32_t cacheCap) {
     const uint32_t M = min(*a.count, a.mcap);
@@ -454,8 +498,8 @@ int maxCooperativeBlocks(int smCount) {
 
 void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &oldCache, const uint32_t *oldCacheCount,
                   const CacheView &newCache, uint32_t *newCacheCount, uint32_t cacheCap, SolverBuffers &sb,
-                  int iterations, int orderMode, int coopBlocks, bool blockPath, uint32_t blockM, bool pairOrderCache,
-                  DevStats *st, Scratch &ws, cudaStream_t s) {
+                  int iterations, int orderMode, int coopBlocks, bool blockPath, uint32_t blockM, bool sweepAll,
+                  bool pairOrderCache, DevStats *st, Scratch &ws, cudaStream_t s) {
     SolveArgs a{w, mv, sb, oldCache, oldCacheCount, st, sb.mcap, iterations, pairOrderCache,
                 w.sleepMode ? &st->solveCount : &st->manifolds};
     if (w.sleepMode) {
@@ -493,6 +537,19 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
     if (!serial) {
         configureColor();
         launchCooperative((const void *)k_color, coopBlocks, a, s, kColorSmem);
+    }
+    if (sweepAll && !serial && pairOrderCache) {
+        k_prepare<<<gridFor(mcap, kPrepareThreads), kPrepareThreads, kPrepareKeyCap * sizeof(unsigned long long), s>>>(
+            a, kPrepareKeyCap);
+        PE_LAUNCHED();
+        const uint32_t tiles = mcap / kScanThreads + 1;
+        PE_CHECK(cudaMemsetAsync(ws.scanState, 0, sizeof(unsigned long long) * (tiles + 1), s));
+        const uint32_t grid = std::min<uint32_t>(tiles, 2u * (uint32_t)smCount());
+        k_cache_offsets<<<grid, kScanThreads, 0, s>>>(a, ws.scanState, (uint32_t *)(ws.scanState + tiles),
+                                                      newCacheCount);
+        PE_LAUNCHED();
+        launchSolveSweep(a, newCache, cacheCap, s);
+        return;
     }
     // the solve order itself is needed by the serial sweep and by a cache
     // rebuilt in solve order; the island sweeps order each island themselves

@@ -201,7 +201,10 @@ __global__ void k_isl_fill(SolveArgs a) {
         if (cnt[r] >= kIslBlock) tiny[a.mcap - 1 - aggregatedAppend(&a.sb.islCounters[8])] = r;
         else if (cnt[r] >= 32) queue[aggregatedAppend(&a.sb.islCounters[4])] = r;
         else if (cnt[r] >= kIslThread) queue[nIsl - 1 - aggregatedAppend(&a.sb.islCounters[5])] = r;
-        else tiny[aggregatedAppend(&a.sb.islCounters[6])] = r;
+        else {
+            tiny[aggregatedAppend(&a.sb.islCounters[6])] = r;
+            aggregatedAdd32(&a.st->loose, cnt[r]);
+        }
     }
 }
 
@@ -612,17 +615,37 @@ __device__ __forceinline__ bool sweepVisit(const SolveArgs &a, SweepLane &f, uin
     return true;
 }
 
-__global__ void __launch_bounds__(kSolveThreads, 2) k_isl_sweep(SolveArgs a) {
+// The solved point's impulse and its warm-start cache entry (cache in manifold
+// order: offsets from k_cache_offsets).
+__device__ __forceinline__ void writePoint(const SolveArgs &a, const CacheView &nc, uint32_t cacheCap, uint32_t m,
+                                           uint32_t p, float4 imp) {
+    imp.w = 0.0f;
+    a.mv.impulse[4 * m + p] = imp;
+    const uint32_t e = a.sb.cacheOff[m] + p;
+    if (e >= cacheCap) return;
+    const float4 aa = a.mv.anchorA[4 * m + p], ab = a.mv.anchorB[4 * m + p];
+    nc.key[e] = ((unsigned long long)a.mv.bodyA[m] << 32) | a.mv.bodyB[m];
+    nc.gens[e] = ((unsigned long long)a.mv.genA[m] << 32) | a.mv.genB[m];
+    nc.anchorA[e] = make_float4(aa.x, aa.y, aa.z, imp.x);
+    nc.anchorB[e] = make_float4(ab.x, ab.y, ab.z, imp.y);
+    nc.tangent2[e] = imp.z;
+}
+
+// ALL: every manifold of the step (colour counts and body masks from k_color,
+// results written here); otherwise those that k_isl_fill left to the sweeps.
+template <bool ALL>
+__global__ void __launch_bounds__(kSolveThreads, 2) k_isl_sweep(SolveArgs a, CacheView nc, uint32_t cacheCap) {
     __shared__ uint32_t s_start[kMaxColors + 1];  // first item of each colour
     const uint32_t M = min(*a.count, a.mcap);
     {
         const uint32_t wideC = islWideColors(a, M);
         if (wideC) {  // every block sees the same colour count
-            islSolveWide(a, M, wideC);
+            if (!ALL) islSolveWide(a, M, wideC);
+            else if (threadIdx.x == 0) atomicOr(&a.st->err, kErrSmallPath);  // re-run on the island path
             return;
         }
     }
-    const uint32_t *count = a.sb.islCounters + kIslColorCount;
+    const uint32_t *count = ALL ? a.sb.colorCount : a.sb.islCounters + kIslColorCount;
     uint32_t *fill = a.sb.islCounters + kIslColorFill;
     if (threadIdx.x == 0) {
         uint32_t acc = 0;
@@ -637,13 +660,16 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_isl_sweep(SolveArgs a) {
     if (items == 0) return;
     // the manifolds colour by colour, each colour from a whole item
     const uint32_t *cnt = islCnt(a);
-    const uint32_t sweepFrom = islSweepFrom(a, M);
+    const uint32_t sweepFrom = ALL ? 0u : islSweepFrom(a, M);
     uint32_t *list = reinterpret_cast<uint32_t *>(a.sb.islKeysTmp);
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
     for (uint32_t m = gtid; m < M; m += gstride) {
-        const uint32_t r = a.sb.islRoot[m];
         const uint32_t c = a.sb.color[m];
-        if (r == kIslNone || cnt[r] < sweepFrom || c >= (uint32_t)kMaxColors) continue;
+        if (c >= (uint32_t)kMaxColors) continue;
+        if (!ALL) {
+            const uint32_t r = a.sb.islRoot[m];
+            if (r == kIslNone || cnt[r] < sweepFrom) continue;
+        }
         list[kItemManifolds * s_start[c] + aggregatedAppendKeyed(fill, c)] =
             m | min(a.sb.pcount[m], 4u) << kEntryShift;
     }
@@ -654,36 +680,67 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_isl_sweep(SolveArgs a) {
     const uint32_t lane = threadIdx.x & 31, p = lane & 3, passes = (uint32_t)a.iterations + 1u;
     // items go round the blocks, so that a colour's are spread over every SM
     const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
-    auto keepImpulse = [&](const SweepLane &f) {
-        if (p < f.npts) a.sb.pimp[(size_t)p * a.mcap + f.m] = f.imp;
+    auto keepImpulse = [&](const SweepLane &f, bool end) {
+        if (p >= f.npts) return;
+        if (ALL && end) writePoint(a, nc, cacheCap, f.m, p, f.imp);
+        else a.sb.pimp[(size_t)p * a.mcap + f.m] = f.imp;
+    };
+    // manifolds at bodies with few others (the host's choice of the next step's path)
+    auto countLoose = [&](const SweepLane &f) {
+        uint32_t g = __ballot_sync(kWarp, f.act && f.degree <= 2);
+        g &= g >> 1;
+        g &= g >> 2;
+        if (lane == 0 && (g & 0x11111111u)) atomicAdd(&a.st->loose, (uint32_t)__popc(g & 0x11111111u));
     };
     if (items <= warps) {
         if (warp >= items) return;
         SweepLane f;
         loadSweepLane(a, __ldcg(&list[kItemManifolds * warp + (lane >> 2)]), p, f);
+        if (ALL) countLoose(f);
         for (uint32_t pass = 0; pass < passes; ++pass)
             if (!sweepVisit(a, f, pass, passes)) return;
-        keepImpulse(f);
+        keepImpulse(f, true);
         return;
     }
     for (uint32_t pass = 0; pass < passes; ++pass)
         for (uint32_t item = warp; item < items; item += warps) {
             SweepLane f;
             loadSweepLane(a, __ldcg(&list[kItemManifolds * item + (lane >> 2)]), p, f);
+            if (ALL && pass == 0) countLoose(f);
             if (!sweepVisit(a, f, pass, passes)) return;
-            keepImpulse(f);
+            keepImpulse(f, pass + 1 == passes);
         }
 }
 
-// Blocks of k_isl_sweep that the device holds at once.
-static int sweepBlocks() {
+// A cooperative launch of k_isl_sweep on every block that the device holds.
+template <bool ALL> static void launchSweep(const SolveArgs &a, const CacheView &nc, uint32_t cacheCap, cudaStream_t s) {
+    // list entries carry the manifold index in kEntryShift bits
+    if (a.mcap > kEntryMask) throw std::length_error("manifold capacity beyond the grid-wide sweeps' index range");
+    const void *kernel = (const void *)k_isl_sweep<ALL>;
     static int perSm = -1;
     if (perSm < 0) {
         int b = 0;
-        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_isl_sweep, kSolveThreads, 0));
+        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kSolveThreads, 0));
         perSm = b < 1 ? 1 : b;
     }
-    return perSm * smCount();
+    SolveArgs args = a;
+    CacheView cache = nc;
+    void *params[] = {&args, &cache, &cacheCap};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(perSm * smCount());
+    cfg.blockDim = dim3(kSolveThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PE_CHECK(cudaLaunchKernelExC(&cfg, kernel, params));
+    PE_LAUNCHED();
+}
+
+void launchSolveSweep(const SolveArgs &a, const CacheView &newCache, uint32_t cacheCap, cudaStream_t s) {
+    launchSweep<true>(a, newCache, cacheCap, s);
 }
 
 void launchSolveIslands(const SolveArgs &a, Scratch &ws, cudaStream_t s) {
@@ -701,21 +758,7 @@ void launchSolveIslands(const SolveArgs &a, Scratch &ws, cudaStream_t s) {
     PE_LAUNCHED();
     k_isl_solve<<<4 * smCount(), kIslThreads, 0, s>>>(a);
     PE_LAUNCHED();
-    // list entries carry the manifold index in kEntryShift bits
-    if (mcap > kEntryMask) throw std::length_error("manifold capacity beyond the grid-wide sweeps' index range");
-    SolveArgs args = a;
-    void *params[] = {&args};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sweepBlocks());
-    cfg.blockDim = dim3(kSolveThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    PE_CHECK(cudaLaunchKernelExC(&cfg, (const void *)k_isl_sweep, params));
-    PE_LAUNCHED();
+    launchSweep<false>(a, CacheView{}, 0u, s);
 }
 
 void setSpinLimitIslands(uint32_t limit) { setSpinLimitOfUnit(limit); }

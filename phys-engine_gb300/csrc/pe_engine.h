@@ -128,6 +128,9 @@ struct DevStats {
     uint32_t awakeInStep;    // sleeping on: live dynamic bodies awake after the contact wake pass
     uint32_t solveCount;     // sleeping on: manifolds handed to the solver (0 when no body is awake)
     uint32_t islandRefused;  // one-cluster solver: the island path cannot take this step
+    uint32_t loose;          // solved manifolds that share bodies with few others: in islands of fewer than
+                             // kIslThread manifolds (island sweeps), at bodies of two at most (whole-grid sweeps)
+    uint32_t pad;
     int32_t cellLo[3];
     int32_t cellHi[3];
     // Phase boundaries of the one-cluster solver (global timer, ns; zero when

@@ -176,6 +176,10 @@ struct SolveArgs;
 // launch).
 constexpr uint32_t kIslCounterWords = 10 + 2 * kMaxColors;
 void launchSolveIslands(const SolveArgs &a, Scratch &ws, cudaStream_t s);
+// The sweeps over the whole grid alone, for every manifold (after k_color,
+// prepare and the cache offsets), with the impulses and the warm-start cache
+// written by the sweeps.
+void launchSolveSweep(const SolveArgs &a, const CacheView &newCache, uint32_t cacheCap, cudaStream_t s);
 void launchSleepWake(const WorldView &w, const ManifoldView &mv, uint32_t Mhost, uint32_t mcap, uint32_t *flags,
                      float *quiet, uint32_t *err, cudaStream_t s);
 void launchSleepContacts(const WorldView &w, const ManifoldView &mv, DevStats *st, uint32_t mcap, uint32_t *bflags,
@@ -222,8 +226,8 @@ void launchNarrowphase(const WorldView &w, const PairBuffers &pb, const Manifold
                        Scratch &ws, cudaStream_t s, unsigned long long *state = nullptr, bool stateCleared = false);
 void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &oldCache, const uint32_t *oldCacheCount,
                   const CacheView &newCache, uint32_t *newCacheCount, uint32_t cacheCap, SolverBuffers &sb,
-                  int iterations, int orderMode, int coopBlocks, bool blockPath, uint32_t blockM, bool pairOrderCache,
-                  DevStats *st, Scratch &ws, cudaStream_t s);
+                  int iterations, int orderMode, int coopBlocks, bool blockPath, uint32_t blockM, bool sweepAll,
+                  bool pairOrderCache, DevStats *st, Scratch &ws, cudaStream_t s);
 // Largest manifold count the single-block solver handles, and the largest
 // body index it can key (bodies < 2^20).
 constexpr uint32_t kBlockMaxManifolds = 4096;

@@ -238,6 +238,8 @@ std::unique_ptr<World> World::clone() {
     c->bodyPairs_ = bodyPairs_;
     c->lastMEstimate_ = lastMEstimate_;
     c->lastRawEstimate_ = lastRawEstimate_;
+    c->sweepAll_ = sweepAll_;
+    c->sweepAge_ = sweepAge_;
     c->lastPairs_ = lastPairs_;
     c->lastManifolds_ = lastManifolds_;
     c->counters_ = counters_;
@@ -810,7 +812,7 @@ void World::runPipeline(float dt) {
     const CacheView tmp{tKey_.ptr, tGens_.ptr, tA_.ptr, tB_.ptr, tT2_.ptr};
     launchSolver(w, mv, cacheView(cache_), &cCount_.ptr[cache_], sleeping ? tmp : cacheView(1 - cache_),
                  sleeping ? tCount_.ptr : &cCount_.ptr[1 - cache_], cacheCap_, sb_, iterations, orderMode, coopBlocks_,
-                 blockSolver_, blockM_, identityColliders_, st, ws_, s);
+                 blockSolver_, blockM_, sweepAll_, identityColliders_, st, ws_, s);
     if (sleeping)
         launchCacheCarry(w, cacheView(cache_), &cCount_.ptr[cache_], tmp, tCount_.ptr, cacheView(1 - cache_),
                          &cCount_.ptr[1 - cache_], cacheCap_, carry_.ptr, carryPos_.ptr, carryTotal_.ptr, st, ws_, s);
@@ -928,6 +930,7 @@ bool World::finishStep() {
     lastMEstimate_ = h.manifolds;
     lastRawEstimate_ = h.rawPairs;
     wideColors_ = orderMode != 0 && !solveSkipped_ && h.colors > (uint32_t)kMaxColors;
+    chooseSweeps(h);
     // Cell-key width: whole bytes with at least two bits of slack, widened
     // early so the captured graph rarely changes.
     if (algorithm == 1) {
@@ -941,11 +944,48 @@ bool World::finishStep() {
     return true;
 }
 
+// The next step's solver path, from what this step's solver found.  All paths
+// give the same bits; changed at most once in kSweepAge steps, since a change
+// captures the step's graphs again.
+//  * The one-cluster solver sweeps islands of up to 16 manifolds alone and is
+//    the best path for them; a pile (it refused its islands) goes colour by
+//    colour there, 2 to 5 us a phase, against a fixed cost about 60 us higher in
+//    the whole-grid sweeps and 1 to 2.5 us a phase.  Measured, us a step: piles
+//    of 10, 36 and 210 boxes in pyramids 238 -> 195, 300 -> 230, 640 -> 508;
+//    fields of 60, 400, 1,501 and 2,000 bodies 182 -> 156, 240 -> 203, 384 ->
+//    274, 926 -> 295.  Spheres on a floor (one point a manifold, three to five
+//    colours) stay: 1,309 manifolds 225 -> 223, fewer lose.
+//  * Above the cluster's size the island sweeps pay where most manifolds lie in
+//    islands of fewer than eight (65,536 boxes in stacks of two: 430 against 500
+//    in the whole-grid sweeps), the whole-grid sweeps elsewhere (fields of 5,000
+//    and 50,000 bodies, islands found and swept as piles: 395 -> 338, 700 -> 630).
+void World::chooseSweeps(const DevStats &h) {
+    constexpr uint32_t kSweepAge = 64, kSweepMin = 8;
+    if (sweepAge_ < kSweepAge) {
+        ++sweepAge_;
+        return;
+    }
+    if (orderMode == 0 || solveSkipped_ || !identityColliders_) return;
+    bool want = sweepAll_;
+    if (sweepAll_) {
+        want = h.manifolds >= kSweepMin && 4ull * h.loose <= 3ull * h.manifolds;
+    } else if (!wideColors_ && h.manifolds >= 2 * kSweepMin) {
+        if (blockSolver_) {
+            const uint64_t phases = (uint64_t)h.colors * (uint32_t)(iterations + 1);
+            want = h.islandRefused != 0 && phases * (4ull * h.points > 5ull * h.manifolds ? 3 : 1) > 100;
+        } else {
+            want = 4ull * h.loose < h.manifolds;
+        }
+    }
+    if (want != sweepAll_) sweepAge_ = 0;
+    sweepAll_ = want;
+}
+
 bool World::GraphKey::operator==(const GraphKey &o) const {
     return nb == o.nb && nc == o.nc && pairCap == o.pairCap && entryCap == o.entryCap && mcap == o.mcap &&
            cacheCap == o.cacheCap && dt == o.dt && gx == o.gx && gy == o.gy && gz == o.gz &&
            algorithm == o.algorithm && iterations == o.iterations && orderMode == o.orderMode &&
-           coopBlocks == o.coopBlocks && blockSolver == o.blockSolver && blockM == o.blockM && pairBits == o.pairBits &&
+           coopBlocks == o.coopBlocks && blockSolver == o.blockSolver && sweepAll == o.sweepAll && blockM == o.blockM && pairBits == o.pairBits &&
            blockPairs == o.blockPairs && bodyPairs == o.bodyPairs && hashed == o.hashed && gridKeyBits == o.gridKeyBits && cellSize == o.cellSize && dense == o.dense &&
            localIdentity == o.localIdentity && forces == o.forces && identityColliders == o.identityColliders &&
            sleeping == o.sleeping && rawForces == o.rawForces && packPoses == o.packPoses && ioMode == o.ioMode &&
@@ -969,6 +1009,7 @@ World::GraphKey World::currentKey(float dt) const {
     k.orderMode = orderMode;
     k.coopBlocks = coopBlocks_;
     k.blockSolver = blockSolver_;
+    k.sweepAll = sweepAll_;
     k.blockM = blockM_;
     k.pairBits = pb_.bits;
     k.blockPairs = pb_.blockPath;
@@ -1003,8 +1044,9 @@ unsigned long long World::launchStep(float dt) {
     coopBlocks_ = maxCooperativeBlocks(smCount_);
     // Small manifold counts run the single-block solver (with headroom over
     // the last step's count; an overflow re-runs the step on the full path).
+    if (wideColors_ || orderMode == 0 || !identityColliders_) sweepAll_ = false;
     blockSolver_ = lastMEstimate_ + lastMEstimate_ / 4 + 64 <= kBlockMaxManifolds && nb_ <= kBlockMaxBodies &&
-                   !wideColors_;
+                   !wideColors_ && !sweepAll_;
     blockM_ = 64;
     while (blockM_ < lastMEstimate_ + lastMEstimate_ / 4 + 64 && blockM_ < kBlockMaxManifolds) blockM_ <<= 1;
     // Pair keys need bits for input indices < nc; the small finalize path is
@@ -1496,7 +1538,7 @@ void World::solveOnly(std::vector<float> &recs, uint32_t count, float dt, int it
     }
     launchSolver(w, mv, cacheView(cache_), &cCount_.ptr[cache_], sleeping ? tmp : cacheView(1 - cache_),
                  sleeping ? tCount_.ptr : &cCount_.ptr[1 - cache_], cacheCap_, sb_, iters, mode, (int)blocks, block, 0u,
-                 false, st, ws_, s);
+                 false, false, st, ws_, s);
     if (sleeping)
         launchCacheCarry(w, cacheView(cache_), &cCount_.ptr[cache_], tmp, tCount_.ptr, cacheView(1 - cache_),
                          &cCount_.ptr[1 - cache_], cacheCap_, carry_.ptr, carryPos_.ptr, carryTotal_.ptr, st, ws_, s);

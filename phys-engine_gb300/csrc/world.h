@@ -216,6 +216,11 @@ class World {
     // the last step needed more than kMaxColors solver colours: solve on the
     // multi-kernel path (the cluster solver's colour ranges hold kMaxColors)
     bool wideColors_ = false;
+    // solve with the sweeps over the whole grid alone: the last steps' contacts
+    // form piles; steps since this was last changed
+    bool sweepAll_ = false;
+    uint32_t sweepAge_ = 0;
+    void chooseSweeps(const DevStats &h);
     uint32_t gridKeyBits_ = 64;
     uint64_t possiblePairs_ = 0, dynamicAlive_ = 0;
     StepCounters counters_;
@@ -309,7 +314,7 @@ class World {
         uint32_t nb, nc, pairCap, entryCap, mcap, cacheCap;
         float dt, gx, gy, gz;
         int algorithm, iterations, orderMode, coopBlocks;
-        bool blockSolver, blockPairs, bodyPairs, hashed;
+        bool blockSolver, sweepAll, blockPairs, bodyPairs, hashed;
         uint32_t blockM;
         uint32_t pairBits, gridKeyBits;
         double cellSize;

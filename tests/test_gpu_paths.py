@@ -154,3 +154,53 @@ def test_rollout_of_a_pile(gpu):
     d = [torch.tensor(rng.normal(size=tuple(o.shape)).astype(np.float32), device="cuda:0") for o in outs]
     for g in roll.backward(*d):
         assert bool(torch.isfinite(g).all())
+
+
+@pytest.mark.parametrize("n, steps, sleeping", [(60, 140, False), (700, 100, False), (700, 160, True),
+                                                (3000, 90, False), (16000, 80, False)])
+def test_whole_grid_sweeps_match_the_oracle(gpu, n, steps, sleeping):
+    """Piles long enough for the step to change to the whole-grid sweeps (64
+    steps): few manifolds, one item of eight a warp, more items than warps, and
+    with sleeping on; poses, velocities, pairs and manifolds with their impulses
+    against the oracle, bit for bit, before and after the change."""
+    from oracle import cpu
+    from test_gpu_parity import compare_worlds
+
+    sc = scenes.mixed_field(n, 5)
+    g = gpu.GpuWorld(algo=0, iterations=8)
+    o = cpu.OracleWorld(algo=0, iterations=8, order_mode=1)
+    for w in (g, o):
+        w.set_sleeping_enabled(sleeping)
+        w.load_scene(sc)
+    for s in range(1, steps + 1):
+        g.step(1 / 120)
+        o.step(1 / 120)
+        if s in (60, 66, 70) or s % 20 == 0:
+            compare_worlds(g, o, f"step {s}")
+    for f in ("solved_contact_count", "prepared_points", "warm_start_matches", "color_count"):
+        assert g.stats()[f] == o.stats()[f], f
+
+
+def test_whole_grid_sweeps_survive_changes_of_path(gpu):
+    """A pile is lifted apart (bodies removed until none touches another) and the
+    copy of the world goes on: the paths change and the oracle agrees."""
+    from oracle import cpu
+    from test_gpu_parity import compare_worlds
+
+    sc = scenes.mixed_field(200, 6)
+    g = gpu.GpuWorld(algo=0, iterations=8)
+    o = cpu.OracleWorld(algo=0, iterations=8, order_mode=1)
+    hg, ho = g.load_scene(sc), o.load_scene(sc)
+    for phase in range(3):
+        for _ in range(70):
+            g.step(1 / 120)
+            o.step(1 / 120)
+        compare_worlds(g, o, f"phase {phase}")
+        c = g.clone()
+        c.step(1 / 120)
+        for i in range(1 + phase, 200, 3):
+            g.remove_body(*hg[i, :2])
+            o.remove_body(*ho[i, :2])
+        g.step(1 / 120)
+        o.step(1 / 120)
+        compare_worlds(g, o, f"phase {phase} after the removal")
