@@ -192,6 +192,8 @@ k_radix_pass(K *buf0, K *buf1, uint32_t *vbuf0, uint32_t *vbuf1, const uint32_t 
         if (threadIdx.x == 0) s_abort = 0;
         __syncthreads();
 
+        // all of a thread's keys requested at once (the ranking below orders its
+        // memory accesses with __syncwarp, which would hold each load back)
         K key[kSortRounds];
         uint32_t val[kSortRounds], dig[kSortRounds], rank[kSortRounds];
 #pragma unroll
@@ -201,6 +203,9 @@ k_radix_pass(K *buf0, K *buf1, uint32_t *vbuf0, uint32_t *vbuf1, const uint32_t 
             key[r] = valid ? kin[idx] : (K)0;
             if (VALS) val[r] = valid ? vin[idx] : 0u;
             dig[r] = valid ? (uint32_t)((key[r] >> shift) & 0xFF) : 0xFFu;
+        }
+#pragma unroll
+        for (int r = 0; r < kSortRounds; ++r) {
             const uint32_t peers = __match_any_sync(0xffffffffu, dig[r]);
             const uint32_t lower = __popc(peers & lanemask_lt);
             const uint32_t old = s_warp[warp][dig[r]];
