@@ -92,13 +92,23 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
     if (!gridBarrier(sb.bar, &a.st->err)) return;
     if (__ldcg(&sb.counters[1]) == 0u && (M + gstride - 1) / gstride <= kColorCached) {
         // Each thread reads its manifolds' neighbour lists once and keeps the
-        // higher-priority neighbours in shared memory; every pass then asks
-        // for all of a manifold's neighbour colours in one round trip.
+        // higher-priority neighbours in shared memory.  A pass asks for the
+        // colours of those a manifold still waits for, in one round trip, and
+        // drops the ones it gets; the colours go to the bodies' masks and to
+        // per-block counts without a wait.
+        __shared__ uint32_t s_count[kMaxColors];
         const uint32_t T = blockDim.x, R = (M + gstride - 1) / gstride;
+        for (uint32_t c = threadIdx.x; c < (uint32_t)kMaxColors; c += T) s_count[c] = 0;
+        __syncthreads();
+        uint32_t waiting[kColorCached];             // neighbours without a colour yet
+        unsigned long long taken[kColorCached][2];  // colours of the others
         uint32_t pendingMask = 0;
-        for (uint32_t k = 0; k < R; ++k) {
+#pragma unroll
+        for (uint32_t k = 0; k < kColorCached; ++k) {
+            waiting[k] = 0;
+            taken[k][0] = taken[k][1] = 0ull;
             const uint32_t m = gtid + k * gstride;
-            if (m >= M) continue;
+            if (k >= R || m >= M) continue;
             pendingMask |= 1u << k;
             uint32_t *row = s_hp + (size_t)k * kColorSlots * T + threadIdx.x;
             const uint32_t p = colorPriority(m), d = sb.dyn[m];
@@ -113,33 +123,38 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
                 const uint32_t e = i / kIslandMax, j = i % kIslandMax;
                 o[i] = j < n[e] ? __ldcg(&inc[(size_t)bs[e] * kIslandMax + j]) : kNoNeighbour;
             }
+            uint32_t w = 0;
 #pragma unroll
             for (uint32_t i = 0; i < kColorSlots; ++i)
-                row[(size_t)i * T] = (o[i] != kNoNeighbour && o[i] != m && colorPriority(o[i]) > p) ? o[i]
-                                                                                                  : kNoNeighbour;
+                if (o[i] != kNoNeighbour && o[i] != m && colorPriority(o[i]) > p) row[(size_t)(w++) * T] = o[i];
+            waiting[k] = w;
         }
-        uint32_t pass = 0;
+        uint32_t pass = 0, top = 0;
         for (; pendingMask && pass < spinLimit(); ++pass) {
-            for (uint32_t k = 0; k < R; ++k) {
+#pragma unroll
+            for (uint32_t k = 0; k < kColorCached; ++k) {
                 if (!(pendingMask >> k & 1u)) continue;
                 const uint32_t m = gtid + k * gstride;
-                const uint32_t *row = s_hp + (size_t)k * kColorSlots * T + threadIdx.x;
-                uint32_t cs[kColorSlots];
+                uint32_t *row = s_hp + (size_t)k * kColorSlots * T + threadIdx.x;
+                uint32_t left = 0;
+                for (uint32_t i0 = 0; i0 < waiting[k]; i0 += 8) {
+                    uint32_t o[8], cs[8];
 #pragma unroll
-                for (uint32_t i = 0; i < kColorSlots; ++i) {
-                    const uint32_t o = row[(size_t)i * T];
-                    cs[i] = o != kNoNeighbour ? ldvol(&sb.color[o]) : 0xFFFFFFFEu;
-                }
-                unsigned long long u0 = 0, u1 = 0;
-                bool ready = true;
+                    for (uint32_t i = 0; i < 8; ++i) {
+                        o[i] = i0 + i < waiting[k] ? row[(size_t)(i0 + i) * T] : kNoNeighbour;
+                        if (o[i] != kNoNeighbour) cs[i] = ldvol(&sb.color[o[i]]);
+                    }
 #pragma unroll
-                for (uint32_t i = 0; i < kColorSlots; ++i) {
-                    if (cs[i] == 0xFFFFFFFEu) continue;
-                    if (cs[i] == kUncolored) ready = false;
-                    else if (cs[i] < 64) u0 |= 1ull << cs[i];
-                    else u1 |= 1ull << (cs[i] - 64);
+                    for (uint32_t i = 0; i < 8; ++i) {
+                        if (o[i] == kNoNeighbour) continue;
+                        if (cs[i] == kUncolored) row[(size_t)(left++) * T] = o[i];
+                        else if (cs[i] < 64) taken[k][0] |= 1ull << cs[i];
+                        else taken[k][1] |= 1ull << (cs[i] - 64);
+                    }
                 }
-                if (!ready) continue;
+                waiting[k] = left;
+                if (left) continue;
+                const unsigned long long u0 = taken[k][0], u1 = taken[k][1];
                 uint32_t c;
                 if (~u0) c = __ffsll((long long)~u0) - 1;
                 else if (~u1) c = 64 + __ffsll((long long)~u1) - 1;
@@ -149,13 +164,17 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
                 }
                 *(volatile uint32_t *)&sb.color[m] = c;
                 addToMasks(a, m, sb.dyn[m], c);
-                aggregatedAppendKeyed(sb.colorCount, c);
-                aggregatedMax32(&a.st->colors, c + 1);
+                atomicAdd(&s_count[c], 1u);
+                top = max(top, c + 1);
                 pendingMask &= ~(1u << k);
             }
         }
         if (pendingMask) atomicOr(&a.st->err, kErrTimeout);
+        aggregatedMax32(&a.st->colors, top);
         aggregatedMax32(&a.st->colorRounds, pass);
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < (uint32_t)kMaxColors; c += T)
+            if (s_count[c]) atomicAdd(&sb.colorCount[c], s_count[c]);
         return;
     }
     if (__ldcg(&sb.counters[1]) == 0u) {
@@ -326,14 +345,17 @@ __global__ void k_order_init(SolveArgs a, int serial) {
 
 // Prepare of every manifold, by manifold index, before the colouring, and the
 // manifold flags (sb.dyn) the single-block front reads.  The old cache's keys
-// are copied to shared memory when at most keyCap of them.
+// are copied to shared memory when at most keyCap of them: every block copies,
+// so a few thousand keys cost more than the dozen loads of a search in L2
+// (3,811 keys, 2,600 manifolds: 35 us with the copy, 13 without).
 constexpr int kPrepareThreads = 64;
-constexpr uint32_t kPrepareKeyCap = 4096;
+constexpr uint32_t kPrepareKeyCap = 512;
 __global__ void __launch_bounds__(kPrepareThreads) k_prepare(SolveArgs a, uint32_t keyCap) {
     extern __shared__ unsigned long long s_keys[];
     const uint32_t M = min(*a.count, a.mcap);
     for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x)
         a.sb.dyn[m] = manifoldFlags(a, m);
+    if (blockIdx.x * blockDim.x >= 4 * M) return;  // no item of this block
     const uint32_t cacheN = *a.oldCount;
     const bool inShared = cacheN <= keyCap;
     if (inShared)
