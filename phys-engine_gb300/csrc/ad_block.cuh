@@ -24,6 +24,7 @@
 // geometry).
 #pragma once
 #include "ad_world.cuh"
+#include "pe_block.cuh"
 
 namespace pe {
 namespace ad {
@@ -88,63 +89,6 @@ __device__ __forceinline__ uint32_t blockScan(uint32_t v, uint32_t &total, uint3
 }
 
 using Key = unsigned long long;
-
-// Compare-exchange stages j = 32 .. 1 of bitonic size kk over the 64 keys
-// v0 (position base + lane) and v1 (base + 32 + lane) of one warp.
-__device__ __forceinline__ void sortStages(Key &v0, Key &v1, uint32_t base, uint32_t kk) {
-    const uint32_t lane = threadIdx.x & 31;
-    const bool up0 = ((base + lane) & kk) == 0, up1 = ((base + 32 + lane) & kk) == 0;
-    if (kk >= 64 && (v0 > v1) == up0) {
-        const Key t = v0;
-        v0 = v1;
-        v1 = t;
-    }
-#pragma unroll
-    for (uint32_t j = 16; j > 0; j >>= 1) {
-        if (j >= kk) continue;
-        const Key p0 = __shfl_xor_sync(0xffffffffu, v0, j), p1 = __shfl_xor_sync(0xffffffffu, v1, j);
-        const bool low = (lane & j) == 0;
-        v0 = (low == up0) == (p0 < v0) ? p0 : v0;
-        v1 = (low == up1) == (p1 < v1) ? p1 : v1;
-    }
-}
-
-// Ascending sort of k[0, n), n a power of two, by the whole block (shared or
-// global memory).  A barrier on either side.
-__device__ __noinline__ void blockSort(Key *k, uint32_t n) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const uint32_t chunks = (n + 63) / 64;
-    __syncthreads();
-    for (uint32_t c = warp; c < chunks; c += nw) {
-        const uint32_t i0 = 64 * c + lane, i1 = i0 + 32;
-        Key v0 = i0 < n ? k[i0] : ~0ull, v1 = i1 < n ? k[i1] : ~0ull;
-#pragma unroll
-        for (uint32_t kk = 2; kk <= 64; kk <<= 1) sortStages(v0, v1, 64 * c, kk);
-        if (i0 < n) k[i0] = v0;
-        if (i1 < n) k[i1] = v1;
-    }
-    __syncthreads();
-    for (uint32_t kk = 128; kk <= n; kk <<= 1) {
-        for (uint32_t j = kk >> 1; j >= 64; j >>= 1) {
-            for (uint32_t t = threadIdx.x; t < n / 2; t += blockDim.x) {
-                const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), x = i | j;
-                const Key a = k[i], b = k[x];
-                if ((a > b) == ((i & kk) == 0)) {
-                    k[i] = b;
-                    k[x] = a;
-                }
-            }
-            __syncthreads();
-        }
-        for (uint32_t c = warp; c < chunks; c += nw) {
-            Key v0 = k[64 * c + lane], v1 = k[64 * c + 32 + lane];
-            sortStages(v0, v1, 64 * c, kk);
-            k[64 * c + lane] = v0;
-            k[64 * c + 32 + lane] = v1;
-        }
-        __syncthreads();
-    }
-}
 
 // ------------------------------------------------------ manifold lane groups --
 // Four lanes of a warp work on one manifold; lane p holds point p.  The whole
@@ -396,7 +340,7 @@ __device__ __noinline__ void contactsBlock(BlockWorld &bw) {
         sh.pairs = 0;
         sc.counts[3] = 0;
     }
-    blockSort(entries, n2);
+    blockChunkSort(entries, n2);
 
     // 2. sweep: a warp for each body, its lanes along the window (bodies sorted
     // by min.x up to the first whose min.x exceeds this body's max.x)
@@ -440,7 +384,7 @@ __device__ __noinline__ void contactsBlock(BlockWorld &bw) {
     } else {
         for (uint32_t p = P + tid; p < P2; p += nt) pairs[p] = ~0ull;
     }
-    blockSort(pairs, P2);
+    blockChunkSort(pairs, P2);
 
     // 3. narrowphase in pair order, manifolds compacted in that order
     uint32_t M = 0;
@@ -570,7 +514,7 @@ __device__ __noinline__ void contactsBlock(BlockWorld &bw) {
         Key *keys = M2 <= sortKeys ? shKeys : sc.sortKeys;
         __syncthreads();  // the masks are read no more
         for (uint32_t i = tid; i < M2; i += nt) keys[i] = i < M ? ((Key)sc.color[i] << 32) | i : ~0ull;
-        blockSort(keys, M2);
+        blockChunkSort(keys, M2);
         for (uint32_t k = tid; k < M; k += nt) {
             const uint32_t m = (uint32_t)keys[k], ck = (uint32_t)(keys[k] >> 32);
             sc.order[k] = m;

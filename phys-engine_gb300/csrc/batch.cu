@@ -350,6 +350,8 @@ BatchView Batch::view(const BatchBucket &bk, float dt, uint32_t parity) const {
     v.worldCount = (uint32_t)desc_.size();
     v.maxM = bk.maxM;
     v.maxN = bk.maxN;
+    v.sortCap = 1;
+    while (2 * v.sortCap * sizeof(unsigned long long) <= batchSharedBytes(bk.maxN, bk.maxM)) v.sortCap <<= 1;
     v.iterations = iterations;
     v.parity = parity;
     v.gx = gravity[0];

@@ -47,6 +47,7 @@ struct BatchView {
     uint32_t worldCount;
     uint32_t maxM;          // shared-memory manifold capacity of this launch
     uint32_t maxN;          // largest world of this bucket (shared-memory SAP keys)
+    uint32_t sortCap;       // 64-bit keys that the launch's shared memory holds (power of two)
     int iterations;
     uint32_t parity;        // state[parity] is read, state[parity ^ 1] written
     float gx, gy, gz, dt;

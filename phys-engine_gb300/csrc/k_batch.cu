@@ -122,6 +122,23 @@ struct BatchShared {
     unsigned long long xWindow;
 };
 
+// 5. pose
+__device__ __forceinline__ void integrateWorldPoses(const WorldView &w, uint32_t N) {
+    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {
+        const uint32_t f = w.bflags[i];
+        float4 p4 = w.cur.pos[i], q4 = w.cur.rot[i];
+        if ((f & kBodyAlive) && !(f & kBodyStatic)) {
+            V3 pos = f4xyz(p4);
+            Q rot = f4q(q4);
+            integratePose(pos, rot, f4xyz(ld4(&w.nxt.lin[i])), f4xyz(ld4(&w.nxt.ang[i])), w.dt);
+            p4 = make4(pos, 0.0f);
+            q4 = make4(rot);
+        }
+        w.nxt.pos[i] = p4;
+        w.nxt.rot[i] = q4;
+    }
+}
+
 // One world, all threads of the block.
 __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned long long *smem, BatchShared &sh) {
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
@@ -164,28 +181,41 @@ __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned
 
     // 2. SAP: sort by (min.x, index), sweep with the reference's break and
     // Y/Z test (broadphase.cpp:212-243), then lexicographic pair order.
-    blockBitonicSort(keys, np);
+    blockChunkSort(keys, np);
     unsigned long long *pk = b.pairKeys + d.pairBase;
+    // A warp for each body, its lanes along the body's window: a floor's window
+    // holds every body, and with a thread for each body the block waited for the
+    // thread that walked it.  With the sorts below in warp chunks and the solver
+    // left out where nothing touches, a step of 2,048 worlds of 4 to 1,500 bodies
+    // went from 772 to 745 us and one of 1,024 worlds of 16 to 300 from 980 to 919.
+    const uint32_t lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     unsigned long long window = 0;
-    for (uint32_t i = tid; i < N; i += nt) {
+    for (uint32_t i = warp; i < N; i += nw) {
         const uint32_t ia = (uint32_t)keys[i];
         const float4 amn = w.aabbMin[ia], amx = w.aabbMax[ia];
         const uint32_t xk = orderedFloatKey(amx.x);
-        uint32_t lo = i + 1, hi = N;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if ((uint32_t)(keys[mid] >> 32) > xk) hi = mid;
-            else lo = mid + 1;
-        }
-        window += lo - i - 1;
-        for (uint32_t j = i + 1; j < lo; ++j) {
-            const uint32_t jb = (uint32_t)keys[j];
-            const float4 bmn = w.aabbMin[jb], bmx = w.aabbMax[jb];
-            if (amn.y <= bmx.y && amx.y >= bmn.y && amn.z <= bmx.z && amx.z >= bmn.z) {
-                const uint32_t slot = atomicAdd(&sh.count, 1u);
-                if (slot < d.pairCap)
-                    pk[slot] = ((unsigned long long)min(ia, jb) << 32) | max(ia, jb);
+        for (uint32_t j0 = i + 1; j0 < N; j0 += 32) {
+            const uint32_t j = j0 + lane;
+            uint32_t jb = 0;
+            bool in = false, hit = false;
+            if (j < N) {
+                const unsigned long long key = keys[j];
+                jb = (uint32_t)key;
+                in = (uint32_t)(key >> 32) <= xk;  // sorted: the lanes inside the window come first
             }
+            if (in) {
+                const float4 bmn = w.aabbMin[jb], bmx = w.aabbMax[jb];
+                hit = amn.y <= bmx.y && amx.y >= bmn.y && amn.z <= bmx.z && amx.z >= bmn.z;
+            }
+            const uint32_t inside = __ballot_sync(0xffffffffu, in), hits = __ballot_sync(0xffffffffu, hit);
+            if (lane == 0) window += __popc(inside);
+            if (hits) {
+                uint32_t slot = 0;
+                if (lane == 0) slot = atomicAdd(&sh.count, (uint32_t)__popc(hits));
+                slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(hits & ((1u << lane) - 1u));
+                if (hit && slot < d.pairCap) pk[slot] = ((unsigned long long)min(ia, jb) << 32) | max(ia, jb);
+            }
+            if (inside != 0xffffffffu) break;
         }
     }
     if (window) atomicAdd(&sh.xWindow, window);
@@ -207,9 +237,16 @@ __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned
         return;
     }
     const uint32_t pp = nextPow2(P > 0 ? P : 1);
-    for (uint32_t i = P + tid; i < pp; i += nt) pk[i] = ~0ull;
-    __syncthreads();
-    blockBitonicSort(pk, pp);
+    if (pp <= b.sortCap) {
+        // in shared memory, and back for the pairs' readers
+        for (uint32_t i = tid; i < pp; i += nt) keys[i] = i < P ? pk[i] : ~0ull;
+        blockChunkSort(keys, pp);
+        for (uint32_t i = tid; i < P; i += nt) pk[i] = keys[i];
+        __syncthreads();
+    } else {
+        for (uint32_t i = P + tid; i < pp; i += nt) pk[i] = ~0ull;
+        blockChunkSort(pk, pp);
+    }
 
     // 3. narrowphase in pair order
     const ManifoldView mv = manifoldSlice(b.mv, d.mBase);
@@ -253,6 +290,15 @@ __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned
     __syncthreads();
 
     // 4. contact solve (graph-colour order)
+    uint32_t *newCount = b.cacheCount + (size_t)(b.parity ^ 1u) * b.worldCount + wi;
+    if (running == 0) {
+        if (tid == 0) {
+            *newCount = 0;
+            st->colorRounds = 1;  // as the colouring of no manifold counts them
+        }
+        integrateWorldPoses(w, N);
+        return;
+    }
     SolveArgs a;
     a.w = w;
     a.mv = mv;
@@ -265,24 +311,10 @@ __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned
     a.pairOrderCache = true;  // collider i is body i in every batched world
     a.count = &st->manifolds;
     const CacheView nc = cacheSlice(b.cache[b.parity ^ 1u], d.cacheBase);
-    uint32_t *newCount = b.cacheCount + (size_t)(b.parity ^ 1u) * b.worldCount + wi;
     solveBlock(a, nc, d.cacheCap, newCount, 0, b.maxM, smem, reinterpret_cast<uint32_t *>(smem + b.maxM), sh.solve);
     __syncthreads();
 
-    // 5. pose
-    for (uint32_t i = tid; i < N; i += nt) {
-        const uint32_t f = w.bflags[i];
-        float4 p4 = w.cur.pos[i], q4 = w.cur.rot[i];
-        if ((f & kBodyAlive) && !(f & kBodyStatic)) {
-            V3 pos = f4xyz(p4);
-            Q rot = f4q(q4);
-            integratePose(pos, rot, f4xyz(ld4(&w.nxt.lin[i])), f4xyz(ld4(&w.nxt.ang[i])), w.dt);
-            p4 = make4(pos, 0.0f);
-            q4 = make4(rot);
-        }
-        w.nxt.pos[i] = p4;
-        w.nxt.rot[i] = q4;
-    }
+    integrateWorldPoses(w, N);
     __syncthreads();
     if (tid == 0 && st->err) atomicOr(b.batchErr, st->err);
 }

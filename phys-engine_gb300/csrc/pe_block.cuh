@@ -27,6 +27,65 @@ template <class K> __device__ __forceinline__ void blockBitonicSort(K *s, uint32
     }
 }
 
+// Compare-exchange stages j = 32 .. 1 of bitonic size kk over the 64 keys
+// v0 (position base + lane) and v1 (base + 32 + lane) of one warp.
+template <class K> __device__ __forceinline__ void chunkSortStages(K &v0, K &v1, uint32_t base, uint32_t kk) {
+    const uint32_t lane = threadIdx.x & 31;
+    const bool up0 = ((base + lane) & kk) == 0, up1 = ((base + 32 + lane) & kk) == 0;
+    if (kk >= 64 && (v0 > v1) == up0) {
+        const K t = v0;
+        v0 = v1;
+        v1 = t;
+    }
+#pragma unroll
+    for (uint32_t j = 16; j > 0; j >>= 1) {
+        if (j >= kk) continue;
+        const K p0 = __shfl_xor_sync(0xffffffffu, v0, j), p1 = __shfl_xor_sync(0xffffffffu, v1, j);
+        const bool low = (lane & j) == 0;
+        v0 = (low == up0) == (p0 < v0) ? p0 : v0;
+        v1 = (low == up1) == (p1 < v1) ? p1 : v1;
+    }
+}
+
+// blockBitonicSort with the stages inside 64 keys in a warp's registers: a
+// barrier only where warps exchange keys (14 for 1,024 keys, not 55; none inside
+// 64).  Any memory; a barrier on either side.
+template <class K> __device__ __noinline__ void blockChunkSort(K *k, uint32_t n) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint32_t chunks = (n + 63) / 64;
+    constexpr K kMax = ~(K)0;
+    __syncthreads();
+    for (uint32_t c = warp; c < chunks; c += nw) {
+        const uint32_t i0 = 64 * c + lane, i1 = i0 + 32;
+        K v0 = i0 < n ? k[i0] : kMax, v1 = i1 < n ? k[i1] : kMax;
+#pragma unroll
+        for (uint32_t kk = 2; kk <= 64; kk <<= 1) chunkSortStages(v0, v1, 64 * c, kk);
+        if (i0 < n) k[i0] = v0;
+        if (i1 < n) k[i1] = v1;
+    }
+    __syncthreads();
+    for (uint32_t kk = 128; kk <= n; kk <<= 1) {
+        for (uint32_t j = kk >> 1; j >= 64; j >>= 1) {
+            for (uint32_t t = threadIdx.x; t < n / 2; t += blockDim.x) {
+                const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), x = i | j;
+                const K a = k[i], b = k[x];
+                if ((a > b) == ((i & kk) == 0)) {
+                    k[i] = b;
+                    k[x] = a;
+                }
+            }
+            __syncthreads();
+        }
+        for (uint32_t c = warp; c < chunks; c += nw) {
+            K v0 = k[64 * c + lane], v1 = k[64 * c + 32 + lane];
+            chunkSortStages(v0, v1, 64 * c, kk);
+            k[64 * c + lane] = v0;
+            k[64 * c + 32 + lane] = v1;
+        }
+        __syncthreads();
+    }
+}
+
 // Sorts a[0, n) ascending (n a power of two, tail padded with the maximum key)
 // by merging: each thread sorts its own C = max(1, n / blockDim.x) consecutive
 // keys in registers, then runs of C, 2C, ... are merged pairwise between a and
