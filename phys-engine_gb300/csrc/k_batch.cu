@@ -186,8 +186,8 @@ __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned
     // A warp for each body, its lanes along the body's window: a floor's window
     // holds every body, and with a thread for each body the block waited for the
     // thread that walked it.  With the sorts below in warp chunks and the solver
-    // left out where nothing touches, a step of 2,048 worlds of 4 to 1,500 bodies
-    // went from 772 to 745 us and one of 1,024 worlds of 16 to 300 from 980 to 919.
+    // left out where nothing touches, a step of 2,048 worlds of 16 to 2,048 bodies
+    // went from 772 to 745 us and one of 1,024 worlds of 16 to 512 from 980 to 919.
     const uint32_t lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     unsigned long long window = 0;
     for (uint32_t i = warp; i < N; i += nw) {

@@ -1,5 +1,5 @@
-// Narrowphase: one candidate pair per thread; manifolds are compacted in pair
-// order in the same pass (block scan of hit flags + decoupled look-back), so
+// Narrowphase: eight lanes or one thread per candidate pair; manifolds are compacted
+// in pair order in the same pass (a tile's hit flags + decoupled look-back), so
 // manifold order equals the reference's (src/world/physics_world.cpp:692-736).
 // Per pair this is the world's generateContact lambda
 // (physics_world.cpp:645-691): collider world transforms, shape dispatch with
@@ -12,93 +12,172 @@
 
 namespace pe {
 
-// Small tiles spread the few candidate pairs of a step over many SMs: each
-// pair is a long dependent chain of arithmetic, so latency, not issue rate,
-// bounds a tile.
-constexpr int kNarrowThreads = 64;
-static_assert(kNarrowThreads >= (int)kMinLookbackTile, "look-back scratch is sized for kMinLookbackTile");
+// A pair is a chain of dependent arithmetic (two boxes: some 7,000 cycles on one
+// thread), so what bounds a step is latency until the chip is full: eight lanes a
+// pair (pe_narrow.cuh), and tiles of 32 pairs, whose hit flags one ballot ranks, so
+// that the few pairs of a small step are on many SMs.  The lanes repeat what a
+// pair's axes and vertices share, though, and hold an eighth of the pairs at a time:
+// from kLaneRounds rounds of the grid's tiles on, a thread takes a pair.  Measured,
+// us a step, a thread a pair in tiles of 64 before: 10 boxes 77 -> 68, field of
+// 1,501 bodies 399 -> 380, 100,000 mixed bodies 143 -> 135, 16 pyramids with hulls
+// 599 -> 574; 65,536 boxes in stacks (65,536 pairs, seven rounds) 320, with lanes 336.
+constexpr int kNarrowThreads = 256;
+constexpr int kNarrowBlocks = 2;  // resident blocks an SM
+constexpr uint32_t kNarrowPairs = kNarrowThreads / kPairLanes;
+constexpr uint32_t kLaneRounds = 4;
+static_assert(kNarrowPairs == 32, "one warp ranks a tile's pairs");
+static_assert(kNarrowPairs >= kMinLookbackTile, "look-back scratch is sized for kMinLookbackTile");
 
-__global__ void __launch_bounds__(kNarrowThreads)
-k_narrowphase(WorldView w, const uint32_t *__restrict__ pairA, const uint32_t *__restrict__ pairB,
-              const uint32_t *d_pairs, ManifoldView out, uint32_t mcap, DevStats *st, unsigned long long *state,
-              uint32_t *counter) {
-    __shared__ uint32_t s_tile, s_scan[9], s_prefix, s_abort;
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->stamp[2] = globalNs();
-    const uint32_t P = min(*d_pairs, mcap);
-    const uint32_t ntiles = max((P + kNarrowThreads - 1) / kNarrowThreads, 1u);
-    for (;;) {
-    const uint32_t tile = takeTile(counter, &s_tile);
-    if (tile >= ntiles) return;
-    const uint32_t p = tile * kNarrowThreads + threadIdx.x;
+struct NarrowShared {
+    uint32_t tile, prefix, abort;
+    uint32_t hits[kNarrowPairs], rank[kNarrowPairs], scan[9];
+};
 
+// Counters of a tested pair (the first lane of its lanes).
+__device__ __forceinline__ void countPair(DevStats *st, uint32_t category, bool epaFailed, bool hit, uint32_t points) {
+    if (epaFailed) atomicAdd(&st->epaFailures, 1ull);
+    aggregatedCount(st->npCandidates, category);
+    if (hit) {
+        aggregatedCount(st->npContacts, category);
+        aggregatedAdd32(&st->points, points);
+    }
+}
+
+// One tile, eight lanes a pair.  False when the look-back's wait ran out (then
+// nothing of the tile is written).
+__device__ __forceinline__ bool laneTile(const WorldView &w, const uint32_t *pairA, const uint32_t *pairB, uint32_t P,
+                                         uint32_t ntiles, const ManifoldView &out, uint32_t mcap, DevStats *st,
+                                         unsigned long long *state, NarrowShared &sh) {
+    const uint32_t lane = threadIdx.x & (kPairLanes - 1), pair = threadIdx.x / kPairLanes;
+    const uint32_t p = sh.tile * kNarrowPairs + pair;
+    const bool act = p < P;
+    // (lanes without a pair run the last pair's arithmetic along)
+    const uint32_t ca = pairA[act ? p : P - 1], cb = pairB[act ? p : P - 1];
+    const PairSide a = loadPairSide(w, ca), b = loadPairSide(w, cb);
+    float restitution = 0.0f, friction = 0.0f;
+    LaneManifold lm;
+    bool epaFailed;
+    narrowphaseLanes(w, act, ca, cb, a, b, lm, restitution, friction, epaFailed);
+    if (act && lane == 0) countPair(st, pairCategory(a, b), epaFailed, lm.hit, lm.count);
+    if (lane == 0) sh.hits[pair] = lm.hit ? 1u : 0u;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t hits = __ballot_sync(0xffffffffu, sh.hits[threadIdx.x] != 0);
+        bool timedOut;
+        const uint32_t pre = lookbackExclusiveWarp(state, sh.tile, __popc(hits), &st->err, &timedOut);
+        sh.rank[threadIdx.x] = pre + __popc(hits & ((1u << threadIdx.x) - 1u));
+        if (threadIdx.x == 0) {
+            sh.abort = timedOut ? 1u : 0u;
+            if (sh.tile + 1 == ntiles && !timedOut) {
+                st->manifolds = pre + __popc(hits);
+                st->stamp[3] = globalNs();
+            }
+        }
+    }
+    // contacts go out by their lanes, empty ones by the lane of their index
+    const uint32_t contacts = (__ballot_sync(0xffffffffu, lm.mine) >> (threadIdx.x & 24u)) & 0xFFu;
+    __syncthreads();
+    if (sh.abort) return false;
+    const uint32_t m = sh.rank[pair];
+    if (act && sh.hits[pair] != 0 && m < mcap) {
+        if (lane == 0) {
+            out.bodyA[m] = a.body;
+            out.genA[m] = a.gen;
+            out.bodyB[m] = b.body;
+            out.genB[m] = b.gen;
+            out.normalFriction[m] = make4(lm.normal, friction);
+            out.restitution[m] = restitution;
+            out.pointCount[m] = lm.count;
+        }
+        if (lm.mine) {
+            out.anchorA[4 * m + lm.slot] = make4(lm.anchorA, lm.depth);
+            out.anchorB[4 * m + lm.slot] = make4(lm.anchorB, 0.0f);
+            out.feature[4 * m + lm.slot] = lm.feature;
+        }
+        if (lane < 4) {
+            if (lane >= (uint32_t)__popc(contacts)) {
+                out.anchorA[4 * m + lane] = make_float4(0, 0, 0, 0);
+                out.anchorB[4 * m + lane] = make_float4(0, 0, 0, 0);
+                out.feature[4 * m + lane] = 0u;
+            }
+            out.impulse[4 * m + lane] = make_float4(0, 0, 0, 0);
+        }
+    }
+    return true;
+}
+
+// One tile, a thread a pair; as laneTile.
+__device__ __forceinline__ bool threadTile(const WorldView &w, const uint32_t *pairA, const uint32_t *pairB,
+                                           uint32_t P, uint32_t ntiles, const ManifoldView &out, uint32_t mcap,
+                                           DevStats *st, unsigned long long *state, NarrowShared &sh) {
+    const uint32_t p = sh.tile * kNarrowThreads + threadIdx.x;
+    PairSide a, b;
     LocalManifold lm;
     lm.count = 0;
-    bool hit = false;
-    uint32_t ca = 0, cb = 0, ba = 0, bb = 0, ga = 0, gb = 0, category = 0;
     float restitution = 0.0f, friction = 0.0f;
+    bool hit = false, epaFailed;
     if (p < P) {
-        ca = pairA[p];
-        cb = pairB[p];
-        bool epaFailed;
-        if (w.npRec) {
-            // both colliders' packed records: one 64-byte line each
-            float4 ra[4], rb[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                ra[k] = w.npRec[4 * (size_t)ca + k];
-                rb[k] = w.npRec[4 * (size_t)cb + k];
-            }
-            ba = __float_as_uint(ra[3].z);
-            bb = __float_as_uint(rb[3].z);
-            ga = __float_as_uint(ra[3].w);
-            gb = __float_as_uint(rb[3].w);
-            hit = narrowphasePairRec(w, ca, cb, ra, rb, lm, restitution, friction, category, epaFailed);
-        } else {
-            ba = w.cbody[ca];
-            bb = w.cbody[cb];
-            ga = w.cbgen[ca];
-            gb = w.cbgen[cb];
-            hit = narrowphasePair(w, ca, cb, ba, bb, lm, restitution, friction, category, epaFailed);
-        }
-        if (epaFailed) atomicAdd(&st->epaFailures, 1ull);
-        aggregatedCount(st->npCandidates, category);
-        if (hit) aggregatedCount(st->npContacts, category);
+        const uint32_t ca = pairA[p], cb = pairB[p];
+        a = loadPairSide(w, ca);
+        b = loadPairSide(w, cb);
+        hit = narrowphaseRecords(w, ca, cb, a, b, lm, restitution, friction, epaFailed);
+        countPair(st, pairCategory(a, b), epaFailed, hit, lm.count);
     }
     uint32_t total;
-    const uint32_t local = blockExclusiveScan(hit ? 1u : 0u, total, s_scan);
+    const uint32_t local = blockExclusiveScan(hit ? 1u : 0u, total, sh.scan);
     if (threadIdx.x < 32) {
         bool timedOut;
-        const uint32_t pre = lookbackExclusiveWarp(state, tile, total, &st->err, &timedOut);
+        const uint32_t pre = lookbackExclusiveWarp(state, sh.tile, total, &st->err, &timedOut);
         if (threadIdx.x == 0) {
-            s_prefix = pre;
-            s_abort = timedOut ? 1u : 0u;
+            sh.prefix = pre;
+            sh.abort = timedOut ? 1u : 0u;
+            if (sh.tile + 1 == ntiles && !timedOut) {
+                st->manifolds = pre + total;
+                st->stamp[3] = globalNs();
+            }
         }
     }
     __syncthreads();
-    if (s_abort) return;  // a bounded wait ran out: nothing of this tile is written
-    const uint32_t m = s_prefix + local;
-    if (hit) {
-        if (m < mcap) storeManifoldGen(out, m, ba, ga, bb, gb, lm, restitution, friction);
-        aggregatedAdd32(&st->points, (uint32_t)lm.count);
+    if (sh.abort) return false;
+    const uint32_t m = sh.prefix + local;
+    if (hit && m < mcap) storeManifoldGen(out, m, a.body, a.gen, b.body, b.gen, lm, restitution, friction);
+    return true;
+}
+
+__global__ void __launch_bounds__(kNarrowThreads, kNarrowBlocks)
+k_narrowphase(WorldView w, const uint32_t *__restrict__ pairA, const uint32_t *__restrict__ pairB,
+              const uint32_t *d_pairs, uint32_t laneMax, ManifoldView out, uint32_t mcap, DevStats *st,
+              unsigned long long *state, uint32_t *counter) {
+    __shared__ NarrowShared sh;
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->stamp[2] = globalNs();
+    const uint32_t P = min(*d_pairs, mcap);
+    if (P == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            st->manifolds = 0;
+            st->stamp[3] = globalNs();
+        }
+        return;
     }
-    if (threadIdx.x == 0 && tile + 1 == ntiles) {
-        st->manifolds = s_prefix + total;
-        st->stamp[3] = globalNs();
-    }
-    __syncthreads();
+    const bool lanes = P <= laneMax;
+    const uint32_t per = lanes ? kNarrowPairs : (uint32_t)kNarrowThreads, ntiles = (P + per - 1) / per;
+    while (takeTile(counter, &sh.tile) < ntiles) {
+        if (!(lanes ? laneTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)
+                    : threadTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)))
+            return;
+        __syncthreads();
     }
 }
 
 void launchNarrowphase(const WorldView &w, const PairBuffers &pb, const ManifoldView &mv, uint32_t mcap, DevStats *st,
                        Scratch &ws, cudaStream_t s, unsigned long long *state, bool stateCleared) {
-    uint32_t tiles = (pb.cap + kNarrowThreads - 1) / kNarrowThreads;
+    uint32_t tiles = (pb.cap + kNarrowPairs - 1) / kNarrowPairs;
     if (tiles == 0) tiles = 1;
     if (!state) state = ws.scanState;
     if (!stateCleared) PE_CHECK(cudaMemsetAsync(state, 0, sizeof(unsigned long long) * (tiles + 1), s));
-    const uint32_t maxGrid = 8u * (uint32_t)smCount();
+    const uint32_t maxGrid = kNarrowBlocks * (uint32_t)smCount();
     const uint32_t grid = tiles < maxGrid ? tiles : maxGrid;
-    k_narrowphase<<<grid, kNarrowThreads, 0, s>>>(w, pb.a, pb.b, &st->pairs, mv, mcap, st, state,
-                                                   (uint32_t *)(state + tiles));
+    k_narrowphase<<<grid, kNarrowThreads, 0, s>>>(w, pb.a, pb.b, &st->pairs, kLaneRounds * kNarrowPairs * maxGrid, mv,
+                                                  mcap, st, state, (uint32_t *)(state + tiles));
     PE_LAUNCHED();
 }
 

@@ -173,6 +173,16 @@ static __device__ __noinline__ void boxFaceCandidates(const V3 &srcHe, const Tf 
     }
 }
 
+// overlapMidpoint (narrowphase.cpp:48-58)
+__device__ __forceinline__ float boxOverlapMidpoint(const V3 &heA, const Tf &tA, const M3 &rA, const V3 &heB,
+                                                    const Tf &tB, const M3 &rB, const V3 &ax) {
+    float cA = dot(tA.p, ax), cB = dot(tB.p, ax);
+    float ra = boxProjectedRadius(heA, rA, ax), rb = boxProjectedRadius(heB, rB, ax);
+    float lower = smax(cA - ra, cB - rb);
+    float upper = smin(cA + ra, cB + rb);
+    return (lower + upper) * 0.5f;
+}
+
 // intersectBoxBox (narrowphase.cpp:250-324)
 __device__ __forceinline__ bool boxBox(const V3 &heA, const Tf &tA, const V3 &heB, const Tf &tB, LocalManifold &m) {
     M3 rA = toMat3(tA.q), rB = toMat3(tB.q);
@@ -196,15 +206,8 @@ __device__ __forceinline__ bool boxBox(const V3 &heA, const Tf &tA, const V3 &he
         float nc = (dot(tA.p, normal) + boxProjectedRadius(heA, rA, normal) + dot(tB.p, normal) -
                     boxProjectedRadius(heB, rB, normal)) *
                    0.5f;
-        // overlapMidpoint (narrowphase.cpp:48-58)
-        auto mid = [&](const V3 &ax) {
-            float cA = dot(tA.p, ax), cB = dot(tB.p, ax);
-            float ra = boxProjectedRadius(heA, rA, ax), rb = boxProjectedRadius(heB, rB, ax);
-            float lower = smax(cA - ra, cB - rb);
-            float upper = smin(cA + ra, cB + rb);
-            return (lower + upper) * 0.5f;
-        };
-        contacts[0] = normal * nc + t1 * mid(t1) + t2 * mid(t2);
+        contacts[0] = normal * nc + t1 * boxOverlapMidpoint(heA, tA, rA, heB, tB, rB, t1) +
+                      t2 * boxOverlapMidpoint(heA, tA, rA, heB, tB, rB, t2);
         depths[0] = penetration;
         feats[0] = kFeatBoxFallback << 24;
         count = 1;
@@ -562,23 +565,155 @@ __device__ inline bool narrowphasePair(const WorldView &w, uint32_t ca, uint32_t
     return hit;
 }
 
-// narrowphasePair with both colliders read from their packed records
-// (WorldView::npRec, written by the integrate kernel with the same world
-// transforms, shapes and materials): one 64-byte line per collider instead of
-// a gather from a dozen arrays.  ra / rb: the four float4 of each record.
-__device__ inline bool narrowphasePairRec(const WorldView &w, uint32_t ca, uint32_t cb, const float4 *ra,
-                                          const float4 *rb, LocalManifold &lm, float &restitution, float &friction,
-                                          uint32_t &category, bool &epaFailed) {
-    epaFailed = false;
-    lm.count = 0;
-    const uint32_t sa = colliderShape(__float_as_uint(ra[2].w)), sb = colliderShape(__float_as_uint(rb[2].w));
-    const Tf tA{V3{ra[0].x, ra[0].y, ra[0].z}, Q{ra[1].x, ra[1].y, ra[1].z, ra[1].w}};
-    const Tf tB{V3{rb[0].x, rb[0].y, rb[0].z}, Q{rb[1].x, rb[1].y, rb[1].z, rb[1].w}};
-    const float4 sha = make_float4(ra[0].w, ra[2].x, ra[2].y, ra[2].z);
-    const float4 shb = make_float4(rb[0].w, rb[2].x, rb[2].y, rb[2].z);
+// ------------------------------------------------------------------ lanes ---
+// A pair on eight lanes of a warp (the multi-kernel step's narrowphase).
+//
+// A box pair is some 7,000 cycles of dependent arithmetic on one thread: fifteen
+// axes with a square root and two divisions each, then eight face vertices, with
+// the contacts in local memory.  The lanes take two axes and one vertex each, and
+// a contact stays in its lane's registers.  The operations of an axis and of a
+// vertex are those of satBoxBox and boxFaceCandidates; what those decide in order
+// (the first smallest depth; a vertex is dropped when it is close to one kept
+// before it or four are kept) is decided here from the lanes' results in that
+// order.
+constexpr uint32_t kPairLanes = 8;
+
+// What a pair's lanes hold of its manifold: the lane's contact, if it has one.
+struct LaneManifold {
     bool hit;
+    uint32_t count;  // of the manifold
+    V3 normal;
+    bool mine;       // the lane has contact `slot`
+    uint32_t slot;
+    V3 anchorA, anchorB;
+    float depth;
+    uint32_t feature;
+};
+
+__device__ __forceinline__ V3 laneShfl(const V3 &v, uint32_t from) {
+    return {__shfl_sync(0xffffffffu, v.x, from, kPairLanes), __shfl_sync(0xffffffffu, v.y, from, kPairLanes),
+            __shfl_sync(0xffffffffu, v.z, from, kPairLanes)};
+}
+__device__ __forceinline__ V3 pick(bool first, const V3 &a, const V3 &b) {
+    return {first ? a.x : b.x, first ? a.y : b.y, first ? a.z : b.z};
+}
+
+// boxBox on the lanes of a pair; whole warps call it, act: the lane's pair is
+// one of two boxes.  Anchors in collider space.
+__device__ __forceinline__ void boxBoxLanes(bool act, const V3 &heA, const Tf &tA, const V3 &heB, const Tf &tB,
+                                            LaneManifold &o) {
+    const uint32_t t = threadIdx.x & (kPairLanes - 1), shift = threadIdx.x & 24u;
+    const M3 rA = toMat3(tA.q), rB = toMat3(tB.q);
+    const V3 cd = tB.p - tA.p;
+    // two axes a lane (satBoxBox's order: t, then t + 8)
+    float best = 3.402823466e+38f;
+    uint32_t bestAxis = 16;
+    V3 normal{0.0f, 0.0f, 0.0f};
+    bool apart = false;
+#pragma unroll
+    for (uint32_t r = 0; r < 2; ++r) {
+        const uint32_t k = t + r * kPairLanes;
+        V3 ax;
+        if (r == 0 && k < 6) {
+            ax = k < 3 ? matColumn(rA, (int)k) : matColumn(rB, (int)k - 3);
+        } else {
+            const uint32_t e = k - 6, i = e < 3 ? 0 : e < 6 ? 1 : 2;
+            ax = cross(matColumn(rA, (int)i), matColumn(rB, (int)(e - 3 * i)));
+        }
+        if (k < 15) {
+            const float before = best;
+            if (!satAxis(rA, heA, rB, heB, cd, ax, normal, best)) apart = true;
+            if (best < before) bestAxis = k;
+        }
+    }
+    const uint32_t separated = (__ballot_sync(0xffffffffu, apart) >> shift) & 0xFFu;
+    const bool hit = act && separated == 0;
+#pragma unroll
+    for (uint32_t j = 1; j < kPairLanes; j <<= 1) {
+        const float d = __shfl_xor_sync(0xffffffffu, best, j);
+        const uint32_t k = __shfl_xor_sync(0xffffffffu, bestAxis, j);
+        if (d < best || (d == best && k < bestAxis)) {
+            best = d;
+            bestAxis = k;
+        }
+    }
+    normal = laneShfl(normal, bestAxis & (kPairLanes - 1));
+    if (dot(cd, normal) < 0.0f) normal = -normal;
+    // one face vertex a lane: box A's face along the normal, then box B's
+    const bool fromA = t < 4;
+    const uint32_t vi = t & 3;
+    const V3 dir = pick(fromA, normal, -normal);
+    const V3 srcHe = pick(fromA, heA, heB), othHe = pick(fromA, heB, heA);
+    const Tf srcTf{pick(fromA, tA.p, tB.p), fromA ? tA.q : tB.q}, othTf{pick(fromA, tB.p, tA.p), fromA ? tB.q : tA.q};
+    const float otherSurface = dot(boxSupport(othHe, othTf, -dir), dir);
+    const V3 ld = rotate(conj(srcTf.q), dir);
+    int faceAxis = 0;
+    float largest = fabsf(ld.x);
+    if (fabsf(ld.y) > largest) { faceAxis = 1; largest = fabsf(ld.y); }
+    if (fabsf(ld.z) > largest) faceAxis = 2;
+    const float comp = faceAxis == 0 ? ld.x : faceAxis == 1 ? ld.y : ld.z;
+    const bool positive = comp >= 0.0f, first = vi & 1, second = vi & 2;
+    // (the face's first side axis follows the face axis, the second follows that)
+    const bool upX = faceAxis == 0 ? positive : faceAxis == 2 ? first : second;
+    const bool upY = faceAxis == 1 ? positive : faceAxis == 0 ? first : second;
+    const bool upZ = faceAxis == 2 ? positive : faceAxis == 1 ? first : second;
+    const V3 v = toWorld(V3{upX ? srcHe.x : -srcHe.x, upY ? srcHe.y : -srcHe.y, upZ ? srcHe.z : -srcHe.z}, srcTf);
+    const V3 l = rotate(conj(othTf.q), v - othTf.p);
+    const float tol = 1e-4f;
+    const bool inside = fabsf(l.x) <= othHe.x + tol && fabsf(l.y) <= othHe.y + tol && fabsf(l.z) <= othHe.z + tol;
+    float depth = smax(dot(v, dir) - otherSurface, 0.0f);
+    V3 contact = v - dir * (depth * 0.5f);
+    uint32_t feature = (kFeatBoxFace << 24) | ((fromA ? 0u : 1u) << 16) | ((uint32_t)faceAxis << 8) |
+                       ((positive ? 0u : 1u) << 4) | vi;
+    uint32_t near = 0;  // vertices within the duplicate distance of this lane's
+#pragma unroll
+    for (uint32_t q = 0; q < kPairLanes; ++q) {
+        const V3 d = laneShfl(contact, q) - contact;
+        if (dot(d, d) <= 1e-6f) near |= 1u << q;
+    }
+    const uint32_t in = (__ballot_sync(0xffffffffu, inside) >> shift) & 0xFFu;
+    uint32_t kept = 0, count = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kPairLanes; ++q) {
+        const uint32_t nq = __shfl_sync(0xffffffffu, near, q, kPairLanes);
+        if (((in >> q) & 1u) && count < 4 && !(nq & kept)) {
+            kept |= 1u << q;
+            ++count;
+        }
+    }
+    if (!act) return;
+    o.hit = hit;
+    o.normal = normal;
+    o.count = count;
+    o.mine = (kept >> t) & 1u;
+    o.slot = __popc(kept & ((1u << t) - 1u));
+    if (hit && count == 0) {
+        // Fallback contact (narrowphase.cpp:270-276, 308-312), as in boxBox.
+        V3 tref = fabsf(normal.x) < 0.9f ? V3{1.0f, 0.0f, 0.0f} : V3{0.0f, 1.0f, 0.0f};
+        V3 t1 = normalize(cross(normal, tref));
+        V3 t2 = cross(normal, t1);
+        float nc = (dot(tA.p, normal) + boxProjectedRadius(heA, rA, normal) + dot(tB.p, normal) -
+                    boxProjectedRadius(heB, rB, normal)) *
+                   0.5f;
+        contact = normal * nc + t1 * boxOverlapMidpoint(heA, tA, rA, heB, tB, rB, t1) +
+                  t2 * boxOverlapMidpoint(heA, tA, rA, heB, tB, rB, t2);
+        depth = best;
+        feature = kFeatBoxFallback << 24;
+        o.count = 1;
+        o.mine = t == 0;
+        o.slot = 0;
+    }
+    o.depth = depth;
+    o.anchorA = toLocal(contact, tA);
+    o.anchorB = toLocal(contact, tB);
+    o.feature = feature;
+}
+
+// One contact of a pair that is not two boxes, on its first lane.
+__device__ __forceinline__ bool singleContact(const WorldView &w, uint32_t sa, const float4 &sha, const Tf &tA,
+                                              uint32_t sb, const float4 &shb, const Tf &tB, LocalManifold &lm,
+                                              bool &epaFailed) {
     if (sa == kShapeHull || sb == kShapeHull) {
-        category = 3;
         auto support = [&](uint32_t shape, const float4 &sh, const Tf &t) {
             SupportShape s;
             s.shape = shape;
@@ -595,42 +730,94 @@ __device__ inline bool narrowphasePairRec(const WorldView &w, uint32_t ca, uint3
             }
             return s;
         };
-        hit = hullContact(support(sa, sha, tA), support(sb, shb, tB), lm, epaFailed);
-    } else {
-        category = sa + sb;
-        if (sa == kShapeSphere && sb == kShapeSphere) {
-            hit = sphereSphere(sha.x, tA, shb.x, tB, lm);
-        } else if (sa == kShapeSphere) {
-            hit = sphereBox(sha.x, tA, V3{shb.x, shb.y, shb.z}, tB, lm);
-        } else if (sb == kShapeSphere) {
-            hit = sphereBox(shb.x, tB, V3{sha.x, sha.y, sha.z}, tA, lm);
-            if (hit) {
-                lm.normal = -lm.normal;
-                for (uint32_t k = 0; k < lm.count; ++k) {
-                    V3 t = lm.anchorA[k];
-                    lm.anchorA[k] = lm.anchorB[k];
-                    lm.anchorB[k] = t;
-                }
-            }
-        } else {
-            hit = boxBox(V3{sha.x, sha.y, sha.z}, tA, V3{shb.x, shb.y, shb.z}, tB, lm);
+        return hullContact(support(sa, sha, tA), support(sb, shb, tB), lm, epaFailed);
+    }
+    if (sa == kShapeSphere && sb == kShapeSphere) return sphereSphere(sha.x, tA, shb.x, tB, lm);
+    if (sa == kShapeSphere) return sphereBox(sha.x, tA, V3{shb.x, shb.y, shb.z}, tB, lm);
+    if (!sphereBox(shb.x, tB, V3{sha.x, sha.y, sha.z}, tA, lm)) return false;
+    lm.normal = -lm.normal;
+    const V3 t = lm.anchorA[0];
+    lm.anchorA[0] = lm.anchorB[0];
+    lm.anchorB[0] = t;
+    return true;
+}
+
+// A collider's packed record (WorldView::npRec, written by the integrate kernel:
+// world transform, shape, material, body): one 64-byte line instead of a gather
+// from a dozen arrays.
+struct PairSide {
+    Tf t;
+    float4 dims;
+    float restitution, friction;
+    uint32_t shape, body, gen;
+};
+__device__ __forceinline__ PairSide loadPairSide(const WorldView &w, uint32_t collider) {
+    const float4 *r = w.npRec + 4 * (size_t)collider;
+    const float4 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
+    return {Tf{f4xyz(r0), f4q(r1)}, make_float4(r0.w, r2.x, r2.y, r2.z), r3.x, r3.y,
+            colliderShape(__float_as_uint(r2.w)), __float_as_uint(r3.z), __float_as_uint(r3.w)};
+}
+// Category of a pair's counters, and what a contact takes from both materials.
+__device__ __forceinline__ uint32_t pairCategory(const PairSide &a, const PairSide &b) {
+    return a.shape == kShapeHull || b.shape == kShapeHull ? 3u : a.shape + b.shape;
+}
+__device__ __forceinline__ void pairMaterial(const PairSide &a, const PairSide &b, float &restitution,
+                                             float &friction) {
+    restitution = smax(a.restitution, b.restitution);
+    friction = sqrtf(smax(a.friction, 0.0f) * smax(b.friction, 0.0f));
+}
+// An anchor from collider space to body space (local transforms only when some
+// collider has one).
+__device__ __forceinline__ V3 bodyAnchor(const WorldView &w, uint32_t collider, const V3 &anchor) {
+    const V3 lp = w.clpos ? f4xyz(w.clpos[collider]) : V3{0.0f, 0.0f, 0.0f};
+    const Q lq = w.clrot ? f4q(w.clrot[collider]) : qidentity();
+    return lp + rotate(lq, anchor);
+}
+
+// narrowphasePair from the records, on one thread and on the lanes of a pair
+// (whole warps call it; act: the lanes have a pair).
+__device__ __forceinline__ bool narrowphaseRecords(const WorldView &w, uint32_t ca, uint32_t cb, const PairSide &a,
+                                                   const PairSide &b, LocalManifold &lm, float &restitution,
+                                                   float &friction, bool &epaFailed) {
+    epaFailed = false;
+    lm.count = 0;
+    const bool boxes = a.shape == kShapeBox && b.shape == kShapeBox;
+    if (!(boxes ? boxBox(V3{a.dims.x, a.dims.y, a.dims.z}, a.t, V3{b.dims.x, b.dims.y, b.dims.z}, b.t, lm)
+                : singleContact(w, a.shape, a.dims, a.t, b.shape, b.dims, b.t, lm, epaFailed)))
+        return false;
+    for (uint32_t k = 0; k < lm.count; ++k) {
+        lm.anchorA[k] = bodyAnchor(w, ca, lm.anchorA[k]);
+        lm.anchorB[k] = bodyAnchor(w, cb, lm.anchorB[k]);
+    }
+    pairMaterial(a, b, restitution, friction);
+    return true;
+}
+__device__ __forceinline__ void narrowphaseLanes(const WorldView &w, bool act, uint32_t ca, uint32_t cb,
+                                                 const PairSide &a, const PairSide &b, LaneManifold &o,
+                                                 float &restitution, float &friction, bool &epaFailed) {
+    epaFailed = false;
+    o.hit = o.mine = false;
+    o.count = o.slot = 0;
+    const bool boxes = act && a.shape == kShapeBox && b.shape == kShapeBox;
+    if (__any_sync(0xffffffffu, boxes))
+        boxBoxLanes(boxes, V3{a.dims.x, a.dims.y, a.dims.z}, a.t, V3{b.dims.x, b.dims.y, b.dims.z}, b.t, o);
+    if (act && !boxes && (threadIdx.x & (kPairLanes - 1)) == 0) {
+        LocalManifold lm;
+        o.hit = singleContact(w, a.shape, a.dims, a.t, b.shape, b.dims, b.t, lm, epaFailed);
+        if (o.hit) {
+            o.mine = true;
+            o.count = 1;
+            o.normal = lm.normal;
+            o.anchorA = lm.anchorA[0];
+            o.anchorB = lm.anchorB[0];
+            o.depth = lm.depth[0];
+            o.feature = lm.feature[0];
         }
     }
-    if (hit) {
-        // anchors from collider space to body space (local transforms only
-        // when some collider has one)
-        const V3 lpa = w.clpos ? f4xyz(w.clpos[ca]) : V3{0.0f, 0.0f, 0.0f};
-        const Q lqa = w.clrot ? f4q(w.clrot[ca]) : qidentity();
-        const V3 lpb = w.clpos ? f4xyz(w.clpos[cb]) : V3{0.0f, 0.0f, 0.0f};
-        const Q lqb = w.clrot ? f4q(w.clrot[cb]) : qidentity();
-        for (uint32_t k = 0; k < lm.count; ++k) {
-            lm.anchorA[k] = lpa + rotate(lqa, lm.anchorA[k]);
-            lm.anchorB[k] = lpb + rotate(lqb, lm.anchorB[k]);
-        }
-        restitution = smax(ra[3].x, rb[3].x);
-        friction = sqrtf(smax(ra[3].y, 0.0f) * smax(rb[3].y, 0.0f));
-    }
-    return hit;
+    if (!o.hit) return;
+    o.anchorA = bodyAnchor(w, ca, o.anchorA);
+    o.anchorB = bodyAnchor(w, cb, o.anchorB);
+    pairMaterial(a, b, restitution, friction);
 }
 
 // Writes one manifold record in pair order: body handles, collider-space

@@ -13,7 +13,7 @@ struct BroadInput {
 
 // Fewest items per tile of any single-pass kernel with a tile look-back
 // (scratch holds one state word per tile).
-constexpr uint32_t kMinLookbackTile = 64;
+constexpr uint32_t kMinLookbackTile = 32;
 
 struct BroadBuffers {
     // SAP

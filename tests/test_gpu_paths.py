@@ -3,7 +3,8 @@ against another path that gives the same result by definition."""
 import numpy as np
 import pytest
 
-from helpers import assert_bit_equal
+from helpers import assert_bit_equal, assert_manifolds_equal
+from oracle import cpu
 from phys_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
@@ -204,3 +205,31 @@ def test_whole_grid_sweeps_survive_changes_of_path(gpu):
         g.step(1 / 120)
         o.step(1 / 120)
         compare_worlds(g, o, f"phase {phase} after the removal")
+
+
+@pytest.mark.parametrize("pairs", [1, 4, 31, 32, 33, 700, 38912, 38913, 45000])
+def test_narrowphase_matches_the_oracle_for_any_number_of_pairs(gpu, pairs):
+    """Couples of turned boxes and spheres, each couple alone: tiles of 32 pairs
+    on eight lanes each up to 38,912 pairs (on 152 SMs), a thread a pair beyond."""
+    rng = np.random.default_rng(pairs)
+    n = 2 * pairs
+    k = np.arange(pairs)
+    cell = np.stack([k % 256, k // 256, np.zeros(pairs)], 1) * 6.0
+    pos = np.repeat(cell, 2, 0)
+    pos[1::2] += rng.uniform(-0.45, 0.45, (pairs, 3))  # every couple's boxes overlap
+    sc = sphere_scene(pos, np.full(n, 0.6), np.zeros(n))
+    sc.shape[:] = rng.random(n) < 0.75
+    boxes = sc.shape == 1
+    sc.dims[boxes] = rng.uniform(0.5, 1.5, (int(boxes.sum()), 3))
+    sc.dims[boxes & (rng.random(n) < 0.4)] = 1.0
+    sc.spin[:] = rng.uniform(-20.0, 20.0, (n, 3)) * (rng.random((n, 1)) < 0.7)
+    gw = gpu.GpuWorld(algo=gpu.SAP, iterations=2, order=gpu.ORDER_COLOR)
+    ow = cpu.OracleWorld(algo=0, iterations=2, order_mode=1)
+    for w in (gw, ow):
+        w.load_scene(sc)
+    for step in range(3):
+        gw.step(1 / 60)
+        ow.step(1 / 60)
+        assert step > 0 or len(gw.pairs()) == pairs
+        assert_bit_equal(gw.pairs(), ow.pairs(), f"{pairs} step {step} pairs")
+        assert_manifolds_equal(gw.contacts(), ow.contacts(), what=f"{pairs} step {step}")
