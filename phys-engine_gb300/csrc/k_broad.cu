@@ -176,6 +176,113 @@ constexpr int kSapBlockThreads = (int)kRegSortThreads;
 constexpr size_t kSapBlockSmem = (size_t)kSapBlockMax * (8 + 8 + 16 + 4 + 4 + 4 + 4) + (size_t)kSapBlockPairs * 4;
 static_assert(kSapBlockPairs * 4 <= kSapBlockMax * 8, "pair flags fit one key buffer");
 
+// Order of P <= kSapBlockPairs raw pairs without duplicates among n <= kSapBlockMax
+// boxes: sPairs holds first << bits | second, sCnt the pairs of each first index.
+// Scratch: sSec kSapBlockPairs words, sLong n, sBits kSapBlockMax bits a warp.
+__device__ __forceinline__ void orderPairLists(uint32_t *sPairs, uint32_t *sCnt, uint32_t *sSec, uint32_t *sLong,
+                                               uint32_t *sBits, uint32_t &count, uint32_t *s_scan, uint32_t n,
+                                               uint32_t P, uint32_t bits, const uint32_t *inSlot,
+                                               const uint32_t *cbody, const uint32_t *cbgen, uint32_t *pairA,
+                                               uint32_t *pairB, DevStats *st) {
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    const uint32_t mask = (1u << bits) - 1u;
+    // Pairs in order of their first index: list offsets, then a scatter with
+    // the counters as cursors (afterwards sCnt[f] is the end of f's list).
+    blockExclusiveScanArray(sCnt, n, s_scan);  // ends with a barrier
+    if (tid == 0) count = 0;                 // now counts the long lists
+    for (uint32_t k = tid; k < P; k += nt) {
+        const uint32_t key = sPairs[k];
+        sSec[atomicAdd(&sCnt[key >> bits], 1u)] = key & mask;
+    }
+    __syncthreads();
+    // Short lists: one thread sorts its list (insertion) and writes the full
+    // keys back in order; long ones are queued for a warp.
+    constexpr uint32_t kShortList = 32;
+    for (uint32_t f = tid; f < n; f += nt) {
+        const uint32_t begin = f ? sCnt[f - 1] : 0u, end = sCnt[f];
+        if (end - begin > kShortList) {
+            sLong[aggregatedAppend(&count)] = f;
+            continue;
+        }
+        for (uint32_t x = begin + 1; x < end; ++x) {
+            const uint32_t v = sSec[x];
+            uint32_t y = x;
+            for (; y > begin && sSec[y - 1] > v; --y) sSec[y] = sSec[y - 1];
+            sSec[y] = v;
+        }
+        for (uint32_t x = begin; x < end; ++x) sPairs[x] = f << bits | sSec[x];
+    }
+    __syncthreads();
+    {
+        const uint32_t lane = tid & 31, warp = tid >> 5, nLong = count;
+        constexpr uint32_t kWords = kSapBlockMax / 32, kPerLane = kWords / 32;
+        uint32_t *bm = sBits + warp * kWords;
+        for (uint32_t q = warp; q < nLong; q += nt / 32) {
+            const uint32_t f = sLong[q];
+            const uint32_t begin = f ? sCnt[f - 1] : 0u, end = sCnt[f];
+#pragma unroll
+            for (uint32_t r = 0; r < kPerLane; ++r) bm[lane * kPerLane + r] = 0u;
+            __syncwarp();
+            for (uint32_t x = begin + lane; x < end; x += 32) atomicOr(&bm[sSec[x] >> 5], 1u << (sSec[x] & 31u));
+            __syncwarp();
+            // lane l owns words [l kPerLane, (l + 1) kPerLane): its set bits
+            // come after those of the lanes before it
+            uint32_t words[kPerLane], cnt = 0;
+#pragma unroll
+            for (uint32_t r = 0; r < kPerLane; ++r) {
+                words[r] = bm[lane * kPerLane + r];
+                cnt += __popc(words[r]);
+            }
+            uint32_t incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)lane >= o) incl += t;
+            }
+            uint32_t out = begin + incl - cnt;
+#pragma unroll
+            for (uint32_t r = 0; r < kPerLane; ++r)
+                for (uint32_t wbits = words[r]; wbits; wbits &= wbits - 1u)
+                    sPairs[out++] = f << bits | ((lane * kPerLane + r) * 32u + (uint32_t)(__ffs(wbits) - 1));
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // slot mapping, same-body filter, compaction (k_pairs_block)
+    uint32_t *sFlag = sSec;
+    uint32_t unique = 0;
+    for (uint32_t k = tid; k < P; k += nt) {
+        const uint32_t key = sPairs[k];
+        bool keep = !(k > 0 && sPairs[k - 1] == key);
+        if (keep) {
+            ++unique;
+            uint32_t a = key >> bits, b = key & mask;
+            if (inSlot) {
+                a = inSlot[a];
+                b = inSlot[b];
+            }
+            if (cbody && cbody[a] == cbody[b] && cbgen[a] == cbgen[b]) keep = false;
+        }
+        sFlag[k] = keep ? 1u : 0u;
+    }
+    if (unique) atomicAdd(&st->uniquePairs, unique);
+    __syncthreads();
+    const uint32_t total = blockExclusiveScanArray(sFlag, P, s_scan);
+    for (uint32_t k = tid; k < P; k += nt) {
+        const uint32_t next = k + 1 < P ? sFlag[k + 1] : total;
+        if (next == sFlag[k]) continue;
+        const uint32_t key = sPairs[k];
+        uint32_t a = key >> bits, b = key & mask;
+        if (inSlot) {
+            a = inSlot[a];
+            b = inSlot[b];
+        }
+        pairA[sFlag[k]] = a;
+        pairB[sFlag[k]] = b;
+    }
+    if (tid == 0) st->pairs = total;
+}
+
 template <int E>
 __device__ __forceinline__ void sapSortKeys(const BroadInput &in, uint32_t n, unsigned long long *bufA,
                                             unsigned long long *bufB, uint32_t *sapKeys, uint32_t *sapVals,
@@ -296,105 +403,8 @@ k_sap_block(BroadInput in, uint32_t *sapKeys, uint32_t *sapVals, uint32_t *unsor
         if (tid == 0) atomicOr(&st->err, kErrSmallPath);
         return;
     }
-    const uint32_t mask = (1u << bits) - 1u;
-    // Pairs in order of their first index: list offsets, then a scatter with
-    // the counters as cursors (afterwards sCnt[f] is the end of f's list).
-    uint32_t *sSec = reinterpret_cast<uint32_t *>(bufB);      // second indices by list
-    uint32_t *sLong = sOff;                                   // first indices with long lists
-    uint32_t *sBits = reinterpret_cast<uint32_t *>(sYZ);      // a bitmap of kSapBlockMax bits per warp
-    blockExclusiveScanArray(sCnt, n, s_scan);  // ends with a barrier
-    if (tid == 0) s_count = 0;                 // now counts the long lists
-    for (uint32_t k = tid; k < P; k += nt) {
-        const uint32_t key = sPairs[k];
-        sSec[atomicAdd(&sCnt[key >> bits], 1u)] = key & mask;
-    }
-    __syncthreads();
-    // Short lists: one thread sorts its list (insertion) and writes the full
-    // keys back in order; long ones are queued for a warp.
-    constexpr uint32_t kShortList = 32;
-    for (uint32_t f = tid; f < n; f += nt) {
-        const uint32_t begin = f ? sCnt[f - 1] : 0u, end = sCnt[f];
-        if (end - begin > kShortList) {
-            sLong[aggregatedAppend(&s_count)] = f;
-            continue;
-        }
-        for (uint32_t x = begin + 1; x < end; ++x) {
-            const uint32_t v = sSec[x];
-            uint32_t y = x;
-            for (; y > begin && sSec[y - 1] > v; --y) sSec[y] = sSec[y - 1];
-            sSec[y] = v;
-        }
-        for (uint32_t x = begin; x < end; ++x) sPairs[x] = f << bits | sSec[x];
-    }
-    __syncthreads();
-    {
-        const uint32_t lane = tid & 31, warp = tid >> 5, nLong = s_count;
-        constexpr uint32_t kWords = kSapBlockMax / 32, kPerLane = kWords / 32;
-        uint32_t *bm = sBits + warp * kWords;
-        for (uint32_t q = warp; q < nLong; q += nt / 32) {
-            const uint32_t f = sLong[q];
-            const uint32_t begin = f ? sCnt[f - 1] : 0u, end = sCnt[f];
-#pragma unroll
-            for (uint32_t r = 0; r < kPerLane; ++r) bm[lane * kPerLane + r] = 0u;
-            __syncwarp();
-            for (uint32_t x = begin + lane; x < end; x += 32) atomicOr(&bm[sSec[x] >> 5], 1u << (sSec[x] & 31u));
-            __syncwarp();
-            // lane l owns words [l kPerLane, (l + 1) kPerLane): its set bits
-            // come after those of the lanes before it
-            uint32_t words[kPerLane], cnt = 0;
-#pragma unroll
-            for (uint32_t r = 0; r < kPerLane; ++r) {
-                words[r] = bm[lane * kPerLane + r];
-                cnt += __popc(words[r]);
-            }
-            uint32_t incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)lane >= o) incl += t;
-            }
-            uint32_t out = begin + incl - cnt;
-#pragma unroll
-            for (uint32_t r = 0; r < kPerLane; ++r)
-                for (uint32_t wbits = words[r]; wbits; wbits &= wbits - 1u)
-                    sPairs[out++] = f << bits | ((lane * kPerLane + r) * 32u + (uint32_t)(__ffs(wbits) - 1));
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    // slot mapping, same-body filter, compaction (k_pairs_block)
-    uint32_t *sFlag = reinterpret_cast<uint32_t *>(bufB);
-    uint32_t unique = 0;
-    for (uint32_t k = tid; k < P; k += nt) {
-        const uint32_t key = sPairs[k];
-        bool keep = !(k > 0 && sPairs[k - 1] == key);
-        if (keep) {
-            ++unique;
-            uint32_t a = key >> bits, b = key & mask;
-            if (inSlot) {
-                a = inSlot[a];
-                b = inSlot[b];
-            }
-            if (cbody && cbody[a] == cbody[b] && cbgen[a] == cbgen[b]) keep = false;
-        }
-        sFlag[k] = keep ? 1u : 0u;
-    }
-    if (unique) atomicAdd(&st->uniquePairs, unique);
-    __syncthreads();
-    const uint32_t total = blockExclusiveScanArray(sFlag, P, s_scan);
-    for (uint32_t k = tid; k < P; k += nt) {
-        const uint32_t next = k + 1 < P ? sFlag[k + 1] : total;
-        if (next == sFlag[k]) continue;
-        const uint32_t key = sPairs[k];
-        uint32_t a = key >> bits, b = key & mask;
-        if (inSlot) {
-            a = inSlot[a];
-            b = inSlot[b];
-        }
-        pairA[sFlag[k]] = a;
-        pairB[sFlag[k]] = b;
-    }
-    if (tid == 0) st->pairs = total;
+    orderPairLists(sPairs, sCnt, reinterpret_cast<uint32_t *>(bufB), sOff, reinterpret_cast<uint32_t *>(sYZ), s_count,
+                   s_scan, n, P, bits, inSlot, cbody, cbgen, pairA, pairB, st);
 }
 
 // --------------------------------------------------------------- grid ------
@@ -1273,6 +1283,47 @@ k_pairs_block(const unsigned long long *keys, uint32_t bits, const uint32_t *inS
         pairB[s_flag[k]] = b;
     }
     if (threadIdx.x == 0) st->pairs = total;
+}
+
+// The finalize of the raw pairs of up to kSapBlockMax boxes, each emitted once.
+__global__ void __launch_bounds__(1024)
+k_pairs_lists(const unsigned long long *keys, uint32_t cap, const uint32_t *d_n, uint32_t bits, const uint32_t *inSlot,
+              const uint32_t *cbody, const uint32_t *cbgen, uint32_t *pairA, uint32_t *pairB, DevStats *st) {
+    extern __shared__ __align__(16) uint32_t s_lists[];
+    uint32_t *sPairs = s_lists, *sSec = sPairs + kSapBlockPairs, *sCnt = sSec + kSapBlockPairs;
+    uint32_t *sLong = sCnt + kSapBlockMax, *sBits = sLong + kSapBlockMax;
+    __shared__ uint32_t s_count, s_scan[40];
+    const uint32_t P = st->rawPairs, n = min(*d_n, kSapBlockMax);
+    if (P > kSapBlockPairs || P > cap) {  // more pairs than the buffer: the host grows it
+        if (threadIdx.x == 0) atomicOr(&st->err, kErrSmallPath);
+        return;
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sCnt[i] = 0u;
+    __syncthreads();
+    const unsigned long long mask = (1ull << bits) - 1ull;
+    for (uint32_t k = threadIdx.x; k < P; k += blockDim.x) {
+        const unsigned long long key = keys[k];
+        const uint32_t first = (uint32_t)(key >> bits);
+        sPairs[k] = first << bits | (uint32_t)(key & mask);
+        atomicAdd(&sCnt[first], 1u);
+    }
+    __syncthreads();
+    orderPairLists(sPairs, sCnt, sSec, sLong, sBits, s_count, s_scan, n, P, bits, inSlot, cbody, cbgen, pairA, pairB,
+                   st);
+}
+
+bool launchPairsLists(const BroadInput &in, const PairMapping &mapping, PairBuffers &pb, DevStats *st, cudaStream_t s) {
+    if (!sapFinalizesPairs(in, pb)) return false;
+    static bool configured = false;
+    const size_t smem = sizeof(uint32_t) * (2 * kSapBlockPairs + 2 * kSapBlockMax + kSapBlockMax);
+    if (!configured) {
+        PE_CHECK(cudaFuncSetAttribute(k_pairs_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = true;
+    }
+    k_pairs_lists<<<1, 1024, smem, s>>>(pb.keys, pb.cap, in.d_n, pb.bits, mapping.inSlot, mapping.cbody, mapping.cbgen, pb.a,
+                                        pb.b, st);
+    PE_LAUNCHED();
+    return true;
 }
 
 void launchPairsFinalize(const uint32_t *inSlot, const uint32_t *cbody, const uint32_t *cbgen, PairBuffers &pb,

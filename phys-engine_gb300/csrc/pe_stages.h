@@ -56,9 +56,10 @@ struct BroadBuffers {
 struct LbvhBuffers {
     unsigned long long *keys, *keysTmp;   // Morton code << index bits | index
     uint32_t *childL, *childR, *parent;   // internal nodes (leaf children flagged)
-    uint32_t *leafParent, *rangeMax, *visit;
+    uint32_t *leafParent, *visit;
     float4 *leafMn, *leafMx;              // leaf bounds in sorted order
     float4 *nodeMn, *nodeMx;              // internal node bounds
+    float4 *rec;                          // [4 n] internal nodes: both children's bounds
     uint32_t *box;                        // [6] ordered-float bounds of the centres
 };
 
@@ -213,8 +214,12 @@ void launchGrid(const BroadInput &in, double fixedCell, BroadBuffers &bb, PairBu
                 cudaStream_t s);
 // DynamicTree: every overlapping pair through a linear BVH (pair keys for
 // launchPairsFinalize).
-void launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, DevStats *st, Scratch &ws,
-                cudaStream_t s);
+bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, DevStats *st, Scratch &ws,
+                cudaStream_t s, const PairMapping &finalize);
+// The finalize of small worlds' raw pairs without duplicates (SAP and the tree), in
+// one block by lists instead of a sort; false, launching nothing, when they may not
+// fit it.
+bool launchPairsLists(const BroadInput &in, const PairMapping &mapping, PairBuffers &pb, DevStats *st, cudaStream_t s);
 // Grid pairs emitted body by body in lexicographic order, mapped to slots and
 // filtered (replaces the per-cell pairs and the finalize when pb.bodyPath).
 void launchGridBodyPairs(const BroadInput &in, const BroadBuffers &bb, PairBuffers &pb, const uint32_t *inSlot,

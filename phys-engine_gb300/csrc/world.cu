@@ -703,16 +703,16 @@ void World::ensureLbvh() {
     lbChildR_.reserve(n);
     lbParent_.reserve(n);
     lbLeafParent_.reserve(n);
-    lbRangeMax_.reserve(n);
     lbVisit_.reserve(n);
     lbBox_.reserve(8);
     lbLeafMn_.reserve(n);
     lbLeafMx_.reserve(n);
     lbNodeMn_.reserve(n);
     lbNodeMx_.reserve(n);
+    lbRec_.reserve(4 * (size_t)n);
     lb_ = LbvhBuffers{lbKeys_.ptr,     lbKeysTmp_.ptr, lbChildL_.ptr,  lbChildR_.ptr,   lbParent_.ptr,
-                      lbLeafParent_.ptr, lbRangeMax_.ptr, lbVisit_.ptr,  lbLeafMn_.ptr,   lbLeafMx_.ptr,
-                      lbNodeMn_.ptr,   lbNodeMx_.ptr,  lbBox_.ptr};
+                      lbLeafParent_.ptr, lbVisit_.ptr,  lbLeafMn_.ptr,   lbLeafMx_.ptr,
+                      lbNodeMn_.ptr,   lbNodeMx_.ptr,  lbRec_.ptr, lbBox_.ptr};
 }
 
 WorldView World::view(float dt) {
@@ -796,7 +796,7 @@ void World::runPipeline(float dt) {
     bool finalized = false;
     if (sap) finalized = launchSap(in, sapKeys_.ptr, sapVals_.ptr, bb_, pb_, st, ws_, s, dense_ ? &coh : nullptr,
                                    &mapping);
-    else if (algorithm == 2) launchLbvh(in, lb_, pb_, st, ws_, s);
+    else if (algorithm == 2) finalized = launchLbvh(in, lb_, pb_, st, ws_, s, mapping);
     else launchGrid(in, cellSize, bb_, pb_, st, ws_, s);
     if (!sap && pb_.bodyPath)
         launchGridBodyPairs(in, bb_, pb_, mapping.inSlot, cbody_.ptr, cbgen_.ptr, st, ws_, s, fused);

@@ -39,6 +39,26 @@ def test_tree_reports_each_pair_once_whatever_the_sizes(gpu, n, sizes):
     assert_bit_equal(got[gpu.TREE], got[gpu.SAP], f"{n} {sizes}")
 
 
+@pytest.mark.parametrize("n", [1024, 1025, 2048, 2049, 4096])
+@pytest.mark.parametrize("alike", [False, True])
+def test_tree_built_in_one_block(gpu, n, alike):
+    """Sizes at which the block's keys a thread change (one, two, four); alike:
+    an eighth of the spheres in one place, so that only the index tells their keys apart
+    and a walk finds hundreds of leaves."""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(-12.0, 12.0, (n, 3))
+    if alike:
+        pos[: n // 8] = pos[0]
+    sc = sphere_scene(pos, np.full(n, 0.25), np.zeros(n))
+    got = {}
+    for algo in (gpu.SAP, gpu.TREE):
+        w = gpu.GpuWorld(algo=algo, iterations=1)
+        w.load_scene(sc)
+        w.step(1e-4)
+        got[algo] = w.pairs()
+    assert_bit_equal(got[gpu.TREE], got[gpu.SAP], f"{n} {alike}")
+
+
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 515])
 @pytest.mark.parametrize("offset", [0, 1, 3])
 def test_batch_poses_reach_any_array(gpu, n, offset):
