@@ -155,7 +155,8 @@ __device__ __forceinline__ unsigned long long mortonKey(const float4 &a, const f
     return ((unsigned long long)code << indexBits) | i;
 }
 
-__global__ void k_lbvh_codes(BroadInput in, const uint32_t *box, unsigned long long *keys, uint32_t indexBits) {
+__global__ void k_lbvh_codes(BroadInput in, const uint32_t *box, unsigned long long *keys, uint32_t indexBits,
+                             uint32_t *counts) {
     const uint32_t n = *in.d_n;
     float lo[3], scale[3];
 #pragma unroll
@@ -164,8 +165,10 @@ __global__ void k_lbvh_codes(BroadInput in, const uint32_t *box, unsigned long l
         const float ext = orderedFloatDecode(box[3 + k]) - lo[k];
         scale[k] = ext > 0.0f ? 1024.0f / ext : 0.0f;
     }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         keys[i] = mortonKey(in.mn[i], in.mx[i], lo, scale, indexBits, i);
+        if (counts) counts[i] = 0u;  // for the walk's pairs
+    }
 }
 
 // Internal node i of n - 1 over the sorted keys: the leaves lo .. hi it covers,
@@ -385,7 +388,7 @@ inline int lbvhWalkGrid(uint32_t n) {
 __global__ void __launch_bounds__(kLbvhWalkThreads)
 k_lbvh_pairs(const uint32_t *d_n, const unsigned long long *keys, uint32_t indexBits, const float4 *leafMn,
              const float4 *leafMx, const float4 *rec, unsigned long long *pkeys, uint32_t cap, uint32_t bits,
-             DevStats *st) {
+             uint32_t *counts, uint32_t *ranks, DevStats *st) {
     __shared__ uint32_t s_stack[kWalkLeaves][kWalkStack];
     const uint32_t n = *d_n;
     if (n < 2) return;
@@ -447,7 +450,9 @@ k_lbvh_pairs(const uint32_t *d_n, const unsigned long long *keys, uint32_t index
                     if (!hit[e]) continue;
                     const uint32_t at = slot + (e ? __popc(hit0) + __popc(hit1 & before) : __popc(hit0 & before));
                     const uint32_t oi = (uint32_t)(keys[c[e]] & idxMask);
-                    if (at < cap) pkeys[at] = ((unsigned long long)min(qi, oi) << bits) | max(qi, oi);
+                    if (at >= cap) continue;
+                    pkeys[at] = ((unsigned long long)min(qi, oi) << bits) | max(qi, oi);
+                    if (counts) ranks[at] = aggregatedAppendKeyed(counts, min(qi, oi));
                 }
             }
         }
@@ -469,6 +474,7 @@ bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, De
                 cudaStream_t s, const PairMapping &finalize) {
     uint32_t indexBits = 1;
     while (indexBits < 32 && (1ull << indexBits) < (unsigned long long)(in.maxN > 2 ? in.maxN : 2)) ++indexBits;
+    const bool lists = in.maxN > kFrontMax && pairListsFit(in, finalize);
     if (in.maxN <= kRegSortThreads) {
         launchFront<1>(in, lb, indexBits, s);
     } else if (in.maxN <= 2 * kRegSortThreads) {
@@ -481,7 +487,7 @@ bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, De
         PE_LAUNCHED();
         k_lbvh_bounds<<<g, kLbvhThreads, 0, s>>>(in, lb.box);
         PE_LAUNCHED();
-        k_lbvh_codes<<<g, kLbvhThreads, 0, s>>>(in, lb.box, lb.keys, indexBits);
+        k_lbvh_codes<<<g, kLbvhThreads, 0, s>>>(in, lb.box, lb.keys, indexBits, lists ? pb.count : nullptr);
         PE_LAUNCHED();
         // The index bits are already ascending (keys are laid out by index) and the
         // sort is stable, so sorting the 30 code bits orders the whole keys.
@@ -495,8 +501,13 @@ bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, De
         PE_LAUNCHED();
     }
     k_lbvh_pairs<<<lbvhWalkGrid(in.maxN), kLbvhWalkThreads, 0, s>>>(in.d_n, lb.keys, indexBits, lb.leafMn, lb.leafMx,
-                                                                    lb.rec, pb.keys, pb.cap, pb.bits, st);
+                                                                    lb.rec, pb.keys, pb.cap, pb.bits, lists ? pb.count : nullptr,
+                                                                    pb.flags, st);
     PE_LAUNCHED();
+    if (lists) {
+        launchPairsOrder(in, pb, st, ws, s);
+        return true;
+    }
     return launchPairsLists(in, finalize, pb, st, s);
 }
 

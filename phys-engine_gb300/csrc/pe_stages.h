@@ -72,6 +72,7 @@ struct PairBuffers {
     uint32_t *flags, *pos;
     uint32_t *a, *b;       // candidate pairs (collider slots), lexicographic
     uint32_t *counters;    // [4]
+    uint32_t *count, *first;  // [n] pairs of each first index, and where its list starts (order by lists)
 };
 
 struct SolverBuffers {
@@ -203,6 +204,7 @@ struct SapCoherence {
 // and the body / generation of each slot, for the pair finalize.
 struct PairMapping {
     const uint32_t *inSlot, *cbody, *cbgen;
+    bool identity;  // input i is the collider of body i: nothing to map or to filter
 };
 // Returns true when the sweep also finalized the pairs (one-block sweep with
 // `finalize` given and the raw pairs expected to fit it): the caller then
@@ -220,6 +222,11 @@ bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, De
 // one block by lists instead of a sort; false, launching nothing, when they may not
 // fit it.
 bool launchPairsLists(const BroadInput &in, const PairMapping &mapping, PairBuffers &pb, DevStats *st, cudaStream_t s);
+// The raw pairs' order by lists over the whole grid, for SAP and the tree where
+// there is nothing to map or to filter: the emitting kernel counts each first
+// index's pairs (count, cleared before) and notes each pair's rank among them (flags).
+bool pairListsFit(const BroadInput &in, const PairMapping &mapping);
+void launchPairsOrder(const BroadInput &in, PairBuffers &pb, DevStats *st, Scratch &ws, cudaStream_t s);
 // Grid pairs emitted body by body in lexicographic order, mapped to slots and
 // filtered (replaces the per-cell pairs and the finalize when pb.bodyPath).
 void launchGridBodyPairs(const BroadInput &in, const BroadBuffers &bb, PairBuffers &pb, const uint32_t *inSlot,

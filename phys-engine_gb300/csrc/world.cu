@@ -539,8 +539,10 @@ void World::ensureCapacity() {
     pairA_.reserve(pairCap_);
     pairB_.reserve(pairCap_);
     pairCounters_.reserve(4);
+    pairCount_.reserve(nc);
+    pairFirst_.reserve(nc);
     pb_ = PairBuffers{pairKeys_.ptr, pairKeysTmp_.ptr, pairCap_, 32u, false, false, pairFlags_.ptr, pairPos_.ptr,
-                      pairA_.ptr, pairB_.ptr, pairCounters_.ptr};
+                      pairA_.ptr, pairB_.ptr, pairCounters_.ptr, pairCount_.ptr, pairFirst_.ptr};
 
     if (mcap_ < pairCap_) mcap_ = pairCap_;
     const uint32_t m = mcap_;
@@ -792,7 +794,7 @@ void World::runPipeline(float dt) {
                       sap ? sapKeys_.ptr : nullptr, sapVals_.ptr, &st->inputCount, ws_, &st->err, s);
     }
     BroadInput in{dense_ ? aabbMin_.ptr : inMin_.ptr, dense_ ? aabbMax_.ptr : inMax_.ptr, &st->inputCount, nc_};
-    const PairMapping mapping{dense_ ? nullptr : inSlot_.ptr, cbody_.ptr, cbgen_.ptr};
+    const PairMapping mapping{dense_ ? nullptr : inSlot_.ptr, cbody_.ptr, cbgen_.ptr, dense_ && identityColliders_};
     bool finalized = false;
     if (sap) finalized = launchSap(in, sapKeys_.ptr, sapVals_.ptr, bb_, pb_, st, ws_, s, dense_ ? &coh : nullptr,
                                    &mapping);

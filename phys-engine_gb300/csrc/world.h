@@ -278,7 +278,7 @@ class World {
     void ensureLbvh();
     PairBuffers pb_{};
     DeviceArray<unsigned long long> pairKeys_, pairKeysTmp_;
-    DeviceArray<uint32_t> pairFlags_, pairPos_, pairA_, pairB_, pairCounters_;
+    DeviceArray<uint32_t> pairFlags_, pairPos_, pairA_, pairB_, pairCounters_, pairCount_, pairFirst_;
     uint32_t pairCap_ = 0;
     // manifolds
     uint32_t mcap_ = 0;

@@ -59,6 +59,32 @@ def test_tree_built_in_one_block(gpu, n, alike):
     assert_bit_equal(got[gpu.TREE], got[gpu.SAP], f"{n} {alike}")
 
 
+@pytest.mark.parametrize("algo", ["SAP", "TREE"])
+@pytest.mark.parametrize("touching", [0, 8, 9, 64, 65, 2048, 2049, 4300])
+def test_pair_order_by_lists(gpu, algo, touching):
+    """Lists sorted by a thread (up to 8 partners), a warp (64), a block (2,048)
+    and as a bitmap: a slab that touches so many spheres, first, in the middle
+    or last in index order, above 4,096 bodies in small groups."""
+    rng = np.random.default_rng(touching)
+    groups = 1470
+    cell = np.stack([np.arange(groups) % 40, np.arange(groups) // 40, np.zeros(groups)], 1) * 3.0
+    pos = np.repeat(cell, 3, 0) + rng.uniform(-0.3, 0.3, (3 * groups, 3))
+    near = np.argsort(pos[:, 0], kind="stable")[:touching]
+    pos[near, 2] -= 40.0  # into the slab below
+    for at in (0, len(pos) // 2, len(pos)):
+        slab = np.arange(len(pos) + 1) == at
+        sc = sphere_scene(np.insert(pos, at, [[58.0, 58.0, -40.0]], 0), np.full(len(slab), 0.4), slab)
+        sc.shape[slab] = 1
+        sc.dims[slab] = [140.0, 140.0, 0.2]
+        ref = gpu.GpuWorld(algo=gpu.GRID, iterations=1)
+        got = gpu.GpuWorld(algo=getattr(gpu, algo), iterations=1)
+        for w in (ref, got):
+            w.load_scene(sc)
+            w.step(1e-4)
+        assert np.count_nonzero(got.pairs() == at) >= touching
+        assert_bit_equal(got.pairs(), ref.pairs(), f"{algo} {touching} at {at}")
+
+
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 515])
 @pytest.mark.parametrize("offset", [0, 1, 3])
 def test_batch_poses_reach_any_array(gpu, n, offset):
