@@ -202,16 +202,23 @@ k_sap_emit(const uint32_t *d_n, const uint32_t *off, const uint32_t *len, const 
 // kErrSmallPath (the step is re-run with the separate finalize).
 constexpr uint32_t kSapBlockMax = 4096;
 constexpr uint32_t kSapBlockPairs = 8192;
-constexpr int kSapBlockThreads = (int)kRegSortThreads;
-// Shared memory: two sort buffers of kSapBlockMax u64 keys (the second also
-// holds the pair flags of the finalize), y/z bounds, min.x, max.x, entry
-// index, window offsets, then kSapBlockPairs u32 pair keys.
-constexpr size_t kSapBlockSmem = (size_t)kSapBlockMax * (8 + 8 + 16 + 4 + 4 + 4 + 4) + (size_t)kSapBlockPairs * 4;
-static_assert(kSapBlockPairs * 4 <= kSapBlockMax * 8, "pair flags fit one key buffer");
+// Variants by the number of boxes, T threads with E keys each: with 64 boxes a
+// barrier of 32 warps and a sort of 1,024 keys cost more than the sweep (10 boxes:
+// the broadphase 15.1 us with 1,024 threads, 9.8 with 128; 1,000 spheres 27.2 us with
+// room for 4,096 boxes and a thread adding the warps' sums in every scan, 24.2 now).
+constexpr uint32_t kSapSmallThreads = 128;
+// Shared memory for N boxes: two sort buffers of N u64 keys, y/z bounds, min.x, max.x,
+// entry index, window offsets, then the pairs' keys and the scratch of their order
+// (the second sort buffer where that is large enough).
+template <uint32_t N> constexpr bool kSapScratchInBuffer = N * 8 >= kSapBlockPairs * 4;
+template <uint32_t N> constexpr size_t sapBlockSmem() {
+    return (size_t)N * (8 + 8 + 16 + 4 + 4 + 4 + 4) + (size_t)kSapBlockPairs * (kSapScratchInBuffer<N> ? 4 : 8);
+}
 
 // Order of P <= kSapBlockPairs raw pairs without duplicates among n <= kSapBlockMax
 // boxes: sPairs holds first << bits | second, sCnt the pairs of each first index.
-// Scratch: sSec kSapBlockPairs words, sLong n, sBits kSapBlockMax bits a warp.
+// Scratch: sSec kSapBlockPairs words, sLong n, sBits max(N, 1024) bits a warp.
+template <uint32_t N>
 __device__ __forceinline__ void orderPairLists(uint32_t *sPairs, uint32_t *sCnt, uint32_t *sSec, uint32_t *sLong,
                                                uint32_t *sBits, uint32_t &count, uint32_t *s_scan, uint32_t n,
                                                uint32_t P, uint32_t bits, const uint32_t *inSlot,
@@ -248,7 +255,7 @@ __device__ __forceinline__ void orderPairLists(uint32_t *sPairs, uint32_t *sCnt,
     __syncthreads();
     {
         const uint32_t lane = tid & 31, warp = tid >> 5, nLong = count;
-        constexpr uint32_t kWords = kSapBlockMax / 32, kPerLane = kWords / 32;
+        constexpr uint32_t kWords = N < 1024 ? 32 : N / 32, kPerLane = kWords / 32;
         uint32_t *bm = sBits + warp * kWords;
         for (uint32_t q = warp; q < nLong; q += nt / 32) {
             const uint32_t f = sLong[q];
@@ -316,7 +323,7 @@ __device__ __forceinline__ void orderPairLists(uint32_t *sPairs, uint32_t *sCnt,
     if (tid == 0) st->pairs = total;
 }
 
-template <int E>
+template <uint32_t T, int E>
 __device__ __forceinline__ void sapSortKeys(const BroadInput &in, uint32_t n, unsigned long long *bufA,
                                             unsigned long long *bufB, uint32_t *sapKeys, uint32_t *sapVals,
                                             float *sMinX, float *sMaxX, float4 *sYZ, uint32_t *sIdx) {
@@ -327,7 +334,7 @@ __device__ __forceinline__ void sapSortKeys(const BroadInput &in, uint32_t n, un
         const uint32_t i = tid * E + r;
         v[r] = i < n ? ((unsigned long long)orderedFloatKey(in.mn[i].x) << 32 | i) : ~0ull;
     }
-    blockRegisterSort<unsigned long long, E>(v, bufA, bufB);
+    blockRegisterSort<unsigned long long, E, T>(v, bufA, bufB);
 #pragma unroll
     for (int r = 0; r < E; ++r) {
         const uint32_t i = tid * E + r;
@@ -343,29 +350,30 @@ __device__ __forceinline__ void sapSortKeys(const BroadInput &in, uint32_t n, un
     }
 }
 
-__global__ void __launch_bounds__(kSapBlockThreads)
+template <uint32_t T, int E>
+__global__ void __launch_bounds__(T)
 k_sap_block(BroadInput in, uint32_t *sapKeys, uint32_t *sapVals, uint32_t *unsorted, unsigned long long *keys,
             uint32_t cap, uint32_t bits, DevStats *st, int finalize, const uint32_t *inSlot, const uint32_t *cbody,
             const uint32_t *cbgen, uint32_t *pairA, uint32_t *pairB) {
+    constexpr uint32_t N = T * E;
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long *bufA = reinterpret_cast<unsigned long long *>(smem);
-    unsigned long long *bufB = bufA + kSapBlockMax;
-    float4 *sYZ = reinterpret_cast<float4 *>(bufB + kSapBlockMax);
-    float *sMinX = reinterpret_cast<float *>(sYZ + kSapBlockMax);
-    float *sMaxX = sMinX + kSapBlockMax;
-    uint32_t *sIdx = reinterpret_cast<uint32_t *>(sMaxX + kSapBlockMax);
-    uint32_t *sOff = sIdx + kSapBlockMax;  // window lengths, then their exclusive scan
-    uint32_t *sPairs = sOff + kSapBlockMax;
+    unsigned long long *bufB = bufA + N;
+    float4 *sYZ = reinterpret_cast<float4 *>(bufB + N);
+    float *sMinX = reinterpret_cast<float *>(sYZ + N);
+    float *sMaxX = sMinX + N;
+    uint32_t *sIdx = reinterpret_cast<uint32_t *>(sMaxX + N);
+    uint32_t *sOff = sIdx + N;  // window lengths, then their exclusive scan
+    uint32_t *sPairs = sOff + N;
+    uint32_t *sSec = kSapScratchInBuffer<N> ? reinterpret_cast<uint32_t *>(bufB) : sPairs + kSapBlockPairs;
     __shared__ uint32_t s_count, s_scan[40];
-    const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    const uint32_t n = min(*in.d_n, kSapBlockMax);  // the host launches this for at most kSapBlockMax boxes
+    const uint32_t tid = threadIdx.x, nt = T;
+    const uint32_t n = min(*in.d_n, N);  // the host launches this for at most N boxes
     if (tid == 0) {
         s_count = 0;
         if (unsorted) *unsorted = 0u;  // as after the multi-kernel sweep
     }
-    if (n <= kRegSortThreads) sapSortKeys<1>(in, n, bufA, bufB, sapKeys, sapVals, sMinX, sMaxX, sYZ, sIdx);
-    else if (n <= 2 * kRegSortThreads) sapSortKeys<2>(in, n, bufA, bufB, sapKeys, sapVals, sMinX, sMaxX, sYZ, sIdx);
-    else sapSortKeys<4>(in, n, bufA, bufB, sapKeys, sapVals, sMinX, sMaxX, sYZ, sIdx);
+    sapSortKeys<T, E>(in, n, bufA, bufB, sapKeys, sapVals, sMinX, sMaxX, sYZ, sIdx);
     __syncthreads();
     uint32_t *sCnt = reinterpret_cast<uint32_t *>(bufA);  // pairs per first index (finalize), n entries
     if (finalize)
@@ -436,8 +444,8 @@ k_sap_block(BroadInput in, uint32_t *sapKeys, uint32_t *sapVals, uint32_t *unsor
         if (tid == 0) atomicOr(&st->err, kErrSmallPath);
         return;
     }
-    orderPairLists(sPairs, sCnt, reinterpret_cast<uint32_t *>(bufB), sOff, reinterpret_cast<uint32_t *>(sYZ), s_count,
-                   s_scan, n, P, bits, inSlot, cbody, cbgen, pairA, pairB, st);
+    orderPairLists<N>(sPairs, sCnt, sSec, sOff, reinterpret_cast<uint32_t *>(sYZ), s_count, s_scan,
+                      n, P, bits, inSlot, cbody, cbgen, pairA, pairB, st);
 }
 
 // --------------------------------------------------------------- grid ------
@@ -1155,22 +1163,31 @@ bool sapFinalizesPairs(const BroadInput &in, const PairBuffers &pb) {
     return in.maxN <= kSapBlockMax && pb.blockPath && 2 * pb.bits <= 32;
 }
 
+template <uint32_t T, int E>
+static void launchSapBlock(const BroadInput &in, uint32_t *sapKeys, uint32_t *sapVals, PairBuffers &pb, DevStats *st,
+                           cudaStream_t s, const SapCoherence *coh, const PairMapping *finalize) {
+    constexpr size_t smem = sapBlockSmem<T * E>();
+    static bool configured = false;
+    if (!configured) {
+        PE_CHECK(cudaFuncSetAttribute(k_sap_block<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = true;
+    }
+    k_sap_block<T, E><<<1, T, smem, s>>>(
+        in, sapKeys, sapVals, coh ? coh->unsorted : nullptr, pb.keys, pb.cap, pb.bits, st, finalize ? 1 : 0,
+        finalize ? finalize->inSlot : nullptr, finalize ? finalize->cbody : nullptr,
+        finalize ? finalize->cbgen : nullptr, pb.a, pb.b);
+    PE_LAUNCHED();
+}
+
 bool launchSap(const BroadInput &in, uint32_t *sapKeys, uint32_t *sapVals, BroadBuffers &bb, PairBuffers &pb,
                DevStats *st, Scratch &ws, cudaStream_t s, const SapCoherence *coh, const PairMapping *finalize) {
     uint32_t *err = &st->err;
     if (in.maxN <= kSapBlockMax) {
-        static bool configured = false;
-        if (!configured) {
-            PE_CHECK(cudaFuncSetAttribute(k_sap_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)kSapBlockSmem));
-            configured = true;
-        }
         const bool fin = finalize && sapFinalizesPairs(in, pb);
-        k_sap_block<<<1, kSapBlockThreads, kSapBlockSmem, s>>>(
-            in, sapKeys, sapVals, coh ? coh->unsorted : nullptr, pb.keys, pb.cap, pb.bits, st, fin ? 1 : 0,
-            fin ? finalize->inSlot : nullptr, fin ? finalize->cbody : nullptr, fin ? finalize->cbgen : nullptr, pb.a,
-            pb.b);
-        PE_LAUNCHED();
+        if (in.maxN <= kSapSmallThreads) launchSapBlock<kSapSmallThreads, 1>(in, sapKeys, sapVals, pb, st, s, coh, fin ? finalize : nullptr);
+        else if (in.maxN <= kRegSortThreads) launchSapBlock<kRegSortThreads, 1>(in, sapKeys, sapVals, pb, st, s, coh, fin ? finalize : nullptr);
+        else if (in.maxN <= 2 * kRegSortThreads) launchSapBlock<kRegSortThreads, 2>(in, sapKeys, sapVals, pb, st, s, coh, fin ? finalize : nullptr);
+        else launchSapBlock<kRegSortThreads, 4>(in, sapKeys, sapVals, pb, st, s, coh, fin ? finalize : nullptr);
         return fin;
     }
     const bool lists = finalize && pairListsFit(in, *finalize);
@@ -1344,8 +1361,8 @@ k_pairs_lists(const unsigned long long *keys, uint32_t cap, const uint32_t *d_n,
         atomicAdd(&sCnt[first], 1u);
     }
     __syncthreads();
-    orderPairLists(sPairs, sCnt, sSec, sLong, sBits, s_count, s_scan, n, P, bits, inSlot, cbody, cbgen, pairA, pairB,
-                   st);
+    orderPairLists<kSapBlockMax>(sPairs, sCnt, sSec, sLong, sBits, s_count, s_scan, n, P, bits, inSlot, cbody, cbgen,
+                                 pairA, pairB, st);
 }
 
 bool launchPairsLists(const BroadInput &in, const PairMapping &mapping, PairBuffers &pb, DevStats *st, cudaStream_t s) {

@@ -142,16 +142,17 @@ template <class K> __device__ __forceinline__ K *blockMergeSort(K *a, K *b, uint
     return src;
 }
 
-// Bitonic sort of N = kRegSortThreads * E keys held in registers, ascending;
+// Bitonic sort of N = T * E keys held in registers, ascending;
 // thread t holds positions [t E, t E + E) before and after.  Compare-exchange
 // stages whose partner is in the same thread run in registers, those whose
 // partner is in the same warp through shuffles, and only the stages with
 // partners in other warps (j >= 32 E) through shared memory: bufA and bufB
 // (N keys each) are used in turn, so one barrier per such stage suffices.
-// All kRegSortThreads threads of the block call it (blockDim.x must be that).
+// All T threads of the block call it (blockDim.x must be T).
 constexpr uint32_t kRegSortThreads = 1024;
-template <class K, int E> __device__ __forceinline__ void blockRegisterSort(K (&v)[E], K *bufA, K *bufB) {
-    constexpr uint32_t N = kRegSortThreads * E;
+template <class K, int E, uint32_t T = kRegSortThreads>
+__device__ __forceinline__ void blockRegisterSort(K (&v)[E], K *bufA, K *bufB) {
+    constexpr uint32_t N = T * E;
     const uint32_t t = threadIdx.x;
     bool useA = true;
 #pragma unroll
@@ -217,14 +218,16 @@ __device__ __forceinline__ uint32_t blockExclusiveScanArray(uint32_t *s, uint32_
     }
     if (lane == 31) scratch[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (int w = 0; w < warps; ++w) {
-            uint32_t t = scratch[w];
-            scratch[w] = acc;
-            acc += t;
+    // (at most 32 warps: one scans the warps' sums)
+    if (warp == 0) {
+        const uint32_t x = lane < warps ? scratch[lane] : 0u;
+        uint32_t xi = x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, xi, o);
+            if (lane >= o) xi += t;
         }
-        scratch[warps] = acc;
+        if (lane < warps) scratch[lane] = xi - x;
+        if (lane == warps - 1) scratch[warps] = xi;
     }
     __syncthreads();
     uint32_t run = scratch[warp] + incl - sum;
