@@ -279,3 +279,22 @@ def test_narrowphase_matches_the_oracle_for_any_number_of_pairs(gpu, pairs):
         assert step > 0 or len(gw.pairs()) == pairs
         assert_bit_equal(gw.pairs(), ow.pairs(), f"{pairs} step {step} pairs")
         assert_manifolds_equal(gw.contacts(), ow.contacts(), what=f"{pairs} step {step}")
+
+
+@pytest.mark.parametrize("n", [40, 128, 129, 1000, 1025, 2049])
+def test_piles_on_one_rank_and_over_the_cluster(gpu, n):
+    """Spheres heaped on a floor: manifolds that fit one block's shared memory
+    (up to a few hundred points) and more; bodies at the edges of the one-block
+    sweep's variants (128, 1,024 and 2,048 with the floor)."""
+    sc = scenes.generate(scenes.SPHERES_ON_FLOOR, n - 1, n)
+    gw = gpu.GpuWorld(algo=gpu.SAP, iterations=6, order=gpu.ORDER_COLOR)
+    ow = cpu.OracleWorld(algo=0, iterations=6, order_mode=1)
+    for w in (gw, ow):
+        w.load_scene(sc)
+    for step in range(60):
+        gw.step(1 / 60)
+        ow.step(1 / 60)
+    assert_bit_equal(gw.pairs(), ow.pairs(), f"{n} pairs")
+    assert_manifolds_equal(gw.contacts(), ow.contacts(), what=f"{n}")
+    for k in ("pos", "quat", "lin", "ang"):
+        assert_bit_equal(gw.bodies()[k], ow.bodies()[k], f"{n} {k}")
