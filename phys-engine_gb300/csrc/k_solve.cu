@@ -451,7 +451,6 @@ __global__ void k_cache_write(SolveArgs a, CacheView nc, uint32_t cacheCap) {
 
 
 // Velocity staging slots of the single-block solver (bodies touched by contacts).
-constexpr uint32_t kStageSlots = 3072;
 constexpr size_t blockSolveSmem(uint32_t blockM, uint32_t stageSlots) {
     return (size_t)blockM * (8 + 4 + 8) + (size_t)stageSlots * (32 + 4);
 }
@@ -542,7 +541,7 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
             bm = 64;
             while (bm < blockM) bm <<= 1;
         }
-        uint32_t slots = 2 * bm < kStageSlots ? 2 * bm : kStageSlots;
+        uint32_t slots = blockStageSlots(bm);
         if (orderMode != 0 && launchSolverCluster(a, newCache, newCacheCount, cacheCap, bm, slots, s)) return;
         const size_t smem = blockSolveSmem(bm, slots);
         k_prepare<<<(4 * bm + kPrepareThreads - 1) / kPrepareThreads, kPrepareThreads,

@@ -713,12 +713,6 @@ __global__ void __launch_bounds__(kIslPrepThreads) k_prepare_islands(SolveArgs a
 // memory, not a cluster barrier and loads from another SM's (1,000 spheres on a floor,
 // 616 manifolds in four colours, 10 iterations: the sweeps with their staging 64 -> 45
 // us, the step 131 -> 118).
-__device__ __forceinline__ uint32_t oneRankOffset(const ClusterSolveLayout &lay) {
-    return (lay.blockM * 20u + lay.stageSlots * 36u + 15u) & ~15u;
-}
-__device__ __forceinline__ uint32_t oneRankBytes(const ClusterSolveLayout &lay, uint32_t M, uint32_t points) {
-    return oneRankOffset(lay) + 32u * M + 176u * points;
-}
 struct SplitVel {
     float4 *l, *w;      // linear and angular velocities by slot (apart: fewer bank conflicts)
     const uint2 *slot;  // per solve index: slots of body A and body B
@@ -737,7 +731,7 @@ __device__ __forceinline__ void solveOnOneRank(const SolveArgs &a, uint32_t M, c
     const uint32_t tid = threadIdx.x, nt = blockDim.x, P = cs.points, S = cs.solve.slots, C = cs.solve.colors;
     uint32_t *s_off = reinterpret_cast<uint32_t *>(smem), *s_cnt = s_off + lay.blockM;
     uint32_t *s_dyn = reinterpret_cast<uint32_t *>(smem + (size_t)lay.blockM * 8);  // manifold of a solve index
-    float4 *spm = reinterpret_cast<float4 *>(smem + oneRankOffset(lay)), *spn = spm + M, *spt = spn + M;
+    float4 *spm = reinterpret_cast<float4 *>(smem + clusterOneRankOffset(lay.blockM, lay.stageSlots)), *spn = spm + M, *spt = spn + M;
     for (uint32_t k = tid; k < M; k += nt) {
         const uint32_t m = s_dyn[k], o = s_off[k], n = s_cnt[k];
         spm[k] = __ldcg(&sb.pm[m]);
@@ -892,7 +886,7 @@ k_solve_cluster(SolveArgs a, CacheView nc, uint32_t cacheCap, uint32_t *newCount
             for (uint32_t k = tid; k < M; k += nt) s_off[k] = s_cnt[k] = min(__ldcg(&sb.pcount[s_dyn[k]]), 4u);
             __syncthreads();
             const uint32_t points = blockExclusiveScanArray(s_off, M, cs.solve.scan);
-            if (oneRankBytes(lay, M, points) <= kClusterSmemMax) path = kPathOneRank;
+            if (clusterFitsOneRank(lay.blockM, lay.stageSlots, M, points)) path = kPathOneRank;
             if (tid == 0) cs.points = points;
         }
         if (path == kPathCluster) {

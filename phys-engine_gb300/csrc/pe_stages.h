@@ -252,6 +252,19 @@ constexpr uint32_t kBlockMaxManifolds = 4096;
 constexpr uint32_t kIslandMax = 16;
 constexpr uint32_t kClusterRanks = 8;
 constexpr uint32_t kClusterSmemMax = 224 * 1024;
+// Bodies whose velocities the one-block and cluster solvers stage for blockM manifolds.
+constexpr uint32_t kStageSlots = 3072;
+__host__ __device__ inline uint32_t blockStageSlots(uint32_t blockM) {
+    return 2 * blockM < kStageSlots ? 2 * blockM : kStageSlots;
+}
+// Rank 0's shared memory with M manifolds and their points next to the arrays of its
+// front (blockM manifolds, stageSlots bodies): it sweeps alone where they fit.
+__host__ __device__ inline uint32_t clusterOneRankOffset(uint32_t blockM, uint32_t stageSlots) {
+    return (blockM * 20u + stageSlots * 36u + 15u) & ~15u;
+}
+__host__ __device__ inline bool clusterFitsOneRank(uint32_t blockM, uint32_t stageSlots, uint32_t M, uint32_t points) {
+    return clusterOneRankOffset(blockM, stageSlots) + 32u * M + 176u * points <= kClusterSmemMax;
+}
 struct ClusterSolveLayout {
     uint32_t blockM, stageSlots;   // capacities of the single-block front (rank 0)
     uint32_t localCap, pointCap;   // manifolds / prepared points held per rank

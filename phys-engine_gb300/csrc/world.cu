@@ -952,11 +952,13 @@ bool World::finishStep() {
 //  * The one-cluster solver sweeps islands of up to 16 manifolds alone and is
 //    the best path for them; a pile (it refused its islands) goes colour by
 //    colour there, 2 to 5 us a phase, against a fixed cost about 60 us higher in
-//    the whole-grid sweeps and 1 to 2.5 us a phase.  Measured, us a step: piles
-//    of 10, 36 and 210 boxes in pyramids 238 -> 195, 300 -> 230, 640 -> 508;
-//    fields of 60, 400, 1,501 and 2,000 bodies 182 -> 156, 240 -> 203, 384 ->
-//    274, 926 -> 295.  Spheres on a floor (one point a manifold, three to five
-//    colours) stay: 1,309 manifolds 225 -> 223, fewer lose.
+//    the whole-grid sweeps and 1 to 2.5 us a phase.  Measured, us a step:
+//    pyramids of 210 boxes 629 -> 472; fields of 400, 700, 1,000 and 1,501 bodies
+//    229 -> 175, 269 -> 190, 302 -> 202, 371 -> 224.  Spheres on a floor (one point
+//    a manifold, three to five colours) stay: 1,309 manifolds 225 -> 223, fewer lose.
+//  * What fits one rank of the cluster is swept there, one block barrier a phase:
+//    fields of 60, 100 and 200 bodies 122, 131, 152 (whole grid 137, 153, 170),
+//    pyramids of 10, 21 and 36 boxes 143, 161, 181 (169, 190, 211).
 //  * Above the cluster's size the island sweeps pay where most manifolds lie in
 //    islands of fewer than eight (65,536 boxes in stacks of two: 430 against 500
 //    in the whole-grid sweeps), the whole-grid sweeps elsewhere (fields of 5,000
@@ -969,7 +971,12 @@ void World::chooseSweeps(const DevStats &h) {
     }
     if (orderMode == 0 || solveSkipped_ || !identityColliders_) return;
     bool want = sweepAll_;
-    if (sweepAll_) {
+    // the cluster solver's capacity for so many manifolds
+    uint32_t blockM = 64;
+    while (blockM < h.manifolds + h.manifolds / 4 + 64 && blockM < kBlockMaxManifolds) blockM <<= 1;
+    if (clusterFitsOneRank(blockM, blockStageSlots(blockM), h.manifolds, h.points)) {
+        want = false;
+    } else if (sweepAll_) {
         want = h.manifolds >= kSweepMin && 4ull * h.loose <= 3ull * h.manifolds;
     } else if (!wideColors_ && h.manifolds >= 2 * kSweepMin) {
         if (blockSolver_) {
