@@ -298,3 +298,25 @@ def test_piles_on_one_rank_and_over_the_cluster(gpu, n):
     assert_manifolds_equal(gw.contacts(), ow.contacts(), what=f"{n}")
     for k in ("pos", "quat", "lin", "ang"):
         assert_bit_equal(gw.bodies()[k], ow.bodies()[k], f"{n} {k}")
+
+
+@pytest.mark.parametrize("n", [4097, 6143, 6144, 6145, 12289, 32767, 32768, 32769])
+@pytest.mark.parametrize("rows", [False, True])
+def test_sweep_order_of_tiles(gpu, n, rows):
+    """Tiles of 2,048 sorted keys and their remainders, the last size placed by
+    lookups and the first that is sorted in passes; rows: few different min.x,
+    so that the index decides the order."""
+    rng = np.random.default_rng(n)
+    side = 1.1 * n ** (1 / 3)
+    pos = rng.uniform(-side / 2, side / 2, (n, 3))
+    if rows:
+        pos[:, 0] = np.round(pos[:, 0])
+    sc = sphere_scene(pos, np.full(n, 0.3), np.zeros(n))
+    got = {}
+    for algo in (gpu.SAP, gpu.GRID):
+        w = gpu.GpuWorld(algo=algo, iterations=1)
+        w.load_scene(sc)
+        for _ in range(2):
+            w.step(1e-3)
+        got[algo] = w.pairs()
+    assert_bit_equal(got[gpu.SAP], got[gpu.GRID], f"{n} {rows}")
