@@ -58,9 +58,10 @@ __global__ void __launch_bounds__(kSolveThreads) k_color(SolveArgs a) {
     }
     for (uint32_t m = gtid; m < M; m += gstride) {
         uint32_t ba = a.mv.bodyA[m], bb = a.mv.bodyB[m];
-        bool da = ba < w.nb && w.bgen[ba] == a.mv.genA[m] && bodyMoves(w.bflags[ba]);
-        bool db = bb < w.nb && w.bgen[bb] == a.mv.genB[m] && bodyMoves(w.bflags[bb]);
-        sb.dyn[m] = (da ? 1u : 0u) | (db ? 2u : 0u);
+        // (the prepare kernel, which may run at the same time, writes the same flags)
+        const uint32_t fl = manifoldFlagsOf(w, ba, bb, a.mv.genA[m], a.mv.genB[m]);
+        const bool da = fl & kFlagDynA, db = fl & kFlagDynB;
+        sb.dyn[m] = fl;
         sb.color[m] = kUncolored;
         if (da) {
             __stcg(&sb.bodyUsed[2 * ba], 0ull);
@@ -520,7 +521,7 @@ int maxCooperativeBlocks(int smCount) {
 void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &oldCache, const uint32_t *oldCacheCount,
                   const CacheView &newCache, uint32_t *newCacheCount, uint32_t cacheCap, SolverBuffers &sb,
                   int iterations, int orderMode, int coopBlocks, bool blockPath, uint32_t blockM, bool sweepAll,
-                  bool pairOrderCache, DevStats *st, Scratch &ws, cudaStream_t s) {
+                  bool pairOrderCache, DevStats *st, Scratch &ws, cudaStream_t s, const SolveFork *fork) {
     SolveArgs a{w, mv, sb, oldCache, oldCacheCount, st, sb.mcap, iterations, pairOrderCache,
                 w.sleepMode ? &st->solveCount : &st->manifolds};
     if (w.sleepMode) {
@@ -555,20 +556,39 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
     PE_CHECK(cudaMemsetAsync(sb.counters, 0, 4 * sizeof(uint32_t), s));
     PE_CHECK(cudaMemsetAsync(sb.bar, 0, 2 * sizeof(uint32_t), s));
     const bool serial = orderMode == 0;
-    if (!serial) {
-        configureColor();
-        launchCooperative((const void *)k_color, coopBlocks, a, s, kColorSmem);
-    }
-    if (sweepAll && !serial && pairOrderCache) {
-        k_prepare<<<gridFor(mcap, kPrepareThreads), kPrepareThreads, kPrepareKeyCap * sizeof(unsigned long long), s>>>(
-            a, kPrepareKeyCap);
+    const bool sweep = sweepAll && !serial && pairOrderCache;
+    // The prepare kernel and the cache's offsets need nothing of the colouring, which
+    // waits for its own chains (33 us for 17,000 manifolds) on a block an SM: beside
+    // it, on the fork's stream, they cost no time of their own.  Measured, us a step:
+    // fields of 1,501 and 10,000 bodies 242 -> 233, 303 -> 296; the others as before.
+    auto prepare = [&](cudaStream_t ps) {
+        k_prepare<<<gridFor(mcap, kPrepareThreads), kPrepareThreads, kPrepareKeyCap * sizeof(unsigned long long),
+                    ps>>>(a, kPrepareKeyCap);
         PE_LAUNCHED();
+        if (!sweep) return;
         const uint32_t tiles = mcap / kScanThreads + 1;
-        PE_CHECK(cudaMemsetAsync(ws.scanState, 0, sizeof(unsigned long long) * (tiles + 1), s));
+        PE_CHECK(cudaMemsetAsync(ws.scanState, 0, sizeof(unsigned long long) * (tiles + 1), ps));
         const uint32_t grid = std::min<uint32_t>(tiles, 2u * (uint32_t)smCount());
-        k_cache_offsets<<<grid, kScanThreads, 0, s>>>(a, ws.scanState, (uint32_t *)(ws.scanState + tiles),
-                                                      newCacheCount);
+        k_cache_offsets<<<grid, kScanThreads, 0, ps>>>(a, ws.scanState, (uint32_t *)(ws.scanState + tiles),
+                                                       newCacheCount);
         PE_LAUNCHED();
+    };
+    if (serial) {
+        prepare(s);
+    } else {
+        configureColor();
+        if (fork) {
+            PE_CHECK(cudaEventRecord(fork->begin, s));
+            PE_CHECK(cudaStreamWaitEvent(fork->side, fork->begin, 0));
+        }
+        launchCooperative((const void *)k_color, coopBlocks, a, s, kColorSmem);
+        prepare(fork ? fork->side : s);
+        if (fork) {
+            PE_CHECK(cudaEventRecord(fork->end, fork->side));
+            PE_CHECK(cudaStreamWaitEvent(s, fork->end, 0));
+        }
+    }
+    if (sweep) {
         launchSolveSweep(a, newCache, cacheCap, s);
         return;
     }
@@ -583,9 +603,6 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
             launchRadixSort<uint32_t>(sb.orderKeys, sb.orderKeysTmp, sb.order, sb.orderTmp, a.count, mcap, 0, 32,
                                       ws, err, s);
     }
-    k_prepare<<<gridFor(mcap, kPrepareThreads), kPrepareThreads, kPrepareKeyCap * sizeof(unsigned long long), s>>>(
-        a, kPrepareKeyCap);
-    PE_LAUNCHED();
     if (serial) {
         k_solve_serial<<<1, 32, 0, s>>>(a);
         PE_LAUNCHED();

@@ -236,10 +236,15 @@ void launchPairsFinalize(const uint32_t *inSlot, const uint32_t *cbody, const ui
                          DevStats *st, Scratch &ws, cudaStream_t s);
 void launchNarrowphase(const WorldView &w, const PairBuffers &pb, const ManifoldView &mv, uint32_t mcap, DevStats *st,
                        Scratch &ws, cudaStream_t s, unsigned long long *state = nullptr, bool stateCleared = false);
+// A second stream for work beside the colouring, with events of its own.
+struct SolveFork {
+    cudaStream_t side;
+    cudaEvent_t begin, end;
+};
 void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &oldCache, const uint32_t *oldCacheCount,
                   const CacheView &newCache, uint32_t *newCacheCount, uint32_t cacheCap, SolverBuffers &sb,
                   int iterations, int orderMode, int coopBlocks, bool blockPath, uint32_t blockM, bool sweepAll,
-                  bool pairOrderCache, DevStats *st, Scratch &ws, cudaStream_t s);
+                  bool pairOrderCache, DevStats *st, Scratch &ws, cudaStream_t s, const SolveFork *fork = nullptr);
 // Largest manifold count the single-block solver handles, and the largest
 // body index it can key (bodies < 2^20).
 constexpr uint32_t kBlockMaxManifolds = 4096;

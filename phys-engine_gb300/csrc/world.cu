@@ -33,6 +33,9 @@ World::World(int device) : device_(device) {
     PE_CHECK(cudaSetDevice(device_));
     PE_CHECK(cudaDeviceGetAttribute(&smCount_, cudaDevAttrMultiProcessorCount, device_));
     PE_CHECK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    PE_CHECK(cudaStreamCreateWithFlags(&fork_.side, cudaStreamNonBlocking));
+    PE_CHECK(cudaEventCreateWithFlags(&fork_.begin, cudaEventDisableTiming));
+    PE_CHECK(cudaEventCreateWithFlags(&fork_.end, cudaEventDisableTiming));
     PE_CHECK(cudaMallocHost(&hostStats_, sizeof(DevStats)));
     std::memset(hostStats_, 0, sizeof(DevStats));
     PE_CHECK(cudaHostAlloc(reinterpret_cast<void **>(&ioHost_), sizeof(StepIo), cudaHostAllocMapped));
@@ -50,6 +53,9 @@ World::~World() {
     if (hostStats_) cudaFreeHost(hostStats_);
     if (ioHost_) cudaFreeHost(ioHost_);
     if (pinned_) cudaFreeHost(pinned_);
+    if (fork_.begin) cudaEventDestroy(fork_.begin);
+    if (fork_.end) cudaEventDestroy(fork_.end);
+    if (fork_.side) cudaStreamDestroy(fork_.side);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -814,7 +820,7 @@ void World::runPipeline(float dt) {
     const CacheView tmp{tKey_.ptr, tGens_.ptr, tA_.ptr, tB_.ptr, tT2_.ptr};
     launchSolver(w, mv, cacheView(cache_), &cCount_.ptr[cache_], sleeping ? tmp : cacheView(1 - cache_),
                  sleeping ? tCount_.ptr : &cCount_.ptr[1 - cache_], cacheCap_, sb_, iterations, orderMode, coopBlocks_,
-                 blockSolver_, blockM_, sweepAll_, identityColliders_, st, ws_, s);
+                 blockSolver_, blockM_, sweepAll_, identityColliders_, st, ws_, s, &fork_);
     if (sleeping)
         launchCacheCarry(w, cacheView(cache_), &cCount_.ptr[cache_], tmp, tCount_.ptr, cacheView(1 - cache_),
                          &cCount_.ptr[1 - cache_], cacheCap_, carry_.ptr, carryPos_.ptr, carryTotal_.ptr, st, ws_, s);

@@ -202,6 +202,7 @@ class World {
     int device_;
     int smCount_ = 0;
     cudaStream_t stream_ = nullptr;
+    SolveFork fork_{};  // beside stream_ within a step
     bool hostDirty_ = true;
     bool deviceNewer_ = false;
     bool dense_ = true;
