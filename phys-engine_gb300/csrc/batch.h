@@ -61,8 +61,11 @@ struct BatchVariant {
 };
 constexpr BatchVariant kBatchVariants[] = {{128, 1}, {128, 4}, {256, 1}, {256, 2}, {512, 1}};
 constexpr int kBatchVariantCount = 5;
+// Worlds of up to this many bodies are coloured and swept on words and velocities in
+// shared memory (16 KB, after the solver's manifold arrays).
+constexpr uint32_t kBatchStageBodies = 512;
 // Dynamic shared memory of a launch: SAP keys of the largest world or the
-// solver's manifold arrays, whichever is larger.
+// solver's arrays, whichever is larger.
 size_t batchSharedBytes(uint32_t maxN, uint32_t maxM);
 // Resident blocks over the whole GPU for a variant (also sets its shared-memory limit).
 uint32_t batchMaxBlocks(int variant, size_t smem);

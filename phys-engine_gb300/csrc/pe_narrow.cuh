@@ -513,8 +513,10 @@ __device__ inline SupportShape supportShape(const WorldView &w, uint32_t c, cons
 // collider slots ca, cb of bodies ba, bb: world transforms, shape dispatch with
 // the box-sphere swap (narrowphase.cpp:353-365), anchors to body space,
 // restitution = max, friction = sqrt(max(fa,0) * max(fb,0)).  category: 0
-// sphere-sphere, 1 sphere-box, 2 box-box, 3 hull.
-__device__ inline bool narrowphasePair(const WorldView &w, uint32_t ca, uint32_t cb, uint32_t ba, uint32_t bb,
+// sphere-sphere, 1 sphere-box, 2 box-box, 3 hull.  HULLS: some collider may be one
+// (the polytopes' storage takes 9 KB of a thread's stack).
+template <bool HULLS = true>
+__device__ __forceinline__ bool narrowphasePair(const WorldView &w, uint32_t ca, uint32_t cb, uint32_t ba, uint32_t bb,
                                        LocalManifold &lm, float &restitution, float &friction, uint32_t &category,
                                        bool &epaFailed) {
     epaFailed = false;
@@ -530,7 +532,7 @@ __device__ inline bool narrowphasePair(const WorldView &w, uint32_t ca, uint32_t
     Tf tB{pb + rotate(qb, lpb), qmul(qb, lqb)};
     const float4 sha = w.cshape[ca], shb = w.cshape[cb];
     bool hit;
-    if (sa == kShapeHull || sb == kShapeHull) {
+    if (HULLS && (sa == kShapeHull || sb == kShapeHull)) {
         category = 3;
         hit = hullContact(supportShape(w, ca, tA), supportShape(w, cb, tB), lm, epaFailed);
     } else {

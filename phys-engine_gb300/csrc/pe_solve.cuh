@@ -126,13 +126,14 @@ __device__ __forceinline__ bool solvedPair(const WorldView &w, uint32_t flA, uin
 // anchors and impulse are in bounds for any p < 4), before the item is known
 // to be live.
 struct PrepItem {
-    uint32_t m, p, npts, ia, ib, gA, gB;
+    uint32_t k, p, npts,  // k: where the manifold's data go
+        ia, ib, gA, gB;
     float4 nf, aa, ab, imp;
     float rest;
 };
 __device__ __forceinline__ PrepItem loadPrepItemAt(const SolveArgs &a, uint32_t m, uint32_t p) {
     PrepItem t;
-    t.m = m;
+    t.k = m;
     t.p = p;
     t.npts = a.mv.pointCount[m];
     t.ia = a.mv.bodyA[m];
@@ -222,7 +223,7 @@ __device__ __forceinline__ void prepareItem(const SolveArgs &a, const PrepItem &
                                             const uint2 *range = nullptr) {
     const uint32_t mcap = a.mcap;
     const WorldView &w = a.w;
-    const uint32_t m = t.m, p = t.p, k = m;  // k: data index
+    const uint32_t p = t.p, k = t.k;
     const uint32_t live = t.npts < 4u ? t.npts : 4u;  // live points (at most four)
     if (p > 0 && p >= live) return;
     const uint32_t ia = t.ia, ib = t.ib;
@@ -366,12 +367,25 @@ __device__ __forceinline__ void prepareItem(const SolveArgs &a, const PrepItem &
     a.sb.pimp[(size_t)p * mcap + k] = imp;
 }
 
+// order (nullable): the manifold of each solve index; the data then go to the solve
+// index, so that the manifolds of a colour, which neighbouring threads sweep, lie side
+// by side.
 __device__ inline void prepareRange(const SolveArgs &a, uint32_t begin, uint32_t stride, uint32_t M,
-                                    const unsigned long long *cacheKeys = nullptr) {
+                                    const unsigned long long *cacheKeys = nullptr, const uint32_t *order = nullptr) {
     if (!cacheKeys) cacheKeys = a.oldCache.key;
     const uint32_t cacheN = *a.oldCount;
     PrepTally tally;
-    for (uint32_t q = begin; q < 4 * M; q += stride) prepareItem(a, loadPrepItem(a, q, M), cacheKeys, cacheN, tally);
+    for (uint32_t q = begin; q < 4 * M; q += stride) {
+        PrepItem t;
+        if (order) {
+            const uint32_t p = q / M, k = q - p * M;
+            t = loadPrepItemAt(a, order[k], p);
+            t.k = k;
+        } else {
+            t = loadPrepItem(a, q, M);
+        }
+        prepareItem(a, t, cacheKeys, cacheN, tally);
+    }
     flushPrepTally(a, tally);
 }
 
@@ -673,10 +687,12 @@ __device__ __forceinline__ uint32_t manifoldFlags(const SolveArgs &a, uint32_t m
 // colour ranges and, when it returns true, vs->slot[k] the staging slots of
 // solve index k's bodies and vs->slotBody / sh.slots the staged bodies.
 // mflags: manifoldFlags of every manifold, written by an earlier launch or
-// cluster rank (nullptr: computed here).
+// cluster rank (nullptr: computed here).  bodyArea (nullable): room in shared memory for
+// three words for each of the world's w.nb bodies, indexed by body (in place of vs).
 __device__ inline bool solveBlockFront(const SolveArgs &a, uint32_t M, int serial, uint32_t maxM,
                                        unsigned long long *s_sort, uint32_t *s_dyn, BlockSolveShared &sh,
-                                       const VelStage *vs, const uint32_t *mflags = nullptr) {
+                                       const VelStage *vs, const uint32_t *mflags = nullptr,
+                                       unsigned long long *bodyArea = nullptr) {
     uint32_t *s_start = sh.start, *s_count = sh.count, *s_scan = sh.scan;
     uint32_t &s_colored = sh.colored, &s_colors = sh.colors;
     const WorldView &w = a.w;
@@ -765,14 +781,19 @@ __device__ inline bool solveBlockFront(const SolveArgs &a, uint32_t M, int seria
         if (slotted) {
             cBest = reinterpret_cast<unsigned long long *>(vs->v);
             cUsed = cBest + vs->cap;
+        } else if (bodyArea) {
+            cBest = bodyArea;
+            cUsed = bodyArea + w.nb;
+            for (uint32_t i = tid; i < 3 * w.nb; i += nt) bodyArea[i] = 0ull;
         }
+        const bool inShared = slotted || bodyArea;
         auto cid = [&](uint32_t m, int side) -> uint32_t {
             return slotted ? (side ? vs->slot[m].y : vs->slot[m].x) : (side ? a.mv.bodyB[m] : a.mv.bodyA[m]);
         };
         // Atomics resolve in L2; global reads go past L1 so no stale line is seen.
-        auto ldc = [&](const unsigned long long *p) { return slotted ? *p : __ldcg(p); };
+        auto ldc = [&](const unsigned long long *p) { return inShared ? *p : __ldcg(p); };
         auto stc = [&](unsigned long long *p, unsigned long long v) {
-            if (slotted) *p = v;
+            if (inShared) *p = v;
             else __stcg(p, v);
         };
         uint32_t *s_color = reinterpret_cast<uint32_t *>(s_sort);  // reused before the order sort
@@ -780,7 +801,7 @@ __device__ inline bool solveBlockFront(const SolveArgs &a, uint32_t M, int seria
             const uint32_t fl = s_dyn[m];
             const bool da = fl & kFlagDynA, db = fl & kFlagDynB;
             s_color[m] = kUncolored;
-            if (!slotted) {
+            if (!inShared) {
                 const uint32_t ba = a.mv.bodyA[m], bb = a.mv.bodyB[m];
                 if (da) {
                     __stcg(&sb.bodyUsed[2 * ba], 0ull);

@@ -320,3 +320,32 @@ def test_sweep_order_of_tiles(gpu, n, rows):
             w.step(1e-3)
         got[algo] = w.pairs()
     assert_bit_equal(got[gpu.SAP], got[gpu.GRID], f"{n} {rows}")
+
+
+@pytest.mark.parametrize("n", [63, 64, 511, 512, 513])
+def test_batched_worlds_equal_single_ones_on_either_memory(gpu, n):
+    """Worlds of up to 512 bodies are coloured and swept in shared memory, larger
+    ones in global memory; beside each a slab on 150 fixed spheres (150 colours:
+    two colour windows, more than the shared colour ranges hold)."""
+    grid = np.stack(np.meshgrid(np.arange(15), np.arange(10)), -1).reshape(-1, 2) * 0.75
+    pos = np.concatenate([np.stack([grid[:, 0], np.zeros(150), grid[:, 1]], 1), [[5.25, 0.54, 3.4]]])
+    slab = sphere_scene(pos, np.full(151, 0.3), np.arange(151) < 150)
+    slab.shape[150] = 1
+    slab.dims[150] = [12.0, 0.5, 8.0]
+    sc = [scenes.mixed_field(n - 1, n), slab]
+    batch = gpu.GpuBatch(sc, iterations=6)
+    worlds = []
+    for x in sc:
+        w = gpu.GpuWorld(algo=gpu.SAP, iterations=6, order=gpu.ORDER_COLOR)
+        w.load_scene(x)
+        worlds.append(w)
+    for _ in range(100):
+        batch.step(1 / 120)
+        for w in worlds:
+            w.step(1 / 120)
+    assert batch.stats(0)["contact_count"] > 0 and batch.stats(1)["color_count"] > 128
+    for k, w in enumerate(worlds):
+        got, want = batch.world_bodies(k), w.bodies()
+        for g, key in zip(got, ("pos", "quat", "lin", "ang")):
+            assert_bit_equal(g, want[key], f"{n} world {k} {key}")
+        assert_manifolds_equal(batch.contacts(k), w.contacts(), what=f"{n} world {k}")
