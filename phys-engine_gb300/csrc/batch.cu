@@ -47,11 +47,14 @@ constexpr uint32_t kBatchMaxWorldBodies = 8192;
 
 Batch::Batch(int device) : device_(device) {
     PE_CHECK(cudaSetDevice(device_));
+    int least = 0, greatest = 0;
+    PE_CHECK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     PE_CHECK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     for (int i = 0; i < 3; ++i) {
         cudaStream_t s;
         cudaEvent_t e;
-        PE_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        // (the first takes the largest worlds)
+        PE_CHECK(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, std::min(least, greatest + (int)side_.size())));
         PE_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         side_.push_back(s);
         joins_.push_back(e);
@@ -364,13 +367,16 @@ BatchView Batch::view(const BatchBucket &bk, float dt, uint32_t parity) const {
 void Batch::launchAll(float dt, uint32_t parity) {
     PE_CHECK(cudaMemsetAsync(queueHead_.ptr, 0, buckets_.size() * sizeof(uint32_t), stream_));
     PE_CHECK(cudaMemsetAsync(batchErr_.ptr, 0, sizeof(uint32_t), stream_));
+    // The buckets' kernels run side by side, the largest worlds first (order and
+    // stream priority): a bucket's last worlds leave most SMs idle, which the next
+    // bucket's smaller worlds then fill.  With the small worlds first the step ended
+    // on the large ones' tail (2,048 worlds of 16 to 2,048 mixed bodies 724 -> 695 us a
+    // step).
     const size_t nbk = buckets_.size();
-    if (nbk > 1) {
-        PE_CHECK(cudaEventRecord(fork_, stream_));
-        for (size_t i = 1; i < nbk; ++i) PE_CHECK(cudaStreamWaitEvent(side_[i - 1], fork_, 0));
-    }
-    for (size_t i = 0; i < nbk; ++i) {
-        cudaStream_t s = i == 0 ? stream_ : side_[i - 1];
+    if (nbk > 1) PE_CHECK(cudaEventRecord(fork_, stream_));
+    for (size_t i = nbk; i-- > 0;) {
+        cudaStream_t s = i == 0 ? stream_ : side_[nbk - 1 - i];
+        if (i > 0) PE_CHECK(cudaStreamWaitEvent(s, fork_, 0));
         launchBatchBucket(view(buckets_[i], dt, parity), buckets_[i].variant, buckets_[i].blocks, s);
     }
     for (size_t i = 1; i < nbk; ++i) {
@@ -471,6 +477,12 @@ bool Batch::finishStep() {
     return false;
 }
 
+void Batch::setVariant(BatchBucket &bk, int variant) {
+    bk.variant = variant;
+    bk.blocks = std::min<uint32_t>((uint32_t)bk.worlds.size(),
+                                   batchMaxBlocks(variant, batchSharedBytes(bk.maxN, bk.maxM)));
+}
+
 void Batch::autotune(float dt, int reps) {
     PE_CHECK(cudaSetDevice(device_));
     if (reps < 1) reps = 1;
@@ -517,11 +529,46 @@ void Batch::autotune(float dt, int reps) {
                 bestV = v;
             }
         }
-        bk.variant = bestV;
-        bk.tunedMs = best;
-        bk.blocks = std::min<uint32_t>((uint32_t)bk.worlds.size(),
-                                       batchMaxBlocks(bestV, batchSharedBytes(bk.maxN, bk.maxM)));
+        setVariant(bk, bestV);
     }
+    // The buckets run side by side in a step, where a variant that is slower alone but
+    // leaves room for the other buckets' worlds can be the better one (1,024 worlds of
+    // 16 to 512 bodies 952 -> 860 us a step, 2,048 of 16 to 2,048 mixed bodies 700 ->
+    // 644).  So each bucket's choice is tried again in the whole step, the largest
+    // worlds first.  (64, 128 and 256 threads with registers for 8, 6 and 3 blocks an
+    // SM were tried as well and never chosen.)
+    if (buckets_.size() > 1) {
+        auto stepMs = [&]() {
+            float total = 0.0f;
+            for (int r = 0; r < reps + 1; ++r) {
+                PE_CHECK(cudaEventRecord(t0_, stream_));
+                launchAll(dt, parity_);
+                PE_CHECK(cudaEventRecord(t1_, stream_));
+                PE_CHECK(cudaStreamSynchronize(stream_));
+                float ms = 0.0f;
+                PE_CHECK(cudaEventElapsedTime(&ms, t0_, t1_));
+                if (r > 0) total += ms;
+            }
+            return (double)total / reps;
+        };
+        double best = stepMs();
+        for (size_t i = buckets_.size(); i-- > 0;) {
+            BatchBucket &bk = buckets_[i];
+            const int from = bk.variant;
+            int bestV = from;
+            for (int v = 0; v < kBatchVariantCount; ++v) {
+                if (v == from || bk.candidateMs[v] <= 0.0) continue;
+                setVariant(bk, v);
+                const double ms = stepMs();
+                if (ms < 0.99 * best) {
+                    best = ms;
+                    bestV = v;
+                }
+            }
+            setVariant(bk, bestV);
+        }
+    }
+    for (BatchBucket &bk : buckets_) bk.tunedMs = bk.candidateMs[bk.variant];
     dropGraphs();
 }
 

@@ -131,6 +131,7 @@ class Batch {
   private:
     void layout(const std::vector<uint32_t> &pairCap, const std::vector<uint32_t> &mCap, bool keepCaches);
     void makeBuckets();
+    void setVariant(BatchBucket &bk, int variant);
     BatchView view(const BatchBucket &bk, float dt, uint32_t parity) const;
     void launchAll(float dt, uint32_t parity);
     bool finishStep();
