@@ -320,9 +320,7 @@ __device__ __noinline__ void stepWorld(const BatchView &b, uint32_t wi, unsigned
             cb = (uint32_t)key;
             ba = w.cbody[ca];
             bb = w.cbody[cb];
-            bool epaFailed;
-            hit = narrowphasePair<false>(w, ca, cb, ba, bb, lm, restitution, friction, category, epaFailed);
-            if (epaFailed) atomicAdd(&st->epaFailures, 1ull);
+            hit = narrowphasePair(w, ca, cb, ba, bb, lm, restitution, friction, category);
             aggregatedCount(st->npCandidates, category);
             if (hit) aggregatedCount(st->npContacts, category);
         }
