@@ -252,8 +252,11 @@ __device__ __noinline__ bool takeWorld(const Args &a, Slot &ws, BlockWorld &bw, 
     return true;
 }
 
-// The step from snapshot `from` to snapshot `to` with scratch `j`.
+// The step from snapshot `from` to snapshot `to` with scratch `j`.  The barrier ahead of
+// the write lets every thread finish with the last step's record: without it a late warp
+// read the error word of a record whose step had not run.
 __device__ __noinline__ void setStep(const Slot &ws, BlockWorld &bw, uint32_t from, uint32_t to, uint32_t j) {
+    __syncthreads();
     if (threadIdx.x == 0) {
         const Snap in = snapshot(ws, from, bw.W.n), out = snapshot(ws, to, bw.W.n);
         bw.in = in.s;
