@@ -1244,11 +1244,8 @@ template <uint32_t T, int E>
 static void launchSapBlock(const BroadInput &in, uint32_t *sapKeys, uint32_t *sapVals, PairBuffers &pb, DevStats *st,
                            cudaStream_t s, const SapCoherence *coh, const PairMapping *finalize) {
     constexpr size_t smem = sapBlockSmem<T * E>();
-    static bool configured = false;
-    if (!configured) {
-        PE_CHECK(cudaFuncSetAttribute(k_sap_block<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
+    static PerDevice raised;
+    allowSharedBytes(raised, k_sap_block<T, E>, smem);
     k_sap_block<T, E><<<1, T, smem, s>>>(
         in, sapKeys, sapVals, coh ? coh->unsorted : nullptr, pb.keys, pb.cap, pb.bits, st, finalize ? 1 : 0,
         finalize ? finalize->inSlot : nullptr, finalize ? finalize->cbody : nullptr,
@@ -1452,12 +1449,9 @@ k_pairs_lists(const unsigned long long *keys, uint32_t cap, const uint32_t *d_n,
 
 bool launchPairsLists(const BroadInput &in, const PairMapping &mapping, PairBuffers &pb, DevStats *st, cudaStream_t s) {
     if (!sapFinalizesPairs(in, pb)) return false;
-    static bool configured = false;
+    static PerDevice raised;
     const size_t smem = sizeof(uint32_t) * (2 * kSapBlockPairs + 2 * kSapBlockMax + kSapBlockMax);
-    if (!configured) {
-        PE_CHECK(cudaFuncSetAttribute(k_pairs_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
+    allowSharedBytes(raised, k_pairs_lists, smem);
     k_pairs_lists<<<1, 1024, smem, s>>>(pb.keys, pb.cap, in.d_n, pb.bits, mapping.inSlot, mapping.cbody, mapping.cbgen, pb.a,
                                         pb.b, st);
     PE_LAUNCHED();
@@ -1591,12 +1585,9 @@ void launchPairsFinalize(const uint32_t *inSlot, const uint32_t *cbody, const ui
                          DevStats *st, Scratch &ws, cudaStream_t s) {
     uint32_t *err = &st->err;
     if (pb.blockPath) {
-        static bool configured = false;
+        static PerDevice raised;
         const size_t smem = kBlockMaxPairs * (2 * sizeof(unsigned long long) + sizeof(uint32_t));
-        if (!configured) {
-            PE_CHECK(cudaFuncSetAttribute(k_pairs_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            configured = true;
-        }
+        allowSharedBytes(raised, k_pairs_block, smem);
         k_pairs_block<<<1, 1024, smem, s>>>(pb.keys, pb.bits, inSlot, cbody, cbgen, pb.a, pb.b, st);
         PE_LAUNCHED();
         return;

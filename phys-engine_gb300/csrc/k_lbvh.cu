@@ -461,11 +461,8 @@ k_lbvh_pairs(const uint32_t *d_n, const unsigned long long *keys, uint32_t index
 
 template <int E> static void launchFront(const BroadInput &in, const LbvhBuffers &lb, uint32_t indexBits, cudaStream_t s) {
     constexpr size_t bytes = frontBytes(kRegSortThreads * E);
-    static bool configured = false;
-    if (!configured) {
-        PE_CHECK(cudaFuncSetAttribute(k_lbvh_front<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        configured = true;
-    }
+    static PerDevice raised;
+    allowSharedBytes(raised, k_lbvh_front<E>, bytes);
     k_lbvh_front<E><<<1, kRegSortThreads, bytes, s>>>(in, lb.keys, indexBits, lb.leafMn, lb.leafMx, lb.rec);
     PE_LAUNCHED();
 }

@@ -501,21 +501,18 @@ static void launchCooperative(const void *fn, int blocks, SolveArgs &args, cudaS
 }
 
 static void configureColor() {
-    static bool configured = false;
-    if (!configured) {
-        PE_CHECK(cudaFuncSetAttribute(k_color, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColorSmem));
-        configured = true;
-    }
+    static PerDevice raised;
+    allowSharedBytes(raised, k_color, kColorSmem);
 }
 
 int maxCooperativeBlocks(int smCount) {
-    static int perSm = -1;
-    if (perSm < 0) {
+    static PerDevice perSm;
+    return smCount * perSm([] {
+        int blocks = 0;
         configureColor();
-        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color, kSolveThreads, kColorSmem));
-        if (perSm < 1) perSm = 1;
-    }
-    return perSm * smCount;
+        PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_color, kSolveThreads, kColorSmem));
+        return blocks < 1 ? 1 : blocks;
+    });
 }
 
 void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &oldCache, const uint32_t *oldCacheCount,
@@ -531,12 +528,8 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
     uint32_t *err = &st->err;
     const uint32_t mcap = sb.mcap;
     if (blockPath) {
-        static bool configured = false;
-        if (!configured) {
-            PE_CHECK(cudaFuncSetAttribute(k_solve_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)blockSolveSmem(kBlockMaxManifolds, kStageSlots)));
-            configured = true;
-        }
+        static PerDevice raised;
+        allowSharedBytes(raised, k_solve_block, blockSolveSmem(kBlockMaxManifolds, kStageSlots));
         uint32_t bm = kBlockMaxManifolds;
         if (blockM && blockM < kBlockMaxManifolds) {
             bm = 64;

@@ -1073,23 +1073,22 @@ ClusterSolveLayout clusterSolveLayout(uint32_t blockM, uint32_t stageSlots) {
 
 bool launchSolverCluster(const SolveArgs &a, const CacheView &newCache, uint32_t *newCacheCount, uint32_t cacheCap,
                          uint32_t blockM, uint32_t stageSlots, cudaStream_t s) {
-    static int usable = -1;
+    static PerDevice usable;
     const ClusterSolveLayout lay = clusterSolveLayout(blockM, stageSlots);
-    if (usable < 0) {
-        usable = 0;
+    const int fits = usable([] {
+        int clusters = 0;
         if (cudaFuncSetAttribute(k_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmemMax) ==
             cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(kClusterRanks);
             cfg.blockDim = dim3(kBlockSolveThreads);
             cfg.dynamicSmemBytes = kClusterSmemMax;
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, k_solve_cluster, &cfg) == cudaSuccess && clusters > 0)
-                usable = 1;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k_solve_cluster, &cfg) != cudaSuccess) clusters = 0;
         }
         cudaGetLastError();  // a refused query leaves no sticky error
-    }
-    if (!usable || lay.smemBytes == 0) return false;
+        return clusters > 0 ? 1 : 0;
+    });
+    if (!fits || lay.smemBytes == 0) return false;
     const uint32_t itemBlocks = (4 * blockM + kIslPrepThreads - 1) / kIslPrepThreads;
     const uint32_t unionBlocks = (blockM + kIslPrepThreads - 1) / kIslPrepThreads;
     k_prepare_islands<<<itemBlocks + unionBlocks, kIslPrepThreads, 0, s>>>(a, blockM, itemBlocks);

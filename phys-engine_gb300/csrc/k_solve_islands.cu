@@ -717,12 +717,12 @@ template <bool ALL> static void launchSweep(const SolveArgs &a, const CacheView 
     // list entries carry the manifold index in kEntryShift bits
     if (a.mcap > kEntryMask) throw std::length_error("manifold capacity beyond the grid-wide sweeps' index range");
     const void *kernel = (const void *)k_isl_sweep<ALL>;
-    static int perSm = -1;
-    if (perSm < 0) {
+    static PerDevice resident;
+    const int perSm = resident([&] {
         int b = 0;
         PE_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kSolveThreads, 0));
-        perSm = b < 1 ? 1 : b;
-    }
+        return b < 1 ? 1 : b;
+    });
     SolveArgs args = a;
     CacheView cache = nc;
     void *params[] = {&args, &cache, &cacheCap};

@@ -1,6 +1,7 @@
 // Internal declarations of the GB300 engine: device-side views of a world,
 // scratch memory, and the stage launchers used by the step pipeline.
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <stdexcept>
@@ -37,6 +38,35 @@ void setSpinLimitIslands(uint32_t limit);
 // Streaming multiprocessors of the current device (queried once per device and
 // cached); launch sizes of the persistent and grid-stride kernels scale with it.
 int smCount();
+
+// A kernel's attributes and occupancy are those of the kernel on one device: what
+// `find` returns, found once on each device (a process may hold worlds on several).
+class PerDevice {
+    static constexpr int kMaxDevices = 64;
+    std::atomic<int64_t> found_[kMaxDevices] = {};  // the value + 2^32; 0: not found yet
+
+  public:
+    template <class Find> int operator()(Find find) {
+        int dev = 0;
+        PE_CHECK(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= kMaxDevices) return find();
+        int64_t v = found_[dev].load(std::memory_order_acquire);
+        if (v == 0) {
+            v = (1ll << 32) + find();
+            found_[dev].store(v, std::memory_order_release);
+        }
+        return (int)(v - (1ll << 32));
+    }
+};
+
+// Raises the kernel's dynamic shared memory to `bytes` on the current device (each
+// kernel with one size; `raised` is the kernel's own).
+template <class Kernel> void allowSharedBytes(PerDevice &raised, Kernel *kernel, size_t bytes) {
+    raised([&] {
+        PE_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        return 1;
+    });
+}
 
 // The device address of a caller's array when kernels on `device` can read and
 // write it in place — pinned host memory (mapped into every device's address
