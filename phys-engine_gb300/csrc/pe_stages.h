@@ -268,7 +268,7 @@ __host__ __device__ inline uint32_t clusterOneRankOffset(uint32_t blockM, uint32
     return (blockM * 20u + stageSlots * 36u + 15u) & ~15u;
 }
 __host__ __device__ inline bool clusterFitsOneRank(uint32_t blockM, uint32_t stageSlots, uint32_t M, uint32_t points) {
-    return clusterOneRankOffset(blockM, stageSlots) + 32u * M + 176u * points <= kClusterSmemMax;
+    return clusterOneRankOffset(blockM, stageSlots) + 32ull * M + 176ull * points <= kClusterSmemMax;
 }
 struct ClusterSolveLayout {
     uint32_t blockM, stageSlots;   // capacities of the single-block front (rank 0)
