@@ -52,7 +52,9 @@ __global__ void k_sap_presort(const uint32_t *d_n, const uint32_t *keyOf, uint32
                 bad = q >= n || !(k < keyOf[q] || (k == keyOf[q] && p < q));
             }
         }
-        if (bad) atomicOr(unsorted, 1u);
+        // one store a warp: thousands of atomics on one word cost more than the check
+        const uint32_t active = __activemask();
+        if (__any_sync(active, bad) && (threadIdx.x & 31) == __ffs(active) - 1) *(volatile uint32_t *)unsorted = 1u;
     }
 }
 
@@ -69,8 +71,7 @@ __global__ void k_sap_order(const uint32_t *d_n, const uint32_t *keyOf, uint32_t
 }
 
 __global__ void k_sap_gather(BroadInput in, const uint32_t *sortedVals, float *sMinX, float *sMaxX, float4 *sYZ,
-                             uint32_t *sIdx, uint32_t *unsorted, uint32_t *counts) {
-    if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) *unsorted = 0u;  // for the next step's check
+                             uint32_t *sIdx, uint32_t *counts) {
     const uint32_t n = *in.d_n;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t idx = sortedVals[i];
@@ -85,17 +86,21 @@ __global__ void k_sap_gather(BroadInput in, const uint32_t *sortedVals, float *s
 
 // The sweep's order of up to kRunSortMax boxes without the sort's passes: tiles of
 // kRunKeys (min.x key, index) keys sorted by a block each, then every key looked up in
-// all other tiles: its rank is its place, and the box goes there at once.  Seven
-// launches of the radix sort (four passes of 8 to 9 us whatever the number of keys)
-// and the check whether the last order still holds cost more than always sorting.
-// Measured, us a step: field of 10,000 bodies 321 -> 303, 16 pyramids with hulls (4,611
-// bodies) 559 -> 529.  The lookups grow with keys times tiles; beyond 16 tiles
-// the sort's passes take over.
+// all other tiles: its rank is its place, and the box goes there at once, in place of
+// the seven launches of the radix sort (four passes of 8 to 9 us whatever the number of
+// keys).  Where the last order still holds (k_sap_presort) neither is done: boxes that
+// fall or rest keep it, and sorting them every step was slower than the check from
+// 16,000 boxes up (field of 20,000 bodies falling: 93 us a step by the radix sort with
+// the check, 104 by tiles always, 85 now; of 30,000 105, 112 and 93).  Measured with
+// bodies that move past one another, us a step: 12,000 mixed bodies 133 by the radix
+// sort, 110 now; 30,000 178 and 153.  The lookups grow with keys times tiles; beyond
+// 16 tiles the sort's passes take over.
 constexpr uint32_t kRunKeys = 2 * kRegSortThreads, kRunSortMax = 16 * kRunKeys;
 
 __global__ void __launch_bounds__(kRegSortThreads)
-k_sap_runs(BroadInput in, unsigned long long *runs) {
+k_sap_runs(BroadInput in, const uint32_t *unsorted, unsigned long long *runs) {
     __shared__ unsigned long long s_a[kRunKeys], s_b[kRunKeys];
+    if (unsorted && *unsorted == 0u) return;  // the last order holds
     const uint32_t n = *in.d_n, base = blockIdx.x * kRunKeys;
     if (base >= n) return;
     unsigned long long v[2];
@@ -112,14 +117,17 @@ k_sap_runs(BroadInput in, unsigned long long *runs) {
     }
 }
 
-__global__ void k_sap_place(BroadInput in, const unsigned long long *runs, float *sMinX, float *sMaxX, float4 *sYZ,
-                            uint32_t *sIdx, uint32_t *counts) {
-    const uint32_t n = *in.d_n, tiles = (n + kRunKeys - 1) / kRunKeys;
+// unsorted, vals (nullable, together): whether the last order holds, and that order,
+// replaced where it does not.
+__global__ void k_sap_place(BroadInput in, const unsigned long long *runs, const uint32_t *unsorted, uint32_t *vals,
+                            float *sMinX, float *sMaxX, float4 *sYZ, uint32_t *sIdx, uint32_t *counts) {
+    const bool held = unsorted && *unsorted == 0u;
+    const uint32_t n = *in.d_n, tiles = held ? 0u : (n + kRunKeys - 1) / kRunKeys;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        const unsigned long long key = runs[q];
+        const unsigned long long key = held ? vals[q] : runs[q];
         const uint32_t own = q / kRunKeys, idx = (uint32_t)key;
         const float4 mn = in.mn[idx], mx = in.mx[idx];
-        uint32_t rank = q - own * kRunKeys;
+        uint32_t rank = held ? q : q - own * kRunKeys;
         // four tiles at a time: keys of the tile below this one
         for (uint32_t t0 = 0; t0 < tiles; t0 += 4) {
             uint32_t lo[4], hi[4];
@@ -149,6 +157,7 @@ __global__ void k_sap_place(BroadInput in, const unsigned long long *runs, float
         sMaxX[rank] = mx.x;
         sYZ[rank] = make_float4(mn.y, mx.y, mn.z, mx.z);
         sIdx[rank] = idx;
+        if (vals && !held) vals[rank] = idx;
         if (counts) counts[q] = 0u;  // for the sweep's pairs
     }
 }
@@ -156,7 +165,8 @@ __global__ void k_sap_place(BroadInput in, const unsigned long long *runs, float
 // Window of sorted entry i: entries i+1 .. e-1 with min.x <= max.x(i), the
 // reference's sweep break (broadphase.cpp:228-231).
 __global__ void k_sap_window(const uint32_t *d_n, const float *sMinX, const float *sMaxX, uint32_t *len,
-                             DevStats *st) {
+                             uint32_t *unsorted, DevStats *st) {
+    if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) *unsorted = 0u;  // for the next step's check
     const uint32_t n = *d_n;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float x = sMaxX[i];
@@ -1265,17 +1275,20 @@ bool launchSap(const BroadInput &in, uint32_t *sapKeys, uint32_t *sapVals, Broad
         return fin;
     }
     const bool lists = finalize && pairListsFit(in, *finalize);
-    if (in.maxN <= kRunSortMax) {
-        k_sap_runs<<<(in.maxN + kRunKeys - 1) / kRunKeys, kRegSortThreads, 0, s>>>(in, pb.keysTmp);
+    if (coh) {
+        k_sap_presort<<<gridFor(in.maxN), 256, 0, s>>>(in.d_n, coh->keyOf, sapKeys, sapVals, coh->unsorted);
         PE_LAUNCHED();
-        k_sap_place<<<gridFor(in.maxN, 128), 128, 0, s>>>(in, pb.keysTmp, bb.sMinX, bb.sMaxX, bb.sYZ, bb.sIdx,
-                                                          lists ? pb.count : nullptr);
+    }
+    if (in.maxN <= kRunSortMax) {
+        const uint32_t *unsorted = coh ? coh->unsorted : nullptr;
+        k_sap_runs<<<(in.maxN + kRunKeys - 1) / kRunKeys, kRegSortThreads, 0, s>>>(in, unsorted, pb.keysTmp);
+        PE_LAUNCHED();
+        k_sap_place<<<gridFor(in.maxN, 128), 128, 0, s>>>(in, pb.keysTmp, unsorted, coh ? sapVals : nullptr, bb.sMinX,
+                                                          bb.sMaxX, bb.sYZ, bb.sIdx, lists ? pb.count : nullptr);
         PE_LAUNCHED();
     } else {
         const uint32_t *sortN = in.d_n;
         if (coh) {
-            k_sap_presort<<<gridFor(in.maxN), 256, 0, s>>>(in.d_n, coh->keyOf, sapKeys, sapVals, coh->unsorted);
-            PE_LAUNCHED();
             k_sap_order<<<gridFor(in.maxN), 256, 0, s>>>(in.d_n, coh->keyOf, sapKeys, sapVals, coh->unsorted,
                                                          coh->sortCount);
             PE_LAUNCHED();
@@ -1283,10 +1296,10 @@ bool launchSap(const BroadInput &in, uint32_t *sapKeys, uint32_t *sapVals, Broad
         }
         launchRadixSort<uint32_t>(sapKeys, bb.keyTmp32, sapVals, bb.valTmp, sortN, in.maxN, 0, 32, ws, err, s);
         k_sap_gather<<<gridFor(in.maxN), 256, 0, s>>>(in, sapVals, bb.sMinX, bb.sMaxX, bb.sYZ, bb.sIdx,
-                                                      coh ? coh->unsorted : nullptr, lists ? pb.count : nullptr);
+                                                      lists ? pb.count : nullptr);
         PE_LAUNCHED();
     }
-    k_sap_window<<<gridFor(in.maxN), 256, 0, s>>>(in.d_n, bb.sMinX, bb.sMaxX, bb.len, st);
+    k_sap_window<<<gridFor(in.maxN), 256, 0, s>>>(in.d_n, bb.sMinX, bb.sMaxX, bb.len, coh ? coh->unsorted : nullptr, st);
     PE_LAUNCHED();
     launchScanExclusive(bb.len, bb.off, in.d_n, in.maxN, &st->windowWork, ws, err, s);
     k_sap_emit<<<6 * smCount(), kSweepThreads, 0, s>>>(in.d_n, bb.off, bb.len, bb.sYZ, bb.sIdx, pb.keys, pb.cap, pb.bits,

@@ -349,3 +349,37 @@ def test_batched_worlds_equal_single_ones_on_either_memory(gpu, n):
         for g, key in zip(got, ("pos", "quat", "lin", "ang")):
             assert_bit_equal(g, want[key], f"{n} world {k} {key}")
         assert_manifolds_equal(batch.contacts(k), w.contacts(), what=f"{n} world {k}")
+
+
+@pytest.mark.parametrize("n", [4097, 6145, 32767])
+def test_sweep_order_held_and_broken(gpu, n):
+    """The tiles' sort is left out while the last order holds: spheres at rest
+    (held), a tenth of them moved past the others (broken, then held again in
+    the new order), two bodies more (other counts: 32,768 and 32,769, where the
+    radix sort takes the order over)."""
+    rng = np.random.default_rng(n)
+    side = 1.1 * n ** (1 / 3)
+    sc = sphere_scene(rng.uniform(-side / 2, side / 2, (n, 3)), np.full(n, 0.3), np.zeros(n))
+    worlds, handles = [], []
+    for algo in (gpu.SAP, gpu.GRID):
+        w = gpu.GpuWorld(algo=algo, iterations=1)
+        w.set_gravity((0.0, 0.0, 0.0))
+        handles.append(w.load_scene(sc))
+        worlds.append(w)
+    movers = rng.choice(n, n // 10, replace=False)
+    to = rng.uniform(-side / 2, side / 2, (len(movers), 3)).astype(np.float32)
+    extra = rng.uniform(-side / 2, side / 2, (2, 3)).astype(np.float32)
+    for phase in range(4):
+        for w, h in zip(worlds, handles):
+            if phase == 1:
+                for i, p in zip(movers, to):
+                    at = gpu.Handle(*(int(x) for x in h[i, :2]))
+                    st = w.get_body(at)
+                    st.position[:] = p
+                    w.set_body(at, st)
+            elif phase > 1:
+                w.create_body(0, (0.3, 0.0, 0.0), extra[phase - 2], 1.0, False, 0.0, 0.5)
+        for step in range(2):
+            for w in worlds:
+                w.step(1e-3)
+            assert_bit_equal(worlds[0].pairs(), worlds[1].pairs(), f"{n} phase {phase} step {step}")
