@@ -14,7 +14,7 @@
 //   k_lbvh_refit  : node bounds bottom-up (the second child to arrive at a node
 //                   unites both children, writes the node's record and climbs on)
 //   k_lbvh_front  : the four above in one block for up to kFrontMax boxes
-//   k_lbvh_pairs  : eight lanes per leaf walk the tree with its AABB and emit
+//   k_lbvh_pairs  : two to eight lanes per leaf walk the tree with its AABB and emit
 //                   the overlapping leaves of a higher size class, and of its
 //                   own class those after it in sorted order (each pair once),
 //                   touching counting as overlap (Aabb::overlaps)
@@ -81,22 +81,30 @@ __device__ __forceinline__ uint32_t reportKey(const float4 &mn, const float4 &mx
     return (u < 0x7F800000u ? u : 0x7F800000u) >> 24 << 24 | l >> shift;
 }
 
-// A node's record: both children's bounds in one 64-byte line, the child (leaf
-// children flagged) in mn.w, the highest reporting key below it in mx.w.
-__device__ __forceinline__ void uniteChildren(const float4 (&mn)[2], const float4 (&mx)[2], const uint32_t (&c)[2],
-                                              float4 *rec, float4 &omn, float4 &omx) {
+// Bounds of two boxes, the higher of their reporting keys in mx.w.
+__device__ __forceinline__ void unite(const float4 (&mn)[2], const float4 (&mx)[2], float4 &omn, float4 &omx) {
     omn = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
     omx = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
     uint32_t top = 0;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        rec[2 * k] = make_float4(mn[k].x, mn[k].y, mn[k].z, __uint_as_float(c[k]));
-        rec[2 * k + 1] = mx[k];
         omn = make_float4(fminf(omn.x, mn[k].x), fminf(omn.y, mn[k].y), fminf(omn.z, mn[k].z), 0.0f);
         omx = make_float4(fmaxf(omx.x, mx[k].x), fmaxf(omx.y, mx[k].y), fmaxf(omx.z, mx[k].z), 0.0f);
         top = max(top, __float_as_uint(mx[k].w));
     }
     omx.w = __uint_as_float(top);
+}
+
+// A node's record: both children's bounds in one 64-byte line, the child (leaf
+// children flagged) in mn.w, the highest reporting key below it in mx.w.
+__device__ __forceinline__ void uniteChildren(const float4 (&mn)[2], const float4 (&mx)[2], const uint32_t (&c)[2],
+                                              float4 *rec, float4 &omn, float4 &omx) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        rec[2 * k] = make_float4(mn[k].x, mn[k].y, mn[k].z, __uint_as_float(c[k]));
+        rec[2 * k + 1] = mx[k];
+    }
+    unite(mn, mx, omn, omx);
 }
 
 // Common-prefix length of sorted keys i and j; -1 outside [0, n).
@@ -219,32 +227,45 @@ __global__ void k_lbvh_build(BroadInput in, const unsigned long long *keys, uint
     }
 }
 
-// Node bounds and records from the leaves up; the second arrival at a node
-// unites both children (their bounds are published before the arrival counter
-// moves).
+// Node records from the leaves up; the second arrival at a node unites both
+// children: its own bounds, which it carries, and the sibling's, from the sibling's
+// record (published before the arrival counter moves).  What bounds it is traffic
+// and the fences (300,000 leaves 71 us; 80 with bounds of the nodes kept beside the
+// records, 57 before there were records).
 __global__ void k_lbvh_refit(const uint32_t *d_n, const uint32_t *childL, const uint32_t *childR,
                              const uint32_t *parent, const uint32_t *leafParent, uint32_t *visit, const float4 *leafMn,
-                             const float4 *leafMx, float4 *nodeMn, float4 *nodeMx, float4 *rec) {
+                             const float4 *leafMx, float4 *rec) {
     const uint32_t n = *d_n;
     if (n < 2) return;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        uint32_t node = leafParent[t];
+        uint32_t node = leafParent[t], from = kLeafBit | t;
+        float4 ownMn = leafMn[t], ownMx = leafMx[t];  // of the child that this thread comes from
         for (uint32_t depth = 0; depth < n; ++depth) {
             __threadfence();
             if (atomicAdd(&visit[node], 1u) == 0u) break;  // the sibling finishes this node
             __threadfence();
             const uint32_t c[2] = {childL[node], childR[node]};
-            float4 mn[2], mx[2], omn, omx;
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const uint32_t l = c[k] & ~kLeafBit;
-                mn[k] = c[k] & kLeafBit ? leafMn[l] : __ldcg(&nodeMn[l]);
-                mx[k] = c[k] & kLeafBit ? leafMx[l] : __ldcg(&nodeMx[l]);
+            const bool second = c[1] == from;
+            const uint32_t other = second ? c[0] : c[1], l = other & ~kLeafBit;
+            float4 mn[2], mx[2];
+            if (other & kLeafBit) {
+                mn[0] = leafMn[l];
+                mx[0] = leafMx[l];
+            } else {  // the sibling's bounds are those of its record's two children
+                const float4 *r = rec + 4 * (size_t)l;
+                const float4 a = __ldcg(r), b = __ldcg(r + 1), e = __ldcg(r + 2), f = __ldcg(r + 3);
+                const float4 cmn[2] = {a, e}, cmx[2] = {b, f};
+                unite(cmn, cmx, mn[0], mx[0]);
             }
-            uniteChildren(mn, mx, c, rec + 4 * (size_t)node, omn, omx);
-            __stcg(&nodeMn[node], omn);
-            __stcg(&nodeMx[node], omx);
+            mn[1] = second ? ownMn : mn[0];
+            mx[1] = second ? ownMx : mx[0];
+            if (!second) {
+                mn[0] = ownMn;
+                mx[0] = ownMx;
+            }
+            uniteChildren(mn, mx, c, rec + 4 * (size_t)node, ownMn, ownMx);
             if (node == 0) break;
+            from = node;
             node = parent[node];
         }
     }
@@ -369,27 +390,31 @@ k_lbvh_front(BroadInput in, unsigned long long *keys, uint32_t indexBits, float4
     }
 }
 
-// Walks are long and uneven, and each step waits for its node's record: eight
-// lanes a leaf take up to eight nodes off the leaf's stack at a time, and 64-thread
-// blocks spread the leaves of a small world over the SMs.
+// Walks are long and uneven, and each step waits for its node's record: up to eight
+// lanes a leaf take as many nodes off the leaf's stack at a time, and 64-thread
+// blocks spread the leaves of a small world over the SMs.  Once the leaves fill the chip,
+// lanes that find no node on the stack take the place of other leaves: a leaf then has
+// four lanes, or two.  Broadphase in us with eight, four and two lanes: 20,000 mixed bodies
+// 116, 112, 117, of a settled field 142, 147, 166; 40,000 135, 125, 128 and 190, 183, 202;
+// 66,000 159, 144, 141 and 230, 215, 214; a falling field of 140,000 218, 177, 160 (a
+// thread a leaf in the kernel before the lanes 199), of 300,000 388, 293, 250 (247).
 constexpr int kLbvhWalkThreads = 64;
-constexpr uint32_t kWalkLanes = 8, kWalkLeaves = kLbvhWalkThreads / kWalkLanes;
 // Stack of a leaf: with fewer than kTreeDepth free entries beyond what a round can
 // push, one node is taken at a time, and what that pushes is at most the tree's depth
 // (a key has 30 + index bits).
-constexpr uint32_t kTreeDepth = 64, kWalkStack = 192;
-inline int lbvhWalkGrid(uint32_t n) {
-    const uint32_t b = (n + kWalkLeaves - 1) / kWalkLeaves, maxGrid = 32u * (uint32_t)smCount();
-    return (int)(b ? (b < maxGrid ? b : maxGrid) : 1u);
-}
+constexpr uint32_t kTreeDepth = 64;
+constexpr uint32_t kWalkThreadsPerSm = 1536;  // three quarters of what an SM holds
 
 // Leaf t's AABB against the tree; pairs with the leaves of a higher size class
 // and the later leaves of its own.
+template <uint32_t kWalkLanes>
 __global__ void __launch_bounds__(kLbvhWalkThreads)
 k_lbvh_pairs(const uint32_t *d_n, const unsigned long long *keys, uint32_t indexBits, const float4 *leafMn,
              const float4 *leafMx, const float4 *rec, unsigned long long *pkeys, uint32_t cap, uint32_t bits,
              uint32_t *counts, uint32_t *ranks, DevStats *st) {
-    __shared__ uint32_t s_stack[kWalkLeaves][kWalkStack];
+    constexpr uint32_t kWalkLeaves = kLbvhWalkThreads / kWalkLanes, kWalkStack = kTreeDepth + 16 * kWalkLanes;
+    constexpr uint32_t kWalkMask = (1u << kWalkLanes) - 1u;
+    __shared__ uint32_t s_stack[kWalkLeaves][kWalkStack + kWalkLanes];  // (rows on different banks)
     const uint32_t n = *d_n;
     if (n < 2) return;
     const unsigned long long idxMask = (1ull << indexBits) - 1ull;
@@ -426,8 +451,8 @@ k_lbvh_pairs(const uint32_t *d_n, const unsigned long long *keys, uint32_t index
                     else push[e] = over && key >= qk;
                 }
             }
-            const uint32_t push0 = (__ballot_sync(0xffffffffu, push[0]) >> shift) & 0xFFu;
-            const uint32_t push1 = (__ballot_sync(0xffffffffu, push[1]) >> shift) & 0xFFu;
+            const uint32_t push0 = (__ballot_sync(0xffffffffu, push[0]) >> shift) & kWalkMask;
+            const uint32_t push1 = (__ballot_sync(0xffffffffu, push[1]) >> shift) & kWalkMask;
             const uint32_t at0 = sp + __popc(push0 & below), at1 = sp + __popc(push0) + __popc(push1 & below);
             sp += __popc(push0) + __popc(push1);
             pops += k;
@@ -467,6 +492,17 @@ template <int E> static void launchFront(const BroadInput &in, const LbvhBuffers
     PE_LAUNCHED();
 }
 
+template <uint32_t LANES>
+static void launchWalk(const BroadInput &in, const LbvhBuffers &lb, uint32_t indexBits, PairBuffers &pb, bool lists,
+                       DevStats *st, cudaStream_t s) {
+    constexpr uint32_t leaves = kLbvhWalkThreads / LANES;
+    const uint32_t b = (in.maxN + leaves - 1) / leaves, maxGrid = 32u * (uint32_t)smCount();
+    k_lbvh_pairs<LANES><<<(b ? (b < maxGrid ? b : maxGrid) : 1u), kLbvhWalkThreads, 0, s>>>(
+        in.d_n, lb.keys, indexBits, lb.leafMn, lb.leafMx, lb.rec, pb.keys, pb.cap, pb.bits,
+        lists ? pb.count : nullptr, pb.flags, st);
+    PE_LAUNCHED();
+}
+
 bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, DevStats *st, Scratch &ws,
                 cudaStream_t s, const PairMapping &finalize) {
     uint32_t indexBits = 1;
@@ -494,13 +530,13 @@ bool launchLbvh(const BroadInput &in, const LbvhBuffers &lb, PairBuffers &pb, De
                                                 lb.leafParent, lb.visit, lb.leafMn, lb.leafMx);
         PE_LAUNCHED();
         k_lbvh_refit<<<g, kLbvhThreads, 0, s>>>(in.d_n, lb.childL, lb.childR, lb.parent, lb.leafParent, lb.visit,
-                                                lb.leafMn, lb.leafMx, lb.nodeMn, lb.nodeMx, lb.rec);
+                                                lb.leafMn, lb.leafMx, lb.rec);
         PE_LAUNCHED();
     }
-    k_lbvh_pairs<<<lbvhWalkGrid(in.maxN), kLbvhWalkThreads, 0, s>>>(in.d_n, lb.keys, indexBits, lb.leafMn, lb.leafMx,
-                                                                    lb.rec, pb.keys, pb.cap, pb.bits, lists ? pb.count : nullptr,
-                                                                    pb.flags, st);
-    PE_LAUNCHED();
+    const uint32_t threads = kWalkThreadsPerSm * (uint32_t)smCount();
+    if (in.maxN <= threads / 8) launchWalk<8>(in, lb, indexBits, pb, lists, st, s);
+    else if (in.maxN <= threads / 4) launchWalk<4>(in, lb, indexBits, pb, lists, st, s);
+    else launchWalk<2>(in, lb, indexBits, pb, lists, st, s);
     if (lists) {
         launchPairsOrder(in, pb, st, ws, s);
         return true;

@@ -58,7 +58,6 @@ struct LbvhBuffers {
     uint32_t *childL, *childR, *parent;   // internal nodes (leaf children flagged)
     uint32_t *leafParent, *visit;
     float4 *leafMn, *leafMx;              // leaf bounds in sorted order
-    float4 *nodeMn, *nodeMx;              // internal node bounds
     float4 *rec;                          // [4 n] internal nodes: both children's bounds
     uint32_t *box;                        // [6] ordered-float bounds of the centres
 };

@@ -715,12 +715,10 @@ void World::ensureLbvh() {
     lbBox_.reserve(8);
     lbLeafMn_.reserve(n);
     lbLeafMx_.reserve(n);
-    lbNodeMn_.reserve(n);
-    lbNodeMx_.reserve(n);
     lbRec_.reserve(4 * (size_t)n);
     lb_ = LbvhBuffers{lbKeys_.ptr,     lbKeysTmp_.ptr, lbChildL_.ptr,  lbChildR_.ptr,   lbParent_.ptr,
                       lbLeafParent_.ptr, lbVisit_.ptr,  lbLeafMn_.ptr,   lbLeafMx_.ptr,
-                      lbNodeMn_.ptr,   lbNodeMx_.ptr,  lbRec_.ptr, lbBox_.ptr};
+                      lbRec_.ptr,      lbBox_.ptr};
 }
 
 WorldView World::view(float dt) {

@@ -275,7 +275,7 @@ class World {
     LbvhBuffers lb_{};
     DeviceArray<unsigned long long> lbKeys_, lbKeysTmp_;
     DeviceArray<uint32_t> lbChildL_, lbChildR_, lbParent_, lbLeafParent_, lbVisit_, lbBox_;
-    DeviceArray<float4> lbLeafMn_, lbLeafMx_, lbNodeMn_, lbNodeMx_, lbRec_;
+    DeviceArray<float4> lbLeafMn_, lbLeafMx_, lbRec_;
     void ensureLbvh();
     PairBuffers pb_{};
     DeviceArray<unsigned long long> pairKeys_, pairKeysTmp_;

@@ -383,3 +383,27 @@ def test_sweep_order_held_and_broken(gpu, n):
             for w in worlds:
                 w.step(1e-3)
             assert_bit_equal(worlds[0].pairs(), worlds[1].pairs(), f"{n} phase {phase} step {step}")
+
+
+@pytest.mark.parametrize("lanes", [8, 4])
+@pytest.mark.parametrize("beyond", [0, 1])
+def test_tree_walk_with_fewer_lanes(gpu, lanes, beyond):
+    """The last size with so many lanes a leaf (they fill three quarters of the
+    chip's threads) and the first beyond: a floor under spheres of three sizes."""
+    import torch
+
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 1536 // lanes + beyond
+    rng = np.random.default_rng(n)
+    side = 1.3 * n ** (1 / 3)
+    pos = rng.uniform(-side / 2, side / 2, (n, 3))
+    sc = sphere_scene(pos, rng.choice([0.2, 0.35, 0.6], n), np.zeros(n))
+    sc.shape[0], sc.is_static[0] = 1, 1
+    sc.pos[0], sc.dims[0] = [0, -side / 2, 0], [side, 1.0, side]
+    got = {}
+    for algo in (gpu.GRID, gpu.TREE):
+        w = gpu.GpuWorld(algo=algo, iterations=1)
+        w.load_scene(sc)
+        w.step(1e-4)
+        got[algo] = w.pairs()
+    assert np.count_nonzero(got[gpu.TREE][:, 0] == 0) > 300 and len(got[gpu.TREE]) > n
+    assert_bit_equal(got[gpu.TREE], got[gpu.GRID], f"{n}")
