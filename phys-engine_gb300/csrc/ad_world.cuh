@@ -39,7 +39,7 @@ constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 constexpr int kTapeScalars = 24; // vA, wA, vB, wB, then 4 x (n, t1, t2)
 constexpr int kPmScalars = 20;   // IA (9), IB (9), imA, imB
 
-enum : uint32_t { kAdErrPairs = 1, kAdErrManifolds = 2, kAdErrColors = 4, kAdErrCache = 8 };
+enum : uint32_t { kAdErrPairs = 1, kAdErrManifolds = 2, kAdErrCache = 8 };
 
 AD_HD uint32_t nextPow2u(uint32_t v) {
     uint32_t p = 1;

@@ -549,6 +549,7 @@ void launchSolver(const WorldView &w, const ManifoldView &mv, const CacheView &o
     PE_CHECK(cudaMemsetAsync(sb.counters, 0, 4 * sizeof(uint32_t), s));
     PE_CHECK(cudaMemsetAsync(sb.bar, 0, 2 * sizeof(uint32_t), s));
     const bool serial = orderMode == 0;
+    // (pairOrderCache: every collider is on a live body, which the sweeps rely on)
     const bool sweep = sweepAll && !serial && pairOrderCache;
     // The prepare kernel and the cache's offsets need nothing of the colouring, which
     // waits for its own chains (33 us for 17,000 manifolds) on a block an SM: beside

@@ -633,6 +633,10 @@ __device__ __forceinline__ void writePoint(const SolveArgs &a, const CacheView &
 
 // ALL: every manifold of the step (colour counts and body masks from k_color,
 // results written here); otherwise those that k_isl_fill left to the sweeps.
+// ALL takes manifolds whose body handles are both live, or whose bodies both do not
+// move (sleeping).  A stale handle beside a moving body would count in that body's mask
+// without an update, and the body's later updates would wait for it until their limit.
+// The host takes this path only where collider i is on live body i (launchSolver).
 template <bool ALL>
 __global__ void __launch_bounds__(kSolveThreads, 2) k_isl_sweep(SolveArgs a, CacheView nc, uint32_t cacheCap) {
     __shared__ uint32_t s_start[kMaxColors + 1];  // first item of each colour

@@ -179,7 +179,7 @@ constexpr uint32_t kIslCounterWords = 10 + 2 * kMaxColors;
 void launchSolveIslands(const SolveArgs &a, Scratch &ws, cudaStream_t s);
 // The sweeps over the whole grid alone, for every manifold (after k_color,
 // prepare and the cache offsets), with the impulses and the warm-start cache
-// written by the sweeps.
+// written by the sweeps.  Every manifold's body handles must be live.
 void launchSolveSweep(const SolveArgs &a, const CacheView &newCache, uint32_t cacheCap, cudaStream_t s);
 void launchSleepWake(const WorldView &w, const ManifoldView &mv, uint32_t Mhost, uint32_t mcap, uint32_t *flags,
                      float *quiet, uint32_t *err, cudaStream_t s);

@@ -506,7 +506,6 @@ void Rollout::checkErrors(cudaStream_t s, const char *what) {
             const uint32_t b = e[w];
             const char *m = (b & kAdErrPairs)       ? "candidate pairs exceed the world's capacity"
                             : (b & kAdErrManifolds) ? "contact manifolds exceed the world's capacity"
-                            : (b & kAdErrColors)    ? "solver colouring failed"
                                                     : "warm-start cache overflow";
             throw std::runtime_error(std::string(what) + ": world " + std::to_string(w) + ": " + m);
         }

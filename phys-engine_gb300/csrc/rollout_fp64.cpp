@@ -84,7 +84,6 @@ struct ScratchMem {
 const char *errorText(uint32_t bits) {
     if (bits & kAdErrPairs) return "candidate pairs exceed the rollout's pair capacity";
     if (bits & kAdErrManifolds) return "contact manifolds exceed the rollout's manifold capacity";
-    if (bits & kAdErrColors) return "more than 128 solver colours";
     if (bits & kAdErrCache) return "warm-start cache overflow";
     return "rollout failed";
 }
