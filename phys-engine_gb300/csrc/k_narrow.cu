@@ -22,7 +22,10 @@ namespace pe {
 // 1,501 bodies 399 -> 380, 100,000 mixed bodies 143 -> 135, 16 pyramids with hulls
 // 599 -> 574; 65,536 boxes in stacks (65,536 pairs, seven rounds) 320, with lanes 336.
 // A round is 9 us and a thread a pair 22 to 23 whatever there is: 25,070 pairs, three
-// rounds, 27.2 with lanes and 21.8 without.
+// rounds, 27.2 with lanes and 21.8 without.  There a warp takes its pairs by itself: in
+// tiles of a block's 256 pairs, which wait for their slowest, 92,476 pairs of boxes took
+// 49 us and 23,082 of hulls 288 (44 and 255 in the blocks of 64 before the lanes), now
+// 42 and 256.
 constexpr int kNarrowThreads = 256;
 constexpr int kNarrowBlocks = 2;  // resident blocks an SM
 constexpr uint32_t kNarrowPairs = kNarrowThreads / kPairLanes;
@@ -31,8 +34,8 @@ static_assert(kNarrowPairs == 32, "one warp ranks a tile's pairs");
 static_assert(kNarrowPairs >= kMinLookbackTile, "look-back scratch is sized for kMinLookbackTile");
 
 struct NarrowShared {
-    uint32_t tile, prefix, abort;
-    uint32_t hits[kNarrowPairs], rank[kNarrowPairs], scan[9];
+    uint32_t tile, abort;
+    uint32_t hits[kNarrowPairs], rank[kNarrowPairs];
 };
 
 // Counters of a tested pair (the first lane of its lanes).
@@ -108,42 +111,41 @@ __device__ __forceinline__ bool laneTile(const WorldView &w, const uint32_t *pai
     return true;
 }
 
-// One tile, a thread a pair; as laneTile.
-__device__ __forceinline__ bool threadTile(const WorldView &w, const uint32_t *pairA, const uint32_t *pairB,
-                                           uint32_t P, uint32_t ntiles, const ManifoldView &out, uint32_t mcap,
-                                           DevStats *st, unsigned long long *state, NarrowShared &sh) {
-    const uint32_t p = sh.tile * kNarrowThreads + threadIdx.x;
-    PairSide a, b;
-    LocalManifold lm;
-    lm.count = 0;
-    float restitution = 0.0f, friction = 0.0f;
-    bool hit = false, epaFailed;
-    if (p < P) {
-        const uint32_t ca = pairA[p], cb = pairB[p];
-        a = loadPairSide(w, ca);
-        b = loadPairSide(w, cb);
-        hit = narrowphaseRecords(w, ca, cb, a, b, lm, restitution, friction, epaFailed);
-        countPair(st, pairCategory(a, b), epaFailed, hit, lm.count);
-    }
-    uint32_t total;
-    const uint32_t local = blockExclusiveScan(hit ? 1u : 0u, total, sh.scan);
-    if (threadIdx.x < 32) {
-        bool timedOut;
-        const uint32_t pre = lookbackExclusiveWarp(state, sh.tile, total, &st->err, &timedOut);
-        if (threadIdx.x == 0) {
-            sh.prefix = pre;
-            sh.abort = timedOut ? 1u : 0u;
-            if (sh.tile + 1 == ntiles && !timedOut) {
-                st->manifolds = pre + total;
-                st->stamp[3] = globalNs();
-            }
+// A thread a pair: each warp takes tiles of 32 pairs by itself, so that it waits for
+// the slowest of 32 pairs and not of a block's 256.
+__device__ __forceinline__ void threadTiles(const WorldView &w, const uint32_t *pairA, const uint32_t *pairB,
+                                            uint32_t P, const ManifoldView &out, uint32_t mcap, DevStats *st,
+                                            unsigned long long *state, uint32_t *counter) {
+    const uint32_t lane = threadIdx.x & 31, ntiles = (P + 31) / 32;
+    for (;;) {
+        uint32_t tile = 0;
+        if (lane == 0) tile = atomicAdd(counter, 1u);
+        tile = __shfl_sync(0xffffffffu, tile, 0);
+        if (tile >= ntiles) return;
+        const uint32_t p = tile * 32 + lane;
+        PairSide a, b;
+        LocalManifold lm;
+        lm.count = 0;
+        float restitution = 0.0f, friction = 0.0f;
+        bool hit = false, epaFailed;
+        if (p < P) {
+            const uint32_t ca = pairA[p], cb = pairB[p];
+            a = loadPairSide(w, ca);
+            b = loadPairSide(w, cb);
+            hit = narrowphaseRecords(w, ca, cb, a, b, lm, restitution, friction, epaFailed);
+            countPair(st, pairCategory(a, b), epaFailed, hit, lm.count);
         }
+        const uint32_t hits = __ballot_sync(0xffffffffu, hit), total = __popc(hits);
+        bool timedOut;
+        const uint32_t pre = lookbackExclusiveWarp(state, tile, total, &st->err, &timedOut);
+        if (timedOut) return;  // nothing of this tile is written
+        if (lane == 0 && tile + 1 == ntiles) {
+            st->manifolds = pre + total;
+            st->stamp[3] = globalNs();
+        }
+        const uint32_t m = pre + __popc(hits & ((1u << lane) - 1u));
+        if (hit && m < mcap) storeManifoldGen(out, m, a.body, a.gen, b.body, b.gen, lm, restitution, friction);
     }
-    __syncthreads();
-    if (sh.abort) return false;
-    const uint32_t m = sh.prefix + local;
-    if (hit && m < mcap) storeManifoldGen(out, m, a.body, a.gen, b.body, b.gen, lm, restitution, friction);
-    return true;
 }
 
 __global__ void __launch_bounds__(kNarrowThreads, kNarrowBlocks)
@@ -160,12 +162,13 @@ k_narrowphase(WorldView w, const uint32_t *__restrict__ pairA, const uint32_t *_
         }
         return;
     }
-    const bool lanes = P <= laneMax;
-    const uint32_t per = lanes ? kNarrowPairs : (uint32_t)kNarrowThreads, ntiles = (P + per - 1) / per;
+    if (P > laneMax) {
+        threadTiles(w, pairA, pairB, P, out, mcap, st, state, counter);
+        return;
+    }
+    const uint32_t ntiles = (P + kNarrowPairs - 1) / kNarrowPairs;
     while (takeTile(counter, &sh.tile) < ntiles) {
-        if (!(lanes ? laneTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)
-                    : threadTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)))
-            return;
+        if (!laneTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)) return;
         __syncthreads();
     }
 }
