@@ -23,9 +23,9 @@ namespace pe {
 // 599 -> 574; 65,536 boxes in stacks (65,536 pairs, seven rounds) 320, with lanes 336.
 // A round is 9 us and a thread a pair 22 to 23 whatever there is: 25,070 pairs, three
 // rounds, 27.2 with lanes and 21.8 without.  There a warp takes its pairs by itself: in
-// tiles of a block's 256 pairs, which wait for their slowest, 92,476 pairs of boxes took
-// 49 us and 23,082 of hulls 288 (44 and 255 in the blocks of 64 before the lanes), now
-// 42 and 256.
+// tiles of a block's 256 pairs, which wait for their slowest and leave SMs without one,
+// 23,082 pairs of hulls took 288 us and 92,476 of boxes 49 (255 and 44 in the blocks of
+// 64 before the lanes), now 200 and 45.
 constexpr int kNarrowThreads = 256;
 constexpr int kNarrowBlocks = 2;  // resident blocks an SM
 constexpr uint32_t kNarrowPairs = kNarrowThreads / kPairLanes;
@@ -115,13 +115,20 @@ __device__ __forceinline__ bool laneTile(const WorldView &w, const uint32_t *pai
 // the slowest of 32 pairs and not of a block's 256.
 __device__ __forceinline__ void threadTiles(const WorldView &w, const uint32_t *pairA, const uint32_t *pairB,
                                             uint32_t P, const ManifoldView &out, uint32_t mcap, DevStats *st,
-                                            unsigned long long *state, uint32_t *counter) {
+                                            unsigned long long *state, uint32_t *counter, NarrowShared &sh) {
     const uint32_t lane = threadIdx.x & 31, ntiles = (P + 31) / 32;
-    for (;;) {
-        uint32_t tile = 0;
-        if (lane == 0) tile = atomicAdd(counter, 1u);
-        tile = __shfl_sync(0xffffffffu, tile, 0);
-        if (tile >= ntiles) return;
+    // a block's share of the first round by one atomic (one a warp is 2 us of them), the
+    // tiles spread over all blocks
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t first = min(kNarrowThreads / 32u, (ntiles + gridDim.x - 1) / gridDim.x);
+    if (threadIdx.x == 0) sh.tile = atomicAdd(counter, first);
+    __syncthreads();
+    auto next = [&] {
+        uint32_t t = 0;
+        if (lane == 0) t = atomicAdd(counter, 1u);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    for (uint32_t tile = warp < first ? sh.tile + warp : next(); tile < ntiles; tile = next()) {
         const uint32_t p = tile * 32 + lane;
         PairSide a, b;
         LocalManifold lm;
@@ -162,15 +169,15 @@ k_narrowphase(WorldView w, const uint32_t *__restrict__ pairA, const uint32_t *_
         }
         return;
     }
-    if (P > laneMax) {
-        threadTiles(w, pairA, pairB, P, out, mcap, st, state, counter);
+    if (P <= laneMax) {
+        const uint32_t ntiles = (P + kNarrowPairs - 1) / kNarrowPairs;
+        while (takeTile(counter, &sh.tile) < ntiles) {
+            if (!laneTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)) return;
+            __syncthreads();
+        }
         return;
     }
-    const uint32_t ntiles = (P + kNarrowPairs - 1) / kNarrowPairs;
-    while (takeTile(counter, &sh.tile) < ntiles) {
-        if (!laneTile(w, pairA, pairB, P, ntiles, out, mcap, st, state, sh)) return;
-        __syncthreads();
-    }
+    threadTiles(w, pairA, pairB, P, out, mcap, st, state, counter, sh);
 }
 
 void launchNarrowphase(const WorldView &w, const PairBuffers &pb, const ManifoldView &mv, uint32_t mcap, DevStats *st,
