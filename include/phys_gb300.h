@@ -358,8 +358,9 @@ pe_status pe_batch_set_gravity(pe_batch *batch, float x, float y, float z);
 pe_status pe_batch_set_iterations(pe_batch *batch, int iterations);
 /* `steps` steps of every world (PhysicsWorld::step(dt) per world). */
 pe_status pe_batch_step(pe_batch *batch, float dt, uint32_t steps);
-/* Times every kernel variant on every bucket (`repetitions` launches each,
-   from the current state, which stays unchanged) and keeps the fastest. */
+/* Times every kernel variant on every bucket (the fastest of `repetitions`
+   launches each, from the current state, which stays unchanged), then, where
+   there are several buckets, in the whole step, and keeps the fastest. */
 pe_status pe_batch_autotune(pe_batch *batch, float dt, int repetitions);
 pe_status pe_batch_bucket_count(pe_batch *batch, uint32_t *count);
 pe_status pe_batch_get_bucket(pe_batch *batch, uint32_t index, pe_batch_bucket *out);

@@ -510,7 +510,7 @@ void Batch::autotune(float dt, int reps) {
                 continue;
             }
             BatchView view = this->view(bk, dt, parity_);
-            float total = 0.0f;
+            float least = 1e30f;
             for (int r = 0; r < reps + 1; ++r) {
                 PE_CHECK(cudaMemsetAsync(queueHead_.ptr + bi, 0, sizeof(uint32_t), stream_));
                 PE_CHECK(cudaMemsetAsync(batchErr_.ptr, 0, sizeof(uint32_t), stream_));
@@ -520,12 +520,11 @@ void Batch::autotune(float dt, int reps) {
                 PE_CHECK(cudaStreamSynchronize(stream_));
                 float ms = 0.0f;
                 PE_CHECK(cudaEventElapsedTime(&ms, t0_, t1_));
-                if (r > 0) total += ms;  // the first launch warms up
+                if (r > 0) least = std::min(least, ms);  // the first launch warms up
             }
-            const double avg = total / reps;
-            bk.candidateMs[v] = avg;
-            if (avg < best) {
-                best = avg;
+            bk.candidateMs[v] = least;
+            if (least < best) {
+                best = least;
                 bestV = v;
             }
         }
@@ -536,10 +535,13 @@ void Batch::autotune(float dt, int reps) {
     // 16 to 512 bodies 952 -> 860 us a step, 2,048 of 16 to 2,048 mixed bodies 700 ->
     // 644).  So each bucket's choice is tried again in the whole step, the largest
     // worlds first.  (64, 128 and 256 threads with registers for 8, 6 and 3 blocks an
-    // SM were tried as well and never chosen.)
+    // SM were tried as well and never chosen.)  A time is the least of its launches: with
+    // their mean, one launch held up by the host chose a step of 950 us in place of one of
+    // 750 three times in fourteen; once now.  Trying the variants in the step takes as
+    // long again as timing them alone (1,024 worlds 23 -> 48 ms, once).
     if (buckets_.size() > 1) {
         auto stepMs = [&]() {
-            float total = 0.0f;
+            float least = 1e30f;
             for (int r = 0; r < reps + 1; ++r) {
                 PE_CHECK(cudaEventRecord(t0_, stream_));
                 launchAll(dt, parity_);
@@ -547,9 +549,9 @@ void Batch::autotune(float dt, int reps) {
                 PE_CHECK(cudaStreamSynchronize(stream_));
                 float ms = 0.0f;
                 PE_CHECK(cudaEventElapsedTime(&ms, t0_, t1_));
-                if (r > 0) total += ms;
+                if (r > 0) least = std::min(least, ms);
             }
-            return (double)total / reps;
+            return (double)least;
         };
         double best = stepMs();
         for (size_t i = buckets_.size(); i-- > 0;) {
