@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kIslPrepThreads) k_prepare_islands(SolveArgs a
 // the front's arrays: a phase then costs a block barrier and loads from the block's own
 // memory, not a cluster barrier and loads from another SM's (1,000 spheres on a floor,
 // 616 manifolds in four colours, 10 iterations: the sweeps with their staging 64 -> 45
-// us, the step 131 -> 118).
+// us; the settled step over eight seeds 117 to 163 -> 114 to 133).
 struct SplitVel {
     float4 *l, *w;      // linear and angular velocities by slot (apart: fewer bank conflicts)
     const uint2 *slot;  // per solve index: slots of body A and body B

@@ -29,6 +29,8 @@
 //                 number of updates they have seen), with no barrier between
 //                 colours.  Every body sees its manifolds in (colour, index)
 //                 order, as in colour-by-colour sweeps, so the result is theirs.
+//                 A world whose last steps were piles runs this kernel alone for
+//                 every manifold, without the island kernels (launchSolveSweep).
 #include <stdexcept>
 
 #include "pe_block.cuh"
